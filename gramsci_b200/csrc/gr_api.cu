@@ -870,7 +870,7 @@ static int pick_pair2_variant(gr_ctx* c, const DevCatalog& C, bool weighted, dou
   int cb = 0;
   while (cb < 20 && ((int64_t)4 << (2 * cb)) <= C.grid.ncell) ++cb;
   char key[128];
-  std::snprintf(key, sizeof(key), "pair2v9|%s|%s|dens%d|hist%d|cells%d", c->P.f32 ? "f32" : "f64",
+  std::snprintf(key, sizeof(key), "pair2v10|%s|%s|dens%d|hist%d|cells%d", c->P.f32 ? "f32" : "f64",
                 weighted ? "w" : "u", dens, hb, cb);
   Tuner& T = tuner();
   {
@@ -1742,7 +1742,7 @@ static int pick_adj2_layout(gr_ctx* c, const DevCatalog& C, const double* c2, co
   int cb = 0;
   while (cb < 20 && ((int64_t)4 << (2 * cb)) <= C.grid.ncell) ++cb;
   char key[128];
-  std::snprintf(key, sizeof(key), "adj2v2|%s|dens%d|hist%d|cells%d", c->P.f32 ? "f32" : "f64", dens,
+  std::snprintf(key, sizeof(key), "adj2v3|%s|dens%d|hist%d|cells%d", c->P.f32 ? "f32" : "f64", dens,
                 hb, cb);
   Tuner& T = tuner();
   {

@@ -610,6 +610,76 @@ __device__ __forceinline__ void fix_merge(unsigned long long* lo, unsigned long 
   if (d) atomicAdd(hi, d);
 }
 
+// Shared-memory accumulators are updated with 32-bit atomics only.  The SM
+// adds 32-bit integers in the shared-memory unit itself, while a 64-bit
+// shared atomic add is a compare-and-swap loop that runs once more for every
+// lane of the warp (or other warp) that meets it on the same word.  Measured
+// with 32 warps per SM on 2,400 bins, cycles per warp-wide update: one 64-bit
+// add with a carry 26 on uniformly spread bins and 179 on bins as uneven as
+// a histogram's; two 32-bit adds with their carries 10 and 12.
+
+// n added to a 64-bit counter held as two words, nh apart.
+__device__ __forceinline__ void smem_count_add(unsigned* c, int nh, unsigned n) {
+  const unsigned old = atomicAdd(c, n);
+  if (old + n < old) atomicAdd(c + nh, 1u);
+}
+
+// v added to a signed 64-bit integer in shared memory (wraps like one).
+__device__ __forceinline__ void smem_add_s64(unsigned long long* p, long long v) {
+  unsigned* w = reinterpret_cast<unsigned*>(p);  // low word first
+  const unsigned v0 = (unsigned)v;
+  const unsigned old = atomicAdd(w, v0);
+  const unsigned h = (unsigned)((unsigned long long)v >> 32) + (old + v0 < old ? 1u : 0u);
+  if (h) atomicAdd(w + 1, h);
+}
+
+// v added to a signed 128-bit integer held as four words, nh apart.  The
+// carry out of the low 64 bits and the sign extension of v cancel or are
+// both zero in most updates, which then touch two words.
+__device__ __forceinline__ void smem_fix_add(unsigned* w, int nh, long long v) {
+  const unsigned v0 = (unsigned)v, v1 = (unsigned)((unsigned long long)v >> 32);
+  const unsigned o0 = atomicAdd(w, v0);
+  const unsigned c0 = o0 + v0 < o0 ? 1u : 0u;
+  const unsigned h = v1 + c0;
+  const unsigned o1 = atomicAdd(w + nh, h);
+  // h = 0 with a carry in means v1 was all ones: that carry goes on
+  const int up = (v < 0 ? -1 : 0) + ((o1 + h < o1 || h < c0) ? 1 : 0);
+  if (up) {
+    const unsigned o2 = atomicAdd(w + 2 * nh, (unsigned)up);
+    if (up < 0 ? o2 == 0u : o2 == 0xffffffffu) atomicAdd(w + 3 * nh, (unsigned)up);
+  }
+}
+
+// One entry of a histogram that lies in shared memory (SHIST: words as
+// above, in the space of nh 64-bit counts and of nh (lo, hi) pairs) or in
+// global memory (64-bit counts; nh lo words, then nh hi words), k the entry.
+template <bool SHIST>
+__device__ __forceinline__ void hist_count_add(unsigned long long* cnt, int nh, int k, unsigned n) {
+  if (SHIST)
+    smem_count_add(reinterpret_cast<unsigned*>(cnt) + k, nh, n);
+  else
+    atomicAdd(&cnt[k], (unsigned long long)n);
+}
+template <bool SHIST>
+__device__ __forceinline__ void hist_fix_add(unsigned long long* fix, int nh, int k, long long v) {
+  if (SHIST)
+    smem_fix_add(reinterpret_cast<unsigned*>(fix) + k, nh, v);
+  else
+    fix_add_int(&fix[k], &fix[nh + k], v);
+}
+// Values of a shared-memory entry (read when no update is in flight).
+__device__ __forceinline__ unsigned long long hist_count_value(const unsigned long long* cnt, int nh,
+                                                               int k) {
+  const unsigned* c = reinterpret_cast<const unsigned*>(cnt);
+  return (unsigned long long)c[k] | ((unsigned long long)c[nh + k] << 32);
+}
+__device__ __forceinline__ void hist_fix_value(const unsigned long long* fix, int nh, int k,
+                                               unsigned long long& lo, unsigned long long& hi) {
+  const unsigned* w = reinterpret_cast<const unsigned*>(fix);
+  lo = (unsigned long long)w[k] | ((unsigned long long)w[nh + k] << 32);
+  hi = (unsigned long long)w[2 * nh + k] | ((unsigned long long)w[3 * nh + k] << 32);
+}
+
 // A 128-bit fixed-point accumulator held in registers.
 struct Fix128 {
   unsigned long long lo, hi;

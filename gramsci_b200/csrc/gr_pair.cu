@@ -35,14 +35,13 @@ __global__ void __launch_bounds__(kPairThreads) pair2_kernel(DevCatalog C, PairP
   const int nbm = P.nbins * P.nmu;
   const int nh = nbm * 4;
   unsigned long long* s_cnt = SHIST ? reinterpret_cast<unsigned long long*>(smem) : g_cnt;
-  unsigned long long* s_lo = SHIST ? s_cnt + nh : g_fix;
-  unsigned long long* s_hi = s_lo + nh;
+  unsigned long long* s_fix = SHIST ? s_cnt + nh : g_fix;
   if (SHIST) {
     for (int k = threadIdx.x; k < nh; k += blockDim.x) {
       s_cnt[k] = 0ull;
       if (WEIGHTED) {
-        s_lo[k] = 0ull;
-        s_hi[k] = 0ull;
+        s_fix[k] = 0ull;
+        s_fix[nh + k] = 0ull;
       }
     }
     __syncthreads();
@@ -114,13 +113,13 @@ __global__ void __launch_bounds__(kPairThreads) pair2_kernel(DevCatalog C, PairP
           if (WEIGHTED) prod = wp * C.w[q];
           if (root_p) {
             const int k = (b - 1) + P.nbins * (mf - 1) + nbm * (2 * rp + rq);
-            atomicAdd(&s_cnt[k], 1ull);
-            if (WEIGHTED) fix_add(&s_lo[k], &s_hi[k], prod, fscale);
+            hist_count_add<SHIST>(s_cnt, nh, k, 1u);
+            if (WEIGHTED) hist_fix_add<SHIST>(s_fix, nh, k, __double2ll_rn(prod * fscale));
           }
           if (!(fq & FLAG_BUFFER)) {
             const int k = (b - 1) + P.nbins * (mr - 1) + nbm * (2 * rq + rp);
-            atomicAdd(&s_cnt[k], 1ull);
-            if (WEIGHTED) fix_add(&s_lo[k], &s_hi[k], prod, fscale);
+            hist_count_add<SHIST>(s_cnt, nh, k, 1u);
+            if (WEIGHTED) hist_fix_add<SHIST>(s_fix, nh, k, __double2ll_rn(prod * fscale));
           }
         }
         if (lane == 0) cands += (unsigned long long)(tn - fstart);
@@ -140,9 +139,14 @@ __global__ void __launch_bounds__(kPairThreads) pair2_kernel(DevCatalog C, PairP
   if (SHIST) {
     __syncthreads();
     for (int k = threadIdx.x; k < nh; k += blockDim.x) {
-      if (s_cnt[k]) {
-        atomicAdd(&g_cnt[k], s_cnt[k]);
-        if (WEIGHTED) fix_merge(&g_fix[k], &g_fix[nh + k], s_lo[k], s_hi[k]);
+      const unsigned long long v = hist_count_value(s_cnt, nh, k);
+      if (v) {
+        atomicAdd(&g_cnt[k], v);
+        if (WEIGHTED) {
+          unsigned long long lo, hi;
+          hist_fix_value(s_fix, nh, k, lo, hi);
+          fix_merge(&g_fix[k], &g_fix[nh + k], lo, hi);
+        }
       }
     }
   }
@@ -169,14 +173,13 @@ __global__ void __launch_bounds__(kPairThreads) pair2_queue_kernel(
   const int nbm = P.nbins * P.nmu;
   const int nh = nbm * 4;
   unsigned long long* s_cnt = SHIST ? reinterpret_cast<unsigned long long*>(smem) : g_cnt;
-  unsigned long long* s_lo = SHIST ? s_cnt + nh : g_fix;
-  unsigned long long* s_hi = s_lo + nh;
+  unsigned long long* s_fix = SHIST ? s_cnt + nh : g_fix;
   if (SHIST) {
     for (int k = threadIdx.x; k < nh; k += blockDim.x) {
       s_cnt[k] = 0ull;
       if (WEIGHTED) {
-        s_lo[k] = 0ull;
-        s_hi[k] = 0ull;
+        s_fix[k] = 0ull;
+        s_fix[nh + k] = 0ull;
       }
     }
     __syncthreads();
@@ -213,13 +216,13 @@ __global__ void __launch_bounds__(kPairThreads) pair2_queue_kernel(
     const double prod = WEIGHTED ? C.w[p] * C.w[q] : 0.0;
     if (root_p) {
       const int k = (b - 1) + P.nbins * (mf - 1) + nbm * (2 * rp + rq);
-      atomicAdd(&s_cnt[k], 1ull);
-      if (WEIGHTED) fix_add(&s_lo[k], &s_hi[k], prod, fscale);
+      hist_count_add<SHIST>(s_cnt, nh, k, 1u);
+      if (WEIGHTED) hist_fix_add<SHIST>(s_fix, nh, k, __double2ll_rn(prod * fscale));
     }
     if (root_q) {
       const int k = (b - 1) + P.nbins * (mr - 1) + nbm * (2 * rq + rp);
-      atomicAdd(&s_cnt[k], 1ull);
-      if (WEIGHTED) fix_add(&s_lo[k], &s_hi[k], prod, fscale);
+      hist_count_add<SHIST>(s_cnt, nh, k, 1u);
+      if (WEIGHTED) hist_fix_add<SHIST>(s_fix, nh, k, __double2ll_rn(prod * fscale));
     }
   };
   for (;;) {
@@ -307,9 +310,14 @@ __global__ void __launch_bounds__(kPairThreads) pair2_queue_kernel(
   if (SHIST) {
     __syncthreads();
     for (int k = threadIdx.x; k < nh; k += blockDim.x) {
-      if (s_cnt[k]) {
-        atomicAdd(&g_cnt[k], s_cnt[k]);
-        if (WEIGHTED) fix_merge(&g_fix[k], &g_fix[nh + k], s_lo[k], s_hi[k]);
+      const unsigned long long v = hist_count_value(s_cnt, nh, k);
+      if (v) {
+        atomicAdd(&g_cnt[k], v);
+        if (WEIGHTED) {
+          unsigned long long lo, hi;
+          hist_fix_value(s_fix, nh, k, lo, hi);
+          fix_merge(&g_fix[k], &g_fix[nh + k], lo, hi);
+        }
       }
     }
   }
@@ -338,14 +346,13 @@ __global__ void __launch_bounds__(NT) pair2_dense_kernel(DevCatalog C, PairParam
   const int nbm = P.nbins * P.nmu;
   const int nh = nbm * 4;
   unsigned long long* s_cnt = SHIST ? reinterpret_cast<unsigned long long*>(smem) : g_cnt;
-  unsigned long long* s_lo = SHIST ? s_cnt + nh : g_fix;
-  unsigned long long* s_hi = s_lo + nh;
+  unsigned long long* s_fix = SHIST ? s_cnt + nh : g_fix;
   if (SHIST) {
     for (int k = threadIdx.x; k < nh; k += NT) {
       s_cnt[k] = 0ull;
       if (WEIGHTED) {
-        s_lo[k] = 0ull;
-        s_hi[k] = 0ull;
+        s_fix[k] = 0ull;
+        s_fix[nh + k] = 0ull;
       }
     }
   }
@@ -424,13 +431,13 @@ __global__ void __launch_bounds__(NT) pair2_dense_kernel(DevCatalog C, PairParam
           const double prod = WEIGHTED ? wp * s_w[f] : 0.0;
           if (root_p) {
             const int k = (b - 1) + P.nbins * (mf - 1) + nbm * (2 * rp + rq);
-            atomicAdd(&s_cnt[k], 1ull);
-            if (WEIGHTED) fix_add(&s_lo[k], &s_hi[k], prod, fscale);
+            hist_count_add<SHIST>(s_cnt, nh, k, 1u);
+            if (WEIGHTED) hist_fix_add<SHIST>(s_fix, nh, k, __double2ll_rn(prod * fscale));
           }
           if (!(fq & FLAG_BUFFER)) {
             const int k = (b - 1) + P.nbins * (mr - 1) + nbm * (2 * rq + rp);
-            atomicAdd(&s_cnt[k], 1ull);
-            if (WEIGHTED) fix_add(&s_lo[k], &s_hi[k], prod, fscale);
+            hist_count_add<SHIST>(s_cnt, nh, k, 1u);
+            if (WEIGHTED) hist_fix_add<SHIST>(s_fix, nh, k, __double2ll_rn(prod * fscale));
           }
         }
       }
@@ -451,9 +458,14 @@ __global__ void __launch_bounds__(NT) pair2_dense_kernel(DevCatalog C, PairParam
   if (SHIST) {
     __syncthreads();
     for (int k = threadIdx.x; k < nh; k += NT) {
-      if (s_cnt[k]) {
-        atomicAdd(&g_cnt[k], s_cnt[k]);
-        if (WEIGHTED) fix_merge(&g_fix[k], &g_fix[nh + k], s_lo[k], s_hi[k]);
+      const unsigned long long v = hist_count_value(s_cnt, nh, k);
+      if (v) {
+        atomicAdd(&g_cnt[k], v);
+        if (WEIGHTED) {
+          unsigned long long lo, hi;
+          hist_fix_value(s_fix, nh, k, lo, hi);
+          fix_merge(&g_fix[k], &g_fix[nh + k], lo, hi);
+        }
       }
     }
   }
@@ -482,14 +494,13 @@ __global__ void __launch_bounds__(NT) pair2_dense_queue_kernel(
   const int nbm = P.nbins * P.nmu;
   const int nh = nbm * 4;
   unsigned long long* s_cnt = SHIST ? reinterpret_cast<unsigned long long*>(smem) : g_cnt;
-  unsigned long long* s_lo = SHIST ? s_cnt + nh : g_fix;
-  unsigned long long* s_hi = s_lo + nh;
+  unsigned long long* s_fix = SHIST ? s_cnt + nh : g_fix;
   if (SHIST) {
     for (int k = threadIdx.x; k < nh; k += NT) {
       s_cnt[k] = 0ull;
       if (WEIGHTED) {
-        s_lo[k] = 0ull;
-        s_hi[k] = 0ull;
+        s_fix[k] = 0ull;
+        s_fix[nh + k] = 0ull;
       }
     }
   }
@@ -523,13 +534,13 @@ __global__ void __launch_bounds__(NT) pair2_dense_queue_kernel(
     const double prod = WEIGHTED ? C.w[p] * s_w[f] : 0.0;
     if (root_p) {
       const int k = (b - 1) + P.nbins * (mf - 1) + nbm * (2 * rp + rq);
-      atomicAdd(&s_cnt[k], 1ull);
-      if (WEIGHTED) fix_add(&s_lo[k], &s_hi[k], prod, fscale);
+      hist_count_add<SHIST>(s_cnt, nh, k, 1u);
+      if (WEIGHTED) hist_fix_add<SHIST>(s_fix, nh, k, __double2ll_rn(prod * fscale));
     }
     if (root_q) {
       const int k = (b - 1) + P.nbins * (mr - 1) + nbm * (2 * rq + rp);
-      atomicAdd(&s_cnt[k], 1ull);
-      if (WEIGHTED) fix_add(&s_lo[k], &s_hi[k], prod, fscale);
+      hist_count_add<SHIST>(s_cnt, nh, k, 1u);
+      if (WEIGHTED) hist_fix_add<SHIST>(s_fix, nh, k, __double2ll_rn(prod * fscale));
     }
   };
   for (;;) {
@@ -622,9 +633,14 @@ __global__ void __launch_bounds__(NT) pair2_dense_queue_kernel(
   if (SHIST) {
     __syncthreads();
     for (int k = threadIdx.x; k < nh; k += NT) {
-      if (s_cnt[k]) {
-        atomicAdd(&g_cnt[k], s_cnt[k]);
-        if (WEIGHTED) fix_merge(&g_fix[k], &g_fix[nh + k], s_lo[k], s_hi[k]);
+      const unsigned long long v = hist_count_value(s_cnt, nh, k);
+      if (v) {
+        atomicAdd(&g_cnt[k], v);
+        if (WEIGHTED) {
+          unsigned long long lo, hi;
+          hist_fix_value(s_fix, nh, k, lo, hi);
+          fix_merge(&g_fix[k], &g_fix[nh + k], lo, hi);
+        }
       }
     }
   }

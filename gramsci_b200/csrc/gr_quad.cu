@@ -127,7 +127,7 @@ __host__ __device__ inline QuadLayout quad_layout(int nbins, int cap, int nwarps
   L.o_rs = w;   w += (size_t)cap * 8;   // row start of each neighbour
   L.o_w = w;    w += (size_t)cap * 8;   // weight
   L.o_mo = w;   w += (size_t)cap * 8;   // (catalogue id << 32) | flags << 24 | meta(p, a)
-  L.o_g = w;    w += adj ? (size_t)cap * 16 : 0;  // gradient (lo, hi) of each neighbour
+  L.o_g = w;    w += adj ? (size_t)cap * 16 : 0;  // 128-bit gradient of each neighbour
   L.o_col = w;  w += (size_t)cap * 4;   // label
   L.o_len = w;  w += (size_t)cap * 4;   // row length
   L.o_xm = w;   w += (size_t)cap * 4;   // X entry z: meta(a, b)
@@ -590,16 +590,16 @@ __device__ __forceinline__ int quad_contrib_flat(const QuadCtx& X, const QVerts&
 // ya, yb, yd.  Returns the number of rooted contributions.
 template <bool WEIGHTED, bool SHC, bool ADJ, bool COMPACT, bool TETRA>
 __device__ __forceinline__ int quad_emit(const QuadCtx& X, const QVerts& V, const uint32_t m[6],
-                                         double gscale, Fix128& racc, unsigned long long* s_glo,
-                                         unsigned long long* s_ghi, int ya, int yb, int yd) {
+                                         double gscale, Fix128& racc, unsigned* s_grad, int gcap,
+                                         int ya, int yb, int yd) {
   if constexpr (ADJ) {
     double g[4];
     const int nroot = quad_grad_c(X, V, m, g);
     if (nroot) {
       fix_acc(racc, g[0], gscale);
-      fix_add(&s_glo[ya], &s_ghi[ya], g[1], gscale);
-      fix_add(&s_glo[yb], &s_ghi[yb], g[2], gscale);
-      fix_add(&s_glo[yd], &s_ghi[yd], g[3], gscale);
+      smem_fix_add(s_grad + ya, gcap, __double2ll_rn(g[1] * gscale));
+      smem_fix_add(s_grad + yb, gcap, __double2ll_rn(g[2] * gscale));
+      smem_fix_add(s_grad + yd, gcap, __double2ll_rn(g[3] * gscale));
     }
     return nroot;
   } else if constexpr (TETRA) {
@@ -648,8 +648,7 @@ __global__ void __launch_bounds__((WEIGHTED || ADJ ? kQuadMaxWarps : kQuadMaxWar
   uint16_t* s_xy = reinterpret_cast<uint16_t*>(wb + L.o_xy);
   uint16_t* s_xz = reinterpret_cast<uint16_t*>(wb + L.o_xz);
   uint32_t* s_bits = reinterpret_cast<uint32_t*>(wb + L.o_bits);
-  unsigned long long* s_glo = reinterpret_cast<unsigned long long*>(wb + L.o_g);
-  unsigned long long* s_ghi = s_glo + Q.cap;
+  unsigned* s_grad = reinterpret_cast<unsigned*>(wb + L.o_g);  // four words per neighbour, cap apart
   const int cap = Q.cap;
   const int lg_max = qhash_lg_max(cap);
   unsigned long long quads = 0, rooted = 0, probes = 0;
@@ -714,8 +713,7 @@ __global__ void __launch_bounds__((WEIGHTED || ADJ ? kQuadMaxWarps : kQuadMaxWar
                   (rec_meta(r) | ((uint32_t)fa << 24));
         if (LW) s_w[x] = C.w[a];
         if (ADJ) {
-          s_glo[x] = 0ull;
-          s_ghi[x] = 0ull;
+          s_grad[x] = s_grad[Q.cap + x] = s_grad[2 * Q.cap + x] = s_grad[3 * Q.cap + x] = 0u;
         }
         const uint32_t off = (uint32_t)(a - p);
         const uint32_t key = (off << 10) | (uint32_t)x;
@@ -804,7 +802,7 @@ __global__ void __launch_bounds__((WEIGHTED || ADJ ? kQuadMaxWarps : kQuadMaxWar
                                          (unsigned)x | ((unsigned)yb << 10) | ((unsigned)yd << 20),
                                          s_w, wp);
         else
-          nroot = quad_emit<WEIGHTED, SHC, ADJ, COMPACT, TETRA>(X, V, m, gscale, racc, s_glo, s_ghi,
+          nroot = quad_emit<WEIGHTED, SHC, ADJ, COMPACT, TETRA>(X, V, m, gscale, racc, s_grad, Q.cap,
                                                                 x, yb, yd);
         quads += nroot > 0;
         rooted += nroot;
@@ -889,7 +887,8 @@ __global__ void __launch_bounds__((WEIGHTED || ADJ ? kQuadMaxWarps : kQuadMaxWar
     if (ADJ) {
       // flush the gradients of this root and of its neighbours
       for (int x = lane; x < k; x += 32) {
-        const unsigned long long lo = s_glo[x], hi = s_ghi[x];
+        unsigned long long lo, hi;
+        hist_fix_value(reinterpret_cast<const unsigned long long*>(s_grad), Q.cap, x, lo, hi);
         if (lo | hi) fix_merge(&g_lo[s_col[x]], &g_hi[s_col[x]], lo, hi);
       }
       racc = fix_warp_sum(racc);
@@ -950,7 +949,7 @@ __host__ __device__ inline QuadGLayout quadg_layout(int nbins, int cap, int nwar
   L.o_pos = w;  w += (size_t)cap * 16;              // float4 position of each member
   L.o_w = w;    w += lw ? (size_t)cap * 8 : 0;      // weight
   L.o_mo = w;   w += (size_t)cap * 8;               // (catalogue id << 32) | flags << 24 | meta(p, a)
-  L.o_g = w;    w += adj ? (size_t)cap * 16 : 0;    // gradient (lo, hi)
+  L.o_g = w;    w += adj ? (size_t)cap * 16 : 0;    // 128-bit gradient of each neighbour
   L.o_col = w;  w += (size_t)cap * 4;               // label
   L.o_adj = w;  w += (size_t)cap * nwd * 4;         // adjacency rows
   L.o_q = w;    w += (size_t)kQQueue * 4;           // cliques: a | b << 8 | d << 16 | bin(a,b) << 24
@@ -983,8 +982,7 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
   float4* s_pos = reinterpret_cast<float4*>(wb + L.o_pos);
   double* s_w = reinterpret_cast<double*>(wb + L.o_w);
   unsigned long long* s_mo = reinterpret_cast<unsigned long long*>(wb + L.o_mo);
-  unsigned long long* s_glo = reinterpret_cast<unsigned long long*>(wb + L.o_g);
-  unsigned long long* s_ghi = s_glo + Q.cap;
+  unsigned* s_grad = reinterpret_cast<unsigned*>(wb + L.o_g);  // four words per neighbour, cap apart
   int* s_col = reinterpret_cast<int*>(wb + L.o_col);
   uint32_t* s_adj = reinterpret_cast<uint32_t*>(wb + L.o_adj);
   uint32_t* s_q = reinterpret_cast<uint32_t*>(wb + L.o_q);
@@ -1019,8 +1017,7 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
       s_mo[x] = ((unsigned long long)(uint32_t)C.orig[a] << 32) | (rec_meta(r) | ((uint32_t)fa << 24));
       if (LW) s_w[x] = C.w[a];
       if (ADJ) {
-        s_glo[x] = 0ull;
-        s_ghi[x] = 0ull;
+        s_grad[x] = s_grad[Q.cap + x] = s_grad[2 * Q.cap + x] = s_grad[3 * Q.cap + x] = 0u;
       }
     }
     for (int i = lane; i < k * nwk; i += 32) s_adj[i] = 0u;
@@ -1100,7 +1097,7 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
                                        (unsigned)x | ((unsigned)y << 10) | ((unsigned)z << 20), s_w,
                                        wp);
       else
-        nroot = quad_emit<WEIGHTED, SHC, ADJ, COMPACT, TETRA>(X, V, m, gscale, racc, s_glo, s_ghi,
+        nroot = quad_emit<WEIGHTED, SHC, ADJ, COMPACT, TETRA>(X, V, m, gscale, racc, s_grad, Q.cap,
                                                               x, y, z);
       quads += nroot > 0;
       rooted += nroot;
@@ -1172,7 +1169,8 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
     }
     if (ADJ) {
       for (int x = lane; x < k; x += 32) {
-        const unsigned long long lo = s_glo[x], hi = s_ghi[x];
+        unsigned long long lo, hi;
+        hist_fix_value(reinterpret_cast<const unsigned long long*>(s_grad), Q.cap, x, lo, hi);
         if (lo | hi) fix_merge(&g_lo[s_col[x]], &g_hi[s_col[x]], lo, hi);
       }
       racc = fix_warp_sum(racc);

@@ -117,15 +117,14 @@ __global__ void __launch_bounds__(kTileThreads, (ADJ && SUB == 2) ? 4 : GR_TILE_
   // per-warp histograms: counts (32-bit), then fixed-point lo and hi words
   const size_t wstride = WHIST ? (size_t)nh * (WEIGHTED ? 20 : 4) : 0;
   unsigned int* w_cnt = reinterpret_cast<unsigned int*>(smem + wstride * wib);
-  unsigned long long* w_lo =
+  unsigned long long* w_fix =
       reinterpret_cast<unsigned long long*>(smem + wstride * wib + (size_t)nh * 4);
-  unsigned long long* w_hi = w_lo + nh;
   if (WHIST) {
     for (int k = lane; k < nh; k += 32) {
       w_cnt[k] = 0u;
       if (WEIGHTED) {
-        w_lo[k] = 0ull;
-        w_hi[k] = 0ull;
+        w_fix[k] = 0ull;
+        w_fix[nh + k] = 0ull;
       }
     }
   }
@@ -150,10 +149,14 @@ __global__ void __launch_bounds__(kTileThreads, (ADJ && SUB == 2) ? 4 : GR_TILE_
         atomicAdd(&o_cnt[k], (unsigned long long)w_cnt[k]);
         w_cnt[k] = 0u;
       }
-      if (WEIGHTED && (w_lo[k] | w_hi[k])) {
-        fix_merge(&o_fix[k], &o_fix[nh + k], w_lo[k], w_hi[k]);
-        w_lo[k] = 0ull;
-        w_hi[k] = 0ull;
+      if (WEIGHTED) {
+        unsigned long long vlo, vhi;
+        hist_fix_value(w_fix, nh, k, vlo, vhi);
+        if (vlo | vhi) {
+          fix_merge(&o_fix[k], &o_fix[nh + k], vlo, vhi);
+          unsigned* w = reinterpret_cast<unsigned*>(w_fix);
+          w[k] = w[nh + k] = w[2 * nh + k] = w[3 * nh + k] = 0u;
+        }
       }
     }
     __syncwarp();
@@ -347,8 +350,8 @@ __global__ void __launch_bounds__(kTileThreads, (ADJ && SUB == 2) ? 4 : GR_TILE_
                 pairs += (!(fp & FLAG_BUFFER) || !(fq & FLAG_BUFFER)) ? 1 : 0;
                 const double cf = pair_coef(A.cot2, A.cot3, P.nbins, bin, mf, mr, fp, fq);
                 if (cf != 0.0) {
-                  atomicAdd(&T.groot[r], (unsigned long long)__double2ll_rn(cf * T.wq[j] * A.gscale));
-                  atomicAdd(&T.gcand[j], (unsigned long long)__double2ll_rn(cf * T.wr[r] * A.gscale));
+                  smem_add_s64(&T.groot[r], __double2ll_rn(cf * T.wq[j] * A.gscale));
+                  smem_add_s64(&T.gcand[j], __double2ll_rn(cf * T.wr[r] * A.gscale));
                 }
               }
             } else if (tile_bins<F32>(C, P, pr, q, a, b, bin, mf, mr, rechecks)) {
@@ -356,25 +359,25 @@ __global__ void __launch_bounds__(kTileThreads, (ADJ && SUB == 2) ? 4 : GR_TILE_
               const bool root_p = !(fp & FLAG_BUFFER), root_q = !(fq & FLAG_BUFFER);
               const int rp = fp & FLAG_RANDOM, rq = fq & FLAG_RANDOM;
               pairs += (root_p || root_q) ? 1 : 0;
-              const double prod = WEIGHTED ? T.wr[r] * T.wq[j] : 0.0;
+              const long long v = WEIGHTED ? __double2ll_rn(T.wr[r] * T.wq[j] * fscale) : 0ll;
               if (root_p) {
                 const int kh = (bin - 1) + P.nbins * (mf - 1) + nbm * (2 * rp + rq);
                 if (WHIST) {
                   atomicAdd(&w_cnt[kh], 1u);
-                  if (WEIGHTED) fix_add(&w_lo[kh], &w_hi[kh], prod, fscale);
+                  if (WEIGHTED) hist_fix_add<true>(w_fix, nh, kh, v);
                 } else {
                   atomicAdd(&o_cnt[kh], 1ull);
-                  if (WEIGHTED) fix_add(&o_fix[kh], &o_fix[nh + kh], prod, fscale);
+                  if (WEIGHTED) fix_add_int(&o_fix[kh], &o_fix[nh + kh], v);
                 }
               }
               if (root_q) {
                 const int kh = (bin - 1) + P.nbins * (mr - 1) + nbm * (2 * rq + rp);
                 if (WHIST) {
                   atomicAdd(&w_cnt[kh], 1u);
-                  if (WEIGHTED) fix_add(&w_lo[kh], &w_hi[kh], prod, fscale);
+                  if (WEIGHTED) hist_fix_add<true>(w_fix, nh, kh, v);
                 } else {
                   atomicAdd(&o_cnt[kh], 1ull);
-                  if (WEIGHTED) fix_add(&o_fix[kh], &o_fix[nh + kh], prod, fscale);
+                  if (WEIGHTED) fix_add_int(&o_fix[kh], &o_fix[nh + kh], v);
                 }
               }
             }

@@ -130,10 +130,10 @@ __device__ __forceinline__ int normal_bin(const TriCtx& X, int mu1, int mu2, boo
   return first_is_1 ? X.norm[(mu1 - 1) + X.nmu * (mu2 - 1)] : X.norm[(mu2 - 1) + X.nmu * (mu1 - 1)];
 }
 
-template <bool WEIGHTED, bool COUNTS>
+template <bool WEIGHTED, bool COUNTS, bool SHIST>
 __device__ __forceinline__ void tri_add(const TriCtx& X, int k, int n, long long v) {
-  if (COUNTS) atomicAdd(&X.cnt[k], (unsigned long long)n);
-  if (WEIGHTED) fix_add_int(&X.lim[k], &X.lim[X.nh + k], v * n);
+  if (COUNTS) hist_count_add<SHIST>(X.cnt, X.nh, k, (unsigned)n);
+  if (WEIGHTED) hist_fix_add<SHIST>(X.lim, X.nh, k, v * n);
 }
 
 // One triangle (p, a, c) with p < a < c in labels.  It adds to the rooted
@@ -144,7 +144,7 @@ __device__ __forceinline__ void tri_add(const TriCtx& X, int k, int n, long long
 // reference multiplies in differ from it by at most an ulp).  Roots that land
 // in the same bin share one update.  Returns the number of rooted
 // contributions.
-template <bool WEIGHTED, bool COUNTS>
+template <bool WEIGHTED, bool COUNTS, bool SHIST>
 __device__ __forceinline__ int tri_bin(const TriCtx& X, uint8_t fp, int op, double wp, uint8_t fa,
                                        int oa, double wa, uint8_t fc, int oc, double wc,
                                        uint32_t mpa, uint32_t mpc, uint32_t mac) {
@@ -173,9 +173,9 @@ __device__ __forceinline__ int tri_bin(const TriCtx& X, uint8_t fp, int op, doub
   if (c2 && m2 == m0 && c0) { c0 += c2; c2 = 0; }
   else if (c2 && m2 == m1 && c1) { c1 += c2; c2 = 0; }
   const int base = (cfg - 1) + X.ncfg * X.nmu * nr;
-  if (c0) tri_add<WEIGHTED, COUNTS>(X, base + X.ncfg * (m0 - 1), c0, v);
-  if (c1) tri_add<WEIGHTED, COUNTS>(X, base + X.ncfg * (m1 - 1), c1, v);
-  if (c2) tri_add<WEIGHTED, COUNTS>(X, base + X.ncfg * (m2 - 1), c2, v);
+  if (c0) tri_add<WEIGHTED, COUNTS, SHIST>(X, base + X.ncfg * (m0 - 1), c0, v);
+  if (c1) tri_add<WEIGHTED, COUNTS, SHIST>(X, base + X.ncfg * (m1 - 1), c1, v);
+  if (c2) tri_add<WEIGHTED, COUNTS, SHIST>(X, base + X.ncfg * (m2 - 1), c2, v);
   return total;
 }
 
@@ -215,8 +215,8 @@ __device__ __forceinline__ int tri_grad(const TriCtx& X, uint8_t fp, int op, dou
   if (C != 0.0) {
     fix_acc(racc, C * (wa * wc), X.gscale);
     if (S64) {
-      atomicAdd(alo, (unsigned long long)__double2ll_rn(C * (wp * wc) * X.gscale));
-      atomicAdd(clo, (unsigned long long)__double2ll_rn(C * (wp * wa) * X.gscale));
+      smem_add_s64(alo, __double2ll_rn(C * (wp * wc) * X.gscale));
+      smem_add_s64(clo, __double2ll_rn(C * (wp * wa) * X.gscale));
     } else {
       fix_add(alo, ahi, C * (wp * wc), X.gscale);
       fix_add(clo, chi, C * (wp * wa), X.gscale);
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(kTriMaxWarps * 32) tri3_kernel(DevCatalog C, C
     if (ADJ)
       return tri_grad<true>(X, fp, op, wp, fa, oa, s_w[qx], fc, oc, s_w[qy], ma, mc, mac, racc,
                             &s_g[qx], nullptr, &s_g[qy], nullptr);
-    return tri_bin<WEIGHTED, COUNTS>(X, fp, op, wp, fa, oa, WEIGHTED ? s_w[qx] : 0.0, fc, oc,
+    return tri_bin<WEIGHTED, COUNTS, SHIST>(X, fp, op, wp, fa, oa, WEIGHTED ? s_w[qx] : 0.0, fc, oc,
                                      WEIGHTED ? s_w[qy] : 0.0, ma, mc, mac);
   };
 
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(kTriMaxWarps * 32) tri3_kernel(DevCatalog C, C
                   ADJ ? tri_grad<false>(X, fp, op, wp, fa, oa, wa, C.flags[c], C.orig[c], C.w[c], mpa,
                                  rec_meta(rowp[y]), rec_meta(r), racc, &g_lo[a], &g_hi[a], &g_lo[c],
                                  &g_hi[c])
-                      : tri_bin<WEIGHTED, COUNTS>(X, fp, op, wp, fa, oa, wa, C.flags[c], C.orig[c],
+                      : tri_bin<WEIGHTED, COUNTS, SHIST>(X, fp, op, wp, fa, oa, wa, C.flags[c], C.orig[c],
                                                   WEIGHTED ? C.w[c] : 0.0, mpa, rec_meta(rowp[y]),
                                                   rec_meta(r));
               tris += nroot > 0;
@@ -615,11 +615,12 @@ __global__ void __launch_bounds__(kTriMaxWarps * 32) tri3_kernel(DevCatalog C, C
     __syncthreads();
     for (int k = threadIdx.x; k < nh; k += blockDim.x) {
       if (COUNTS) {
-        const unsigned long long v = X.cnt[k];
+        const unsigned long long v = hist_count_value(X.cnt, nh, k);
         if (v) atomicAdd(&g_cnt[k], v);
       }
       if (WEIGHTED) {
-        const unsigned long long lo = X.lim[k], hi = X.lim[nh + k];
+        unsigned long long lo, hi;
+        hist_fix_value(X.lim, nh, k, lo, hi);
         if (lo | hi) fix_merge(&g_lim[k], &g_lim[nh + k], lo, hi);
       }
     }
