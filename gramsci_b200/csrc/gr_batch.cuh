@@ -25,6 +25,9 @@ struct RegionGeomDev {
   const GridParams* grid;
   const int* cell_off;   // nreg + 1
   int ns;                // subcubes per axis (subcube split)
+  // subcube split: box origin and 1/extent per axis, and Rmax in subcube
+  // widths with a margin for rounding (2 or more: no axis test)
+  double lo[3], inv_span[3], reach[3];
 };
 
 // How the catalogue is split into regions.
@@ -48,9 +51,11 @@ struct RegionLayout {
   // ids / mocks: the region of every point (in `sub`) and, for mocks, the
   // random flag of every point
   DevBuf<uint8_t> pflag;
+  DevBuf<int64_t> mock_off;  // bounds of the mocks' galaxies and randoms
   // ids: coarse grid over the catalogue; cell c lists the regions whose halo
   // reaches it (coarse_off[c] .. coarse_off[c+1] in coarse_list)
   GridGeom coarse{};
+  double cat_lo[3] = {0, 0, 0}, cat_inv_span[3] = {0, 0, 0}, reach[3] = {2, 2, 2};
   int64_t ncoarse = 0;
   DevBuf<int> coarse_off, coarse_list;
   // device geometry
@@ -67,7 +72,9 @@ struct RegionLayout {
   DevBuf<float4> pos4;
   DevBuf<double4> posd;
   DevBuf<double> w;
-  // replay of the per-call device work
+  // replay of the per-call device work; swept: a batched 2PCF has run on the
+  // current plan (and picked its variant)
+  bool swept = false;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
 
@@ -77,8 +84,9 @@ struct RegionLayout {
   // plan's sub_policy 0 picks 2 when the rmax-wide grids would hold at least
   // dense_per_cell members per cell
   int grid_sub = 1;
-  void plan(const double* d_xyz, int64_t n, int64_t n_data, double rmax, int nsplit, cudaStream_t s,
-            int sub_policy = 1, double dense_per_cell = 0.0);
+  // box: the catalogue's bounding box
+  void plan(const double* d_xyz, int64_t n, int64_t n_data, const CatalogBox& box, double rmax,
+            int nsplit, cudaStream_t s, int sub_policy = 1, double dense_per_cell = 0.0);
   // ids: region of every point (host array of n entries in [0, nregions));
   // mocks: galaxies and randoms of each mock, the catalogue being the mocks
   // one after another, each with its galaxies first.  Both replace the
@@ -89,11 +97,13 @@ struct RegionLayout {
     mode = kRegionsSplit;
     valid = false;
   }
-  void enqueue_layout(const double* d_xyz, const double* d_w, cudaStream_t s);
+  // planned: just after plan(), whose membership counts (mcount) still stand
+  void enqueue_layout(const double* d_xyz, const double* d_w, cudaStream_t s, bool planned = false);
+  RegionGeomDev geom_dev() const;
   DevCatalog view() const;
   CoarseDev coarse_dev() const;
-  // membership kernels (pass 0: members per region, 1: memberships per
-  // point, 2: the members)
+  // membership kernels (pass 0: members per region and memberships per
+  // point, 1: memberships per point, 2: the members)
   void launch_members(int pass, const double* d_xyz, const RegionGeomDev& G, cudaStream_t s);
 };
 

@@ -184,6 +184,42 @@ int blocks_for(int64_t n, int threads, int waves = 16) {
 
 }  // namespace
 
+namespace {
+
+// The raw box of bbox_kernel as doubles.
+CatalogBox box_of_keys(const unsigned long long h[8], int64_t n) {
+  CatalogBox b;
+  for (int d = 0; d < 3; ++d) {
+    b.lo[d] = n > 0 ? key_to_dbl(h[d]) : 0.0;
+    b.hi[d] = n > 0 ? key_to_dbl(h[3 + d]) : 0.0;
+  }
+  b.coord_max = n > 0 ? key_to_dbl(h[6]) : 0.0;
+  for (int d = 0; d < 3; ++d)
+    if (h[7] != 0 || !std::isfinite(b.lo[d]) || !std::isfinite(b.hi[d]))
+      throw Error{-1, "catalogue has non-finite coordinates"};
+  return b;
+}
+
+// Queue the raw box (order keys, see bbox_kernel); returns the launches.
+int enqueue_box(const double* d_xyz, int64_t n, unsigned long long* raw, cudaStream_t s) {
+  init_bbox_kernel<<<1, 32, 0, s>>>(raw);
+  if (n > 0) bbox_kernel<<<blocks_for(n, 256, 2), 256, 0, s>>>(d_xyz, n, raw);
+  GR_CHECK_LAUNCH();
+  return n > 0 ? 2 : 1;
+}
+
+}  // namespace
+
+CatalogBox catalog_box(const double* d_xyz, int64_t n, DevBuf<unsigned long long>& raw,
+                       cudaStream_t s) {
+  raw.reserve(8);
+  enqueue_box(d_xyz, n, raw.p, s);
+  unsigned long long h[8];
+  GR_CUDA_TRY(cudaMemcpyAsync(h, raw.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+  GR_CUDA_TRY(cudaStreamSynchronize(s));
+  return box_of_keys(h, n);
+}
+
 void CellIndex::build(const double* d_xyz, const double* d_w, const int* d_buffer, int64_t n_pts,
                       int64_t n_data_pts, double rmax, cudaStream_t s, bool speculate, int sub,
                       double dense_per_cell) {
@@ -194,13 +230,7 @@ void CellIndex::build(const double* d_xyz, const double* d_w, const int* d_buffe
   launches = 0;
   bbox_raw.reserve(8);
   bbox_prev.reserve(8);
-  init_bbox_kernel<<<1, 32, 0, s>>>(bbox_raw.p);
-  launches++;
-  if (n > 0) {
-    bbox_kernel<<<blocks_for(n, 256, 2), 256, 0, s>>>(d_xyz, n, bbox_raw.p);
-    launches++;
-  }
-  GR_CHECK_LAUNCH();
+  launches += enqueue_box(d_xyz, n, bbox_raw.p, s);
   unsigned long long h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   // an automatic choice of sub decides from the bounding box, so it speculates
   // on the previous build's box like the grid does
@@ -214,7 +244,7 @@ void CellIndex::build(const double* d_xyz, const double* d_w, const int* d_buffe
   } else {
     GR_CUDA_TRY(cudaMemcpyAsync(h, bbox_raw.p, sizeof(h), cudaMemcpyDeviceToHost, s));
     GR_CUDA_TRY(cudaStreamSynchronize(s));
-    if (h[7] != 0) throw Error{-1, "catalogue has non-finite coordinates"};
+    box_of_keys(h, n);  // raises on a non-finite coordinate
     std::memcpy(prev_raw, h, sizeof(prev_raw));
     prev_n = n;
     prev_rmax = rmax;
@@ -224,24 +254,17 @@ void CellIndex::build(const double* d_xyz, const double* d_w, const int* d_buffe
     GR_CUDA_TRY(cudaMemcpyAsync(bbox_prev.p, prev_raw, sizeof(prev_raw), cudaMemcpyHostToDevice, s));
     GR_CUDA_TRY(cudaMemsetAsync(bbox_prev.p + 7, 0, sizeof(unsigned long long), s));
   }
-  double lo[3], hi[3];
-  for (int d = 0; d < 3; ++d) {
-    lo[d] = n > 0 ? key_to_dbl(h[d]) : 0.0;
-    hi[d] = n > 0 ? key_to_dbl(h[3 + d]) : 0.0;
-  }
-  coord_max = n > 0 ? key_to_dbl(h[6]) : 0.0;
-  for (int d = 0; d < 3; ++d)
-    if (!std::isfinite(lo[d]) || !std::isfinite(hi[d]))
-      throw Error{-1, "catalogue has non-finite coordinates"};
+  const CatalogBox box = box_of_keys(h, n);
+  coord_max = box.coord_max;
   // cells at least rmax (sub 2: rmax/2) wide; the cell table stays O(N)
   GridGeom g;
   {
-    const int64_t cells1 = make_grid_geom(lo, hi, rmax, 2048, std::max<int64_t>(4 * n, 4096), g);
+    const int64_t cells1 = make_grid_geom(box.lo, box.hi, rmax, 2048, std::max<int64_t>(4 * n, 4096), g);
     per_cell_rmax = cells1 > 0 ? (double)n / (double)cells1 : 0.0;
     if (auto_sub) sub = (dense_per_cell > 0.0 && per_cell_rmax >= dense_per_cell) ? 2 : 1;
   }
   const int64_t total =
-      make_grid_geom(lo, hi, rmax / sub, 2048, std::max<int64_t>(4 * n, 4096), g);
+      make_grid_geom(box.lo, box.hi, rmax / sub, 2048, std::max<int64_t>(4 * n, 4096), g);
   grid.nx = g.nc[0];
   grid.ny = g.nc[1];
   grid.nz = g.nc[2];

@@ -48,6 +48,13 @@ struct CellIndex {
   DevCatalog view() const;
 };
 
+// Bounding box of a catalogue and its largest |coordinate| (all zero without
+// points), read back with one wait; raises on non-finite coordinates.
+struct CatalogBox {
+  double lo[3], hi[3], coord_max;
+};
+CatalogBox catalog_box(const double* d_xyz, int64_t n, DevBuf<unsigned long long>& raw,
+                       cudaStream_t s);
 
 // Upper adjacency: row p lists the neighbours q > p (internal labels) of the
 // (rmin, rmax) graph in increasing label order, with packed bin / mu
