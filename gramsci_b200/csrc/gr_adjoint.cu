@@ -26,7 +26,7 @@ __device__ __forceinline__ bool adj_edge(const DevCatalog& C, const PairParams& 
                                          const float4& pi, const float4& pj, int& b, int& mf,
                                          int& mr) {
   if (F32) {
-    const int r = classify_f32<true>(pi, pj, P, b, mf, mr);
+    const int r = classify_f32(pi, pj, P, b, mf, mr);
     if (r != 2) return r == 1;
   }
   return edge_f64(C.posd[p], C.posd[q], P, b, mf, mr);

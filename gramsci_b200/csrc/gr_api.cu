@@ -163,20 +163,21 @@ void make_pair_params(PairParams& P, double rmin, double rmax, int nbins, int nm
   P.f_rmin = (float)rmin;
   P.f_inv_dr = (float)P.inv_dr;
   P.f_mu_scale = (float)P.mu_scale;
-  P.f_nmu = (float)nmu;
   const double tmax = nbins + 1.0;
   double tg = (d0 + u * std::fabs(rmin) + u * R) * P.inv_dr + 4.0 * u * tmax;
   tg = 2.0 * tg + 1e-9 * tmax;
   P.tguard = (float)tg;
+  P.f_t0 = (float)(-rmin * P.inv_dr);
   // line-of-sight cosine: (pi/2)(|ds|/|s| + |dm|/|m|) + arithmetic, doubled.
-  // The arithmetic term eC = 128 u covers the cosine evaluated with
-  // approximate square roots and division (about 21 u: dot product 3 u,
-  // |m| and d 6.5 u each, product u, __fdividef 4 u) with a margin of six.
+  // The arithmetic term 128 u covers the cosine evaluated with approximate
+  // reciprocal square roots (about 16 u: dot product 3 u, 1/|m| and 1/d 5.5 u
+  // each, two products) with a margin of eight; 8 u nmu more covers the
+  // rounding of the mu coordinate itself.
   const double pi = 3.14159265358979323846;
-  P.eA = (float)(pi * std::sqrt(3.0) * e1);
+  const double eA = pi * std::sqrt(3.0) * e1, eB = pi * 2.0 * std::sqrt(3.0) * X * u;
   P.mB = (float)(8.0 * X * u + 1e-30);
-  P.eB = (float)(pi * 2.0 * std::sqrt(3.0) * X * u);
-  P.eC = (float)(128.0 * u);
+  P.k1 = (float)((eA + eB) * P.mu_scale);
+  P.k2 = (float)(128.0 * u * P.mu_scale + 8.0 * u * nmu);
   P.f32 = (!force_fp64 && !logbins && std::isfinite(tg) && tg < 0.05 && std::isfinite(X)) ? 1 : 0;
 }
 
@@ -486,6 +487,16 @@ float ev_ms(cudaEvent_t a, cudaEvent_t b) {
 void set_pair_params(gr_ctx* c, double coord_max) {
   make_pair_params(c->P, c->rmin, c->rmax, c->nbins, c->nmu, c->logbins, coord_max,
                    c->precision == 1);
+}
+
+// Host state of a replayed index build that other calls may have changed
+// since it was captured (a batched call sets the pair parameters without a
+// build, another catalogue its own flags); the replay's key holds the rest.
+void restore_index(gr_ctx* c) {
+  c->index.n_data = c->n_data;
+  c->index.has_buffer = c->has_buffer ? 1 : 0;
+  set_pair_params(c, c->index.coord_max);
+  c->csr_valid = false;
 }
 
 void build_index(gr_ctx* c, bool speculate = false, int sub = 1) {
@@ -953,11 +964,8 @@ int gr_count_2pcf(gr_ctx* c, double* N2, double* N3, int64_t* counts, double* ca
     GR_CUDA_TRY(cudaEventRecord(c->ev[0], s));
     if (!reuse) {
       if (replayed) {
-        // the host state of the last identical build stands (but a batched
-        // call sets the pair parameters without a build)
-        set_pair_params(c, c->index.coord_max);
+        restore_index(c);
         GR_CUDA_TRY(cudaGraphLaunch(c->spec_index.idx, s));
-        c->csr_valid = false;
       } else {
         build_index(c, spec, sub);
       }
@@ -1117,11 +1125,8 @@ static int count_tri(gr_ctx* c, bool equi, double* N2, double* N3, int64_t* coun
     GR_CUDA_TRY(cudaEventRecord(c->ev[0], s));
     if (!reuse) {
       if (replay) {
-        // the host state of the last identical build stands (but a batched
-        // call sets the pair parameters without a build)
-        set_pair_params(c, c->index.coord_max);
+        restore_index(c);
         GR_CUDA_TRY(cudaGraphLaunch(c->spec_graph.idx, s));
-        c->csr_valid = false;
       } else {
         build_index(c, spec);
       }
@@ -1731,7 +1736,7 @@ static void finish_grad(gr_ctx* c, double gscale, double* grad_w, cudaEvent_t q0
 // or 256 threads): timed and cached like the forward sweep's variant, under
 // its own key (the fastest adjoint layout is not always the forward's).
 static int pick_adj2_layout(gr_ctx* c, const DevCatalog& C, const double* c2, const double* c3,
-                            double gscale, unsigned long long* g_lo, unsigned long long* g_hi,
+                            const double* tab, double gscale, unsigned long long* g_lo, unsigned long long* g_hi,
                             int* work, cudaStream_t s) {
   // a grid of rmax/2 cells is read by the tile sweep only
   if (C.grid.sub == 2) return kPairTile2;
@@ -1765,7 +1770,7 @@ static int pick_adj2_layout(gr_ctx* c, const DevCatalog& C, const double* c2, co
   c->stats.reserve(8);
   auto run = [&](int v) {
     if (layouts[v] == kPairTile)
-      launch_adj2_tile(C, c->P, c2, c3, gscale, g_lo, g_hi, c->stats.p, work, s);
+      launch_adj2_tile(C, c->P, tab, gscale, g_lo, g_hi, c->stats.p, work, s);
     else
       launch_adj2(C, c->P, c2, c3, gscale, g_lo, g_hi, work, s, layouts[v]);
   };
@@ -1801,15 +1806,17 @@ int gr_adjoint_2pcf(gr_ctx* c, const double* cot2, const double* cot3, double* g
   const int nbm = c->nbins * c->nmu;
   const int64_t n = c->n;
   const double cmax = max_abs(cot2, nbm) + max_abs(cot3, nbm);
-  c->cot.reserve(2 * nbm);
+  // cot2, cot3 and the tile sweep's table of pair coefficients
+  std::vector<double> cots(6 * (size_t)nbm, 0.0);
+  std::memcpy(cots.data(), cot2, sizeof(double) * nbm);
+  if (cot3) std::memcpy(cots.data() + nbm, cot3, sizeof(double) * nbm);
+  pair_coef_table(cots.data(), cots.data() + nbm, c->nbins, c->nmu, cots.data() + 2 * nbm);
+  c->cot.reserve(6 * nbm);
   c->gfix.reserve(2 * n + 2);
   c->work.reserve(4);
   c->stats.reserve(8);
-  GR_CUDA_TRY(cudaMemcpyAsync(c->cot.p, cot2, sizeof(double) * nbm, cudaMemcpyHostToDevice, s));
-  if (cot3)
-    GR_CUDA_TRY(cudaMemcpyAsync(c->cot.p + nbm, cot3, sizeof(double) * nbm, cudaMemcpyHostToDevice, s));
-  else
-    GR_CUDA_TRY(cudaMemsetAsync(c->cot.p + nbm, 0, sizeof(double) * nbm, s));
+  GR_CUDA_TRY(cudaMemcpyAsync(c->cot.p, cots.data(), sizeof(double) * cots.size(),
+                              cudaMemcpyHostToDevice, s));
   GR_CUDA_TRY(cudaEventRecord(c->ev[0], s));
   if (!reuse_graph(c)) {
     // dense catalogues: cells of rmax/2 and the tile sweep
@@ -1825,7 +1832,7 @@ int gr_adjoint_2pcf(gr_ctx* c, const double* cot2, const double* cot3, double* g
   // headroom over the largest term (2 cotangents times a weight)
   const double gscale_t = fix_scale(64.0 * 2.0 * cmax * c->wmax);
   const double gscale_c = fix_scale(2.0 * cmax * c->wmax);
-  const int variant = pick_adj2_layout(c, c->index.view(), c->cot.p, dc3, gscale_t, c->gfix.p,
+  const int variant = pick_adj2_layout(c, c->index.view(), c->cot.p, dc3, c->cot.p + 2 * nbm, gscale_t, c->gfix.p,
                                        c->gfix.p + n, c->work.p, s);
   const bool tile = variant == kPairTile || variant == kPairTile2;
   const double gscale = tile ? gscale_t : gscale_c;
@@ -1833,7 +1840,7 @@ int gr_adjoint_2pcf(gr_ctx* c, const double* cot2, const double* cot3, double* g
   GR_CUDA_TRY(cudaMemsetAsync(c->gfix.p, 0, sizeof(unsigned long long) * (2 * n + 2), s));
   if (tile) {
     GR_CUDA_TRY(cudaMemsetAsync(c->stats.p, 0, sizeof(unsigned long long) * 8, s));
-    launch_adj2_tile(c->index.view(), c->P, c->cot.p, dc3, gscale, c->gfix.p, c->gfix.p + n,
+    launch_adj2_tile(c->index.view(), c->P, c->cot.p + 2 * nbm, gscale, c->gfix.p, c->gfix.p + n,
                      c->stats.p, c->work.p, s);
   } else {
     launch_adj2(c->index.view(), c->P, c->cot.p, dc3, gscale, c->gfix.p, c->gfix.p + n, c->work.p,

@@ -742,6 +742,7 @@ DevCatalog RegionLayout::view() const {
   c.cell_start = cell_start.p;
   c.n = (int)n_members;
   c.n_data = (int)n_data;
+  c.has_buffer = mode != kRegionsMocks;
   c.grid = GridParams{1, 1, 1, ncell, grid_sub};
   c.cell_region = cell_region.p;
   c.region_grid = grid.p;

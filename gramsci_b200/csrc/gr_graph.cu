@@ -21,12 +21,12 @@ constexpr int kGraphWarps = 8;
 constexpr int kGraphThreads = kGraphWarps * 32;
 
 // Decide one candidate pair exactly.  Returns true for an edge.
-template <bool F32, bool NEED_BINS>
+template <bool F32>
 __device__ __forceinline__ bool pair_edge(const DevCatalog& C, const PairParams& P, int p, int q,
                                           const float4& pi, const float4& pj, int& bin, int& muf,
                                           int& mur, unsigned long long& rechecks) {
   if (F32) {
-    int r = classify_f32<NEED_BINS>(pi, pj, P, bin, muf, mur);
+    int r = classify_f32(pi, pj, P, bin, muf, mur);
     if (r != 2) return r == 1;
     rechecks++;
   }
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kGraphThreads) csr_fill_kernel(
     const int p = cb + (int)i;
     const int q = s_lab[wib][f];
     int b = 1, mf = 1, mr = 1;
-    if (!pair_edge<F32, true>(C, P, p, q, C.pos4[p], s_pos[wib][f], b, mf, mr, rechecks)) {
+    if (!pair_edge<F32>(C, P, p, q, C.pos4[p], s_pos[wib][f], b, mf, mr, rechecks)) {
       // the membership test and the binning disagree: reported, never expected
       disagree++;
       b = 1;

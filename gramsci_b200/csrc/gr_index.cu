@@ -227,6 +227,7 @@ void CellIndex::build(const double* d_xyz, const double* d_w, const int* d_buffe
   if (sub != 2) sub = 1;
   n = n_pts;
   n_data = n_data_pts;
+  has_buffer = d_buffer ? 1 : 0;
   launches = 0;
   bbox_raw.reserve(8);
   bbox_prev.reserve(8);
@@ -360,6 +361,7 @@ DevCatalog CellIndex::view() const {
   c.cell_start = cell_start.p;
   c.n = (int)n;
   c.n_data = (int)n_data;
+  c.has_buffer = has_buffer;
   c.grid = grid;
   c.cell_region = nullptr;
   c.region_grid = nullptr;

@@ -14,6 +14,7 @@ namespace gr {
 // Uniform-grid index over the catalogue, points laid out in cell order.
 struct CellIndex {
   int64_t n = 0, n_data = 0;
+  int has_buffer = 0;
   double coord_max = 0.0;  // max |coordinate|, bounds the FP32 rounding error
   GridParams grid{};
   int launches = 0;

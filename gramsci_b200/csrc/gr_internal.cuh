@@ -87,14 +87,15 @@ struct PairParams {
   // FP32 fast path with guard band
   int f32;           // 1 = FP32 path enabled
   float f_rmin, f_inv_dr, f_mu_scale;
+  float f_t0;        // -rmin / dr
   float rmax2_hi;    // d2 >= rmax2_hi: certainly d >= rmax
   float rmin2_lo;    // d2 <= rmin2_lo: certainly d <= rmin (or -1)
   float rmax2_lo;    // d2 < rmax2_lo: certainly d < rmax (or -1)
   float rmin2_hi;    // d2 > rmin2_hi: certainly d > rmin
   float tguard;      // |t - nearest integer| below this -> FP64
   float d0;          // bound on |d_f - d_true|
-  float eA, eB, mB, eC;  // cosine error model eA/(d-d0) + eB/(|m|-mB) + eC
-  float f_nmu;
+  // guard of the mu coordinate: k1 / min(d - d0, |m| - mB) + k2
+  float k1, k2, mB;
 };
 
 // Host: fill PairParams.  coord_max bounds |x|,|y|,|z| over the catalogue.
@@ -162,13 +163,67 @@ __device__ __forceinline__ bool edge_f64(const double4 pi, const double4 pj, con
   return true;
 }
 
-// FP32 classification.  Returns 0: certainly not an edge; 1: edge with the
-// bins written; 2: inside the guard band, re-evaluate with edge_f64.
-// NEED_BINS=false only decides membership (guards only at rmin and rmax).
-// The separation is d2 * rsqrtf(d2) and the cosine and its error bound use
-// __fdividef: make_pair_params sizes the guard band for these approximate
-// operations (d0 and eC), so outside the band the bins equal the FP64 ones.
-template <bool NEED_BINS>
+// 1/sqrt(x) within 2.14 units of 2^-24; subnormal x count as zero, which
+// gives infinity.
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// FP32 binning of a pair, the radial bin b0 and mu bin m0 from 0 (mu seen from
+// pi; from pj it is nmu - 1 - m0).  Returns 0: not an edge; 1: an edge with
+// these bins; 2: inside the guard band, re-evaluate with edge_f64.  There are
+// no branches and no divisions: 40 instructions with mu bins, the cost that
+// bounds every sweep that bins pairs.  The nearest integers of the radial and
+// mu coordinates come from adding and subtracting 1.5 * 2^23, whose low bits
+// are the integer.  A value nearer to any integer than its guard is decided in
+// FP64, the ends of the range included, so the bins need no clamping.  The
+// comparisons are written so that a NaN (a coincident pair, a midpoint at the
+// origin) is decided in FP64 too.  make_pair_params sizes the guards for these
+// operations: t with one rounding of c - rmin/dr and one of the sum beside
+// the error of d, and a cosine within 16 units of 2^-24.
+__device__ __forceinline__ int bin_pair_f32(const float4 pi, const float4 pj, const PairParams& P,
+                                            int& b0, int& m0) {
+  constexpr float kRound = 12582912.0f;
+  constexpr int kRoundBits = 0x4B400000;
+  const float dx = pj.x - pi.x;
+  const float dy = pj.y - pi.y;
+  const float dz = pj.z - pi.z;
+  const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+  const float rd = rsqrt_approx(d2);
+  const float d = d2 * rd;
+  const float t = fmaf(d, P.f_inv_dr, P.f_t0);
+  const float tr = __fadd_rn(t, kRound);
+  const float tn = __fadd_rn(tr, -kRound);
+  bool near_edge = !(fabsf(t - tn) >= P.tguard);
+  b0 = __float_as_int(tr) - kRoundBits - (t < tn ? 1 : 0);
+  m0 = 0;
+  if (P.rsd) {
+    // s = pi + pj is twice the midpoint m: the factors of 2 cancel in the
+    // cosine th = m.(-d) / (|m| d) and are exact, so th is as with m
+    const float sx = pi.x + pj.x;
+    const float sy = pi.y + pj.y;
+    const float sz = pi.z + pj.z;
+    const float s2 = fmaf(sz, sz, fmaf(sy, sy, sx * sx));
+    const float rs = rsqrt_approx(s2);
+    const float dot = fmaf(sz, -dz, fmaf(sy, -dy, sx * -dx));
+    // u = (th + 1) nmu/2; the mu bins of th and -th mirror each other, so
+    // one guard test covers both
+    const float u = fmaf(dot * (rd * rs), P.f_mu_scale, P.f_mu_scale);
+    const float ur = __fadd_rn(u, kRound);
+    const float un = __fadd_rn(ur, -kRound);
+    // |u - un| < k1 / den + k2 with den = min(d - d0, |m| - mB), times den
+    // (both error terms of the cosine share the smaller denominator)
+    const float den = fminf(d - P.d0, fmaf(0.5f * s2, rs, -P.mB));
+    near_edge = near_edge || !(fabsf(u - un) * den >= fmaf(P.k2, den, P.k1));
+    m0 = __float_as_int(ur) - kRoundBits - (u < un ? 1 : 0);
+  }
+  return near_edge ? 2 : ((unsigned)b0 < (unsigned)P.nbins ? 1 : 0);
+}
+
+// The same with a quick exit for pairs certainly outside (rmin, rmax), and
+// the bins from 1 as edge_f64 gives them.
 __device__ __forceinline__ int classify_f32(const float4 pi, const float4 pj, const PairParams& P,
                                             int& bin, int& muf, int& mur) {
   const float dx = pj.x - pi.x;
@@ -176,51 +231,12 @@ __device__ __forceinline__ int classify_f32(const float4 pi, const float4 pj, co
   const float dz = pj.z - pi.z;
   const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
   if (d2 >= P.rmax2_hi || d2 <= P.rmin2_lo) return 0;
-  // d2 = 0 (coincident points, rmin = 0): t = -rmin/dr, decided in FP64
-  const float d = d2 > 0.0f ? d2 * rsqrtf(d2) : 0.0f;
-  const float t = (d - P.f_rmin) * P.f_inv_dr;
-  const float tn = rintf(t);
-  if (NEED_BINS) {
-    if (fabsf(t - tn) < P.tguard) return 2;
-  } else {
-    if ((tn == 0.0f || tn == (float)P.nbins) && fabsf(t - tn) < P.tguard) return 2;
-  }
-  if (t <= 0.0f || t >= (float)P.nbins) return 0;
-  if (!NEED_BINS) return 1;
-  bin = (int)t + 1;
-  if (P.rsd) {
-    // s = pi + pj is twice the midpoint m: the factors of 2 cancel in the
-    // cosine th = m.(-d) / (|m| d) and are exact, so th is as with m
-    const float dd = d - P.d0;
-    const float sx = pi.x + pj.x;
-    const float sy = pi.y + pj.y;
-    const float sz = pi.z + pj.z;
-    const float s2 = fmaf(sz, sz, fmaf(sy, sy, sx * sx));
-    const float sn = s2 * rsqrtf(s2);
-    const float mmm = fmaf(0.5f, sn, -P.mB);  // |m| - mB
-    // one bound for both error terms: eA/dd + eB/mmm <= (eA + eB)/min(dd, mmm);
-    // __fdividef needs denominators of at least 2^-126
-    const float den = fminf(dd, mmm);
-    if (!(den > 1e-30f) || !(s2 > 0.0f)) return 2;
-    const float dot = fmaf(sz, -dz, fmaf(sy, -dy, sx * -dx));
-    const float th = __fdividef(dot, sn * d);
-    const float eth = __fdividef(P.eA + P.eB, den) + P.eC;
-    const float ug = eth * P.f_mu_scale + 8.0f * 5.96046448e-8f * P.f_nmu;
-    // mu bins of th (root p) and of -th (root q): u2 = (1 - th) nmu/2 is
-    // nmu - u1, so the interior bin edges of u2 are those of u1 mirrored
-    // and one guard test covers both; outside it the bin of -th is
-    // nmu + 1 - (bin of th), also at the clamped ends th = -1 and 1
-    const float u1 = (th + 1.0f) * P.f_mu_scale;
-    const float k1 = rintf(u1);
-    if (k1 >= 1.0f && k1 <= P.f_nmu - 1.0f && fabsf(u1 - k1) < ug) return 2;
-    const int a = (int)floorf(u1) + 1;
-    muf = a < 1 ? 1 : (a > P.nmu ? P.nmu : a);
-    mur = P.nmu + 1 - muf;
-  } else {
-    muf = 1;
-    mur = 1;
-  }
-  return 1;
+  int b0, m0;
+  const int r = bin_pair_f32(pi, pj, P, b0, m0);
+  bin = b0 + 1;
+  muf = m0 + 1;
+  mur = P.nmu - m0;
+  return r;
 }
 
 // Square root for the inversion of the triangular pair index of k members
@@ -282,8 +298,7 @@ __device__ __forceinline__ int edge_rbin(const double4* __restrict__ posd, const
     const float dy = pc.y - pa.y;
     const float dz = pc.z - pa.z;
     const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-    const float d = d2 > 0.0f ? d2 * rsqrtf(d2) : 0.0f;
-    const float t = (d - P.f_rmin) * P.f_inv_dr;
+    const float t = fmaf(d2 * rsqrt_approx(d2), P.f_inv_dr, P.f_t0);
     const float tn = rintf(t);
     if (fabsf(t - tn) >= P.tguard && t > 0.0f && t < (float)P.nbins) return (int)t + 1;
   }
@@ -371,40 +386,35 @@ __device__ __forceinline__ void forward_ranges(int p, int key, const GridParams&
   }
 }
 
-// Forward candidate ranges on a grid of cells at least rmax/2 wide (sub 2):
-// labels from `first` on in the root's own cell and every cell after it in
-// key order within two cells on each axis, as 13 contiguous label ranges in
-// increasing order: the root's x-row up to two cells on (slot 0), the two
-// following rows of its z plane (slots 1-2), and the five rows of each of
-// the next two z planes (slots 3-12).  Lane k of the calling warp (k < 13)
-// returns slot k's [beg, end).
-__device__ __forceinline__ void forward_range2_slot(int k, int first, int key, const GridParams& g,
-                                                    const int* __restrict__ cell_start, int& beg,
-                                                    int& end) {
-  const int cx = key % g.nx;
-  const int cy = (key / g.nx) % g.ny;
-  const int cz = key / (g.nx * g.ny);
-  const int x0 = cx > 1 ? cx - 2 : 0;
-  const int x1 = cx + 2 < g.nx ? cx + 2 : g.nx - 1;
+// Forward candidate ranges of a run of points in the cells x0 .. x1 of one
+// x-row (row yz = y + ny z): labels from `first` on in the cells from the
+// run's own on in key order, within SUB cells on each axis (cells at least
+// rmax/SUB wide), as contiguous label ranges in increasing order.  SUB 1: 5
+// ranges, the rest of the run's row (slot 0), the following row of its z plane
+// and three rows of the next plane; SUB 2: 13, the rest of the row, the two
+// following rows and five rows of each of the next two planes.  Lane k of the
+// calling warp (k < 5 or 13) returns slot k's [beg, end).
+template <int SUB>
+__device__ __forceinline__ void forward_slot(int k, int first, int x0, int x1, int yz,
+                                             const GridParams& g,
+                                             const int* __restrict__ cell_start, int& beg,
+                                             int& end) {
+  const int cy = yz % g.ny;
+  const int cz = yz / g.ny;
+  const int xa = x0 > SUB ? x0 - SUB : 0;
+  const int xb = x1 + SUB < g.nx ? x1 + SUB : g.nx - 1;
+  int y = cy, z = cz;
+  if (k > SUB) {
+    y = cy - SUB + (k - 1 - SUB) % (2 * SUB + 1);
+    z = cz + 1 + (k - 1 - SUB) / (2 * SUB + 1);
+  } else {
+    y = cy + k;
+  }
   int b = 0, e = 0;
-  if (k == 0) {
-    b = first;
-    e = cell_start[key - cx + x1 + 1];
-  } else if (k < 3) {
-    const int y = cy + k;
-    if (y < g.ny) {
-      const int kb = (cz * g.ny + y) * g.nx;
-      b = cell_start[kb + x0];
-      e = cell_start[kb + x1 + 1];
-    }
-  } else if (k < 13) {
-    const int z = cz + 1 + (k - 3) / 5;
-    const int y = cy - 2 + (k - 3) % 5;
-    if (z < g.nz && y >= 0 && y < g.ny) {
-      const int kb = (z * g.ny + y) * g.nx;
-      b = cell_start[kb + x0];
-      e = cell_start[kb + x1 + 1];
-    }
+  if (y >= 0 && y < g.ny && z < g.nz) {
+    const int kb = (z * g.ny + y) * g.nx;
+    b = k == 0 ? first : cell_start[kb + xa];
+    e = cell_start[kb + xb + 1];
   }
   beg = b;
   end = e > b ? e : b;
@@ -515,6 +525,7 @@ struct DevCatalog {
   const int* cell_start; // ncell + 1
   int n;
   int n_data;
+  int has_buffer;        // some points may be buffer points
   GridParams grid;
   // Batched regions: when cell_region is set, cells are grouped by region;
   // region r owns cells [region_cell_off[r], region_cell_off[r+1]) laid out

@@ -50,7 +50,6 @@ size_t pair2_smem_bytes(const PairParams& P, bool weighted);
 // per region, g_cnt nregions*nh and g_fix nregions*2*nh (region r's lo
 // words at 2*r*nh, hi words at 2*r*nh + nh), all zeroed.
 constexpr size_t kMaxTileHistSmem = 160 * 1024;
-size_t pair2_tile_smem_bytes(const PairParams& P, bool weighted);
 void launch_pair2_tile(const DevCatalog& C, const PairParams& P, bool weighted,
                        unsigned long long* g_cnt, unsigned long long* g_fix, double fscale,
                        unsigned long long* stats, int* work, cudaStream_t s,
@@ -101,10 +100,16 @@ int launch_adj3(const DevCatalog& C, const CSRView& G, const TriParams& T, const
 // partials take at most 32 terms each before they are merged, so gscale
 // needs 2^6 of headroom over the largest term: fix_scale(64 * term bound).
 // stats as launch_pair2 (zeroed).
-void launch_adj2_tile(const DevCatalog& C, const PairParams& P, const double* cot2,
-                      const double* cot3, double gscale, unsigned long long* g_lo,
+// coef: the table of pair_coef_table on the device.
+void launch_adj2_tile(const DevCatalog& C, const PairParams& P, const double* coef, double gscale, unsigned long long* g_lo,
                       unsigned long long* g_hi, unsigned long long* stats, int* work,
                       cudaStream_t s);
+// Coefficients of a pair in the 2PCF adjoint (pair_coef) by what the tile
+// sweep knows of it, 4 * nbins * nmu values: entry bin + nbins * mu (from 0)
+// of part 2 * sided + rr, where rr = both points are randoms (cot3 added) and
+// sided = 0: both points are roots, mu seen from either (the other's bin is
+// nmu - 1 - mu); sided = 1: one is, mu seen from it.
+void pair_coef_table(const double* cot2, const double* cot3, int nbins, int nmu, double* coef);
 void launch_grad_finish(int n, const int* orig, const unsigned long long* g_lo,
                         const unsigned long long* g_hi, double gscale, double* grad,
                         cudaStream_t s);

@@ -376,6 +376,7 @@ extern "C" int gr_count_2pcf_noalloc(const double* d_xyz, const double* d_w, int
     C.cell_start = start;
     C.n = ni;
     C.n_data = (int)n_data;
+    C.has_buffer = 0;
     C.grid.nx = g.nc[0];
     C.grid.ny = g.nc[1];
     C.grid.nz = g.nc[2];

@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kPairThreads) pair2_kernel(DevCatalog C, PairP
           int b, mf, mr;
           bool e;
           if (F32) {
-            const int r = classify_f32<true>(pi, s_pos[wib][f], P, b, mf, mr);
+            const int r = classify_f32(pi, s_pos[wib][f], P, b, mf, mr);
             if (r == 2) {
               rechecks++;
               e = edge_f64(C.posd[p], C.posd[q], P, b, mf, mr);
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kPairThreads) pair2_queue_kernel(
     int b = 1, mf = 1, mr = 1;
     bool ok;
     if (F32) {
-      const int r = classify_f32<true>(C.pos4[p], s_pos[wib][f], P, b, mf, mr);
+      const int r = classify_f32(C.pos4[p], s_pos[wib][f], P, b, mf, mr);
       if (r == 2) {
         rechecks++;
         ok = edge_f64(C.posd[p], C.posd[q], P, b, mf, mr);
@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(NT) pair2_dense_kernel(DevCatalog C, PairParam
           int b, mf, mr;
           bool e;
           if (F32) {
-            const int r = classify_f32<true>(pi, s_pos[f], P, b, mf, mr);
+            const int r = classify_f32(pi, s_pos[f], P, b, mf, mr);
             if (r == 2) {
               rechecks++;
               e = edge_f64(C.posd[p], C.posd[s_lab[f]], P, b, mf, mr);
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(NT) pair2_dense_queue_kernel(
     int b = 1, mf = 1, mr = 1;
     bool ok;
     if (F32) {
-      const int r = classify_f32<true>(C.pos4[p], s_pos[f], P, b, mf, mr);
+      const int r = classify_f32(C.pos4[p], s_pos[f], P, b, mf, mr);
       if (r == 2) {
         rechecks++;
         ok = edge_f64(C.posd[p], C.posd[q], P, b, mf, mr);

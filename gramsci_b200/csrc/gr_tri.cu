@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(kTriMaxWarps * 32) tri3_kernel(DevCatalog C, C
     if (GEO) {
       // bins of the edge (a, c) exactly as the graph build computes them
       int b = 1, mf = 1, mr = 1;
-      const int r = T.P.f32 ? classify_f32<true>(s_pos[qx], s_pos[qy], T.P, b, mf, mr) : 2;
+      const int r = T.P.f32 ? classify_f32(s_pos[qx], s_pos[qy], T.P, b, mf, mr) : 2;
       if (r == 2) edge_f64(C.posd[s_col[qx]], C.posd[s_col[qy]], T.P, b, mf, mr);
       mac = pack_meta(b, mf, mr);
     }
