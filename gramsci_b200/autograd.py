@@ -53,8 +53,8 @@ class _PCF(torch.autograd.Function):
     def forward(ctx, w, xyz, n_data, bins, order):
         c = _context(w.device)
         _load(c, w, xyz, n_data, bins)
-        count = {2: c.count_2pcf, 3: c.count_3pcf, 4: c.count_4pcf}[order]
-        out = count()
+        # the sums alone; the integer counts are not returned
+        out = c.count_2pcf() if order == 2 else {3: c.count_3pcf, 4: c.count_4pcf}[order](counts=False)
         ctx.save_for_backward(w, xyz)
         ctx.n_data, ctx.bins, ctx.order = n_data, bins, order
         # the context keeps this catalogue (and its graph) until another

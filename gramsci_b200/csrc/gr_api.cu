@@ -63,6 +63,7 @@ struct gr_ctx {
   CellIndex index;
   UpperCSR csr;
   bool csr_valid = false;
+  bool index_valid = false;  // index: the current catalogue and bins on rmax-wide cells
   int clique_mode = 0;  // GR_OPT_CLIQUE_MODE
   // speculative rebuilds (count_tri): catalogue generation (set_catalog),
   // generation of the last verified build, and whether speculating on a new
@@ -74,6 +75,7 @@ struct gr_ctx {
   PairParams P{};
   DevBuf<uint8_t> normal_dev;
   int normal_nmu = 0;                     // nmu of the table in normal_dev (0: none)
+  bool normal_asym = false;               // that table is not symmetric
   DevBuf<unsigned long long> hcnt, dcnt, stats;
   DevBuf<unsigned long long> hfix, dfix;  // fixed-point sums (lo words, then hi words)
   double wmax = 0.0;                      // max |w| over the catalogue
@@ -83,6 +85,10 @@ struct gr_ctx {
   HostBuf<unsigned long long> stage;     // pinned read-back of a call's results
   DevBuf<double> hval;                   // fixed-point sums converted on the device
   DevBuf<int> qorder;                    // 4-clique root order (n) + its class counts
+  DevBuf<int> long_list;                 // 3PCF: roots with rows beyond a warp's capacity
+  DevBuf<float4> row_pos;                // their rows (second launch)
+  DevBuf<double> row_w;
+  DevBuf<int> row_q, row_id;
   SpecGraph spec_graph;                  // captured speculative rebuild (count_tri)
   SpecGraph spec_index;                  // captured speculative index (gr_count_2pcf)
   DevBuf<double> cot, grad;              // adjoint inputs / output
@@ -263,6 +269,10 @@ static void ensure_normal(gr_ctx* c, int nmu, cudaStream_t s) {
   if (c->normal_nmu == nmu && c->normal_dev.p) return;
   std::vector<uint8_t> nt;
   normal_table(nmu, nt);
+  c->normal_asym = false;
+  for (int a = 0; a < nmu; ++a)
+    for (int b = 0; b < a; ++b)
+      if (nt[a + (size_t)nmu * b] != nt[b + (size_t)nmu * a]) c->normal_asym = true;
   c->normal_dev.reserve(nt.size());
   GR_CUDA_TRY(cudaMemcpyAsync(c->normal_dev.p, nt.data(), nt.size(), cudaMemcpyHostToDevice, s));
   GR_CUDA_TRY(cudaStreamSynchronize(s));  // nt is pageable and goes out of scope
@@ -495,16 +505,21 @@ void set_pair_params(gr_ctx* c, double coord_max) {
 void restore_index(gr_ctx* c) {
   c->index.n_data = c->n_data;
   c->index.has_buffer = c->has_buffer ? 1 : 0;
+  c->index.speculated = true;
   set_pair_params(c, c->index.coord_max);
   c->csr_valid = false;
+  c->index_valid = false;
 }
 
 void build_index(gr_ctx* c, bool speculate = false, int sub = 1) {
   cudaStream_t s = c->stream();
+  c->csr_valid = false;
+  c->index_valid = false;
   c->index.build(c->xyz.p, c->w.p, c->has_buffer ? c->buffer.p : nullptr, c->n, c->n_data, c->rmax, s,
                  speculate, sub, kDenseCellPoints);
   set_pair_params(c, c->index.coord_max);
-  c->csr_valid = false;
+  // a speculative index is valid once its flag has been read
+  c->index_valid = !c->index.speculated && c->index.grid.sub == 1;
 }
 
 void build_csr(gr_ctx* c, bool speculate = false) {
@@ -515,6 +530,10 @@ void build_csr(gr_ctx* c, bool speculate = false) {
 // The index and graph of the last call (or of gr_graph_load) are current and
 // may be reused by this call.
 bool reuse_graph(const gr_ctx* c) { return c->csr_valid && (c->keep_graph || c->graph_loaded); }
+// The same for a call that needs the index alone.
+bool reuse_index(const gr_ctx* c) {
+  return (c->csr_valid || c->index_valid) && (c->keep_graph || c->graph_loaded);
+}
 
 int round_cap(int64_t maxdeg, int lo, int hi) {
   int64_t c = ((maxdeg + 31) / 32) * 32;
@@ -777,6 +796,7 @@ static int set_catalog_impl(gr_ctx* c, const double* xyz, const double* w, const
   c->w_ran = wr;
   c->cat_set = true;
   c->csr_valid = false;
+  c->index_valid = false;
   c->graph_loaded = false;
   c->regions.valid = false;
   // region ids and mocks describe the points of the previous catalogue
@@ -812,6 +832,7 @@ int gr_set_bins(gr_ctx* c, double rmin, double rmax, int32_t nbins, int32_t nmu,
   c->logbins = logbins ? 1 : 0;
   c->bins_set = true;
   c->csr_valid = false;
+  c->index_valid = false;
   c->graph_loaded = false;
   c->regions.valid = false;
   GR_API_END(c)
@@ -823,6 +844,7 @@ int gr_set_option(gr_ctx* c, int32_t key, int64_t value) {
     if (value != 0 && value != 1) return set_err(c, GR_E_ARG, "precision must be 0 or 1");
     if (c->precision != (int)value) {
       c->csr_valid = false;
+      c->index_valid = false;
       c->graph_loaded = false;
       c->regions.valid = false;
       c->regions.release_graph();
@@ -1060,14 +1082,61 @@ static const int* root_order(gr_ctx* c, cudaStream_t s, const int** above = null
   return c->qorder.p;
 }
 
-// Third-edge test of the triangle kernel: the geometric pair test unless the
-// hash probes are forced.  Measured: 3PCF catalogue with 5 mu bins and upper
-// degree 13.7, 0.743 ms geometric against 0.754 ms (the FP32 binning of the
-// re-tested third edges with approximate square root and division; 0.78
-// against 0.75 ms with correctly rounded ones); without mu bins 0.56
-// against 0.64 ms; upper degree 156, 197 against 250 ms with 5 mu bins.
-static int tri_geometric(const gr_ctx* c) {
-  return c->clique_mode == 1 ? 0 : 1;
+// The triangle kernels' number of points per unit volume is taken from the
+// catalogue's box.
+static double box_volume(const CatalogBox& b) {
+  return (b.hi[0] - b.lo[0]) * (b.hi[1] - b.lo[1]) * (b.hi[2] - b.lo[2]);
+}
+
+// Parameters of the rooted triangle kernel (find_normal table uploaded,
+// pair parameters set); n points lie in `volume`.
+static RootParams root_params(gr_ctx* c, bool equi, int ncfg, int64_t n, double volume) {
+  RootParams T{};
+  T.nbins = c->nbins;
+  T.nmu = c->nmu;
+  T.ncfg = ncfg;
+  T.rsd = c->nmu >= 2;
+  T.equi = equi ? 1 : 0;
+  T.asym = c->normal_asym ? 1 : 0;
+  root3_plan(T, n, volume, c->rmax);
+  T.normal = c->normal_dev.p;
+  make_rank_tables(T.rank, c->nbins, 3);
+  T.P = c->P;
+  return T;
+}
+
+constexpr int kRootStats = 9;  // statistics of launch_root3
+
+// The second launch of the rooted kernel, for the rows the first one listed
+// (st: its statistics on the host).
+static RootLong long_rows(gr_ctx* c, const unsigned long long* st) {
+  RootLong R{};
+  R.n = (int)st[6];
+  R.cap = (int)std::min<unsigned long long>(st[8], 0x7fffffffull);
+  // a block per root, a few per SM, the rows of all blocks within about 1 GB
+  const int64_t fit = std::max<int64_t>(1, ((int64_t)1 << 30) / ((int64_t)R.cap * 32));
+  R.blocks = (int)std::min<int64_t>({(int64_t)R.n, 4 * (int64_t)sm_count(), fit});
+  const size_t entries = (size_t)R.blocks * R.cap;
+  c->row_pos.reserve(entries);
+  c->row_w.reserve(entries);
+  c->row_q.reserve(entries);
+  c->row_id.reserve(entries);
+  R.pos = c->row_pos.p;
+  R.w = c->row_w.p;
+  R.q = c->row_q.p;
+  R.id = c->row_id.p;
+  return R;
+}
+
+// Statistics of a call from those of the rooted kernel.
+static void root_stats(gr_ctx* c, const unsigned long long* st) {
+  c->st.tuples = (int64_t)st[0];
+  c->st.rooted = (int64_t)st[1];
+  c->st.probes = (int64_t)st[2];
+  c->st.upper_edges = (int64_t)st[3];
+  c->st.n_edges = 2 * c->st.upper_edges;
+  c->st.candidates = (int64_t)st[4];
+  c->st.fp64_rechecks = (int64_t)st[5];
 }
 
 static int count_tri(gr_ctx* c, bool equi, double* N2, double* N3, int64_t* counts, double* catsum) {
@@ -1080,46 +1149,61 @@ static int count_tri(gr_ctx* c, bool equi, double* N2, double* N3, int64_t* coun
   const int nbin = ncfg * nmu, nh = nbin * 4;
   const bool weighted = !c->uniform;
   const bool want_counts = counts != nullptr || !weighted;
+  // GR_OPT_CLIQUE_MODE 1: the triangles from the neighbour graph, third edges
+  // by hash probes of its rows; else the rooted kernel on the index alone
+  const bool hash = c->clique_mode == 1;
   double fscale[4];
   for (int nr = 0; nr < 4; ++nr)
     fscale[nr] = fix_scale(std::pow(c->wgmax, 3 - nr) * std::pow(c->wrmax, nr));
   c->hcnt.reserve(nh);
   c->hfix.reserve(2 * nh);
-  c->stats.reserve(8);
+  c->stats.reserve(kRootStats);
   ensure_normal(c, nmu, s);
-  const bool reuse = reuse_graph(c);
+  const bool reuse = hash ? reuse_graph(c) : reuse_index(c);
   // A rebuild of a catalogue seen before runs without waiting on the host:
-  // the grid is taken from the last bounding box, the graph is filled in the
-  // scratch area as it is, and the triangle kernel's row capacity is taken
-  // from the last graph (longer rows take its global-memory path, so any
+  // the grid is taken from the last bounding box and, for the hash probes, the
+  // graph is filled in the scratch area as it is and the kernel's row capacity
+  // taken from the last graph (longer rows take its global-memory path, so any
   // capacity gives the same result).  A device flag records a changed
   // bounding box and the graph build one that ran out of room; both are
   // read with the results, and the call is then repeated with waits.
   const bool can_spec =
       !reuse && c->index.have_prev && (c->cat_gen == c->spec_gen || c->spec_new_ok);
   // read-back layout in the pinned stage: counts (nh), the sums converted
-  // on the device (nh doubles), kernel stats (8), graph control (4) and
-  // stats (3), bbox flag (1)
-  c->stage.reserve(2 * (size_t)nh + 16);
+  // on the device (nh doubles), kernel stats, graph control (4) and stats
+  // (3), bbox flag (1)
+  c->stage.reserve(2 * (size_t)nh + kRootStats + 8);
   c->hval.reserve(nh);
   unsigned long long* hc = c->stage.p;
   double* hv = reinterpret_cast<double*>(hc + nh);
   unsigned long long* st = hc + 2 * (size_t)nh;
-  unsigned long long* gctl = st + 8;
+  unsigned long long* gctl = st + kRootStats;
   unsigned long long* gsts = gctl + 4;
   unsigned long long* gflag = gsts + 3;
   std::vector<double> hs(nh, 0.0);
   cudaEvent_t q0 = c->ev[4];  // owned by the context
   c->work.reserve(4);
+  if (!hash) c->long_list.reserve(c->n + 1);
   int tri_launches = 0;
   std::vector<unsigned long long> key;
   bool replayed = false;
+  // results to the stage
+  auto read_back = [&]() {
+    if (want_counts)
+      GR_CUDA_TRY(cudaMemcpyAsync(hc, c->hcnt.p, sizeof(unsigned long long) * nh, cudaMemcpyDeviceToHost, s));
+    if (weighted) {
+      enqueue_fix_convert(c->hfix.p, nh, nh, nbin, fscale, false, c->hval.p, s);
+      GR_CUDA_TRY(cudaMemcpyAsync(hv, c->hval.p, sizeof(double) * nh, cudaMemcpyDeviceToHost, s));
+    }
+    GR_CUDA_TRY(cudaMemcpyAsync(st, c->stats.p, sizeof(unsigned long long) * kRootStats,
+                                cudaMemcpyDeviceToHost, s));
+  };
   for (int attempt = 0; attempt < 2; ++attempt) {
     const bool spec = can_spec && attempt == 0;
     bool replay = false;
     if (spec) {
-      key = spec_key(c, 1, true);
-      replay = c->spec_graph.idx && c->spec_graph.csr && key == c->spec_graph.key;
+      key = spec_key(c, 1, hash);
+      replay = c->spec_graph.idx && (c->spec_graph.csr || !hash) && key == c->spec_graph.key;
     }
     replayed = replay;
     GR_CUDA_TRY(cudaEventRecord(c->ev[0], s));
@@ -1132,7 +1216,7 @@ static int count_tri(gr_ctx* c, bool equi, double* N2, double* N3, int64_t* coun
       }
     }
     GR_CUDA_TRY(cudaEventRecord(c->ev[1], s));
-    if (!reuse) {
+    if (!reuse && hash) {
       if (replay) {
         GR_CUDA_TRY(cudaGraphLaunch(c->spec_graph.csr, s));
         c->csr.compacted = false;
@@ -1145,66 +1229,76 @@ static int count_tri(gr_ctx* c, bool equi, double* N2, double* N3, int64_t* coun
       ZeroList z;
       z.add(c->hcnt.p, sizeof(unsigned long long) * nh);
       z.add(c->hfix.p, sizeof(unsigned long long) * 2 * nh);
-      z.add(c->stats.p, sizeof(unsigned long long) * 8);
+      z.add(c->stats.p, sizeof(unsigned long long) * kRootStats);
       zero_async(z, s);
     }
-    TriParams T{};
-    T.nbins = c->nbins;
-    T.nmu = nmu;
-    T.ncfg = ncfg;
-    T.rsd = nmu >= 2;
-    T.equi = equi ? 1 : 0;
-    T.cap = round_cap(c->csr.max_deg, 32, 256);
-    T.normal = c->normal_dev.p;
-    make_rank_tables(T.rank, c->nbins, 3);
-    for (int nr = 0; nr < 4; ++nr) T.fscale[nr] = fscale[nr];
-    T.P = c->P;
-    T.geo = tri_geometric(c);
-    T.maxdeg = (int)std::min<int64_t>(c->csr.max_deg, 1 << 30);
-    T.long_geo = c->clique_mode != 1;
-    const CSRView G = c->csr.view();
     GR_CUDA_TRY(cudaEventRecord(q0, s));
-    tri_launches = 1 + launch_tri3(c->index.view(), G, T, weighted, want_counts, c->hcnt.p,
-                                   c->hfix.p, c->stats.p, c->work.p, s);  // + the zero fill
-    GR_CUDA_TRY(cudaEventRecord(c->ev[3], s));
-    if (want_counts)
-      GR_CUDA_TRY(cudaMemcpyAsync(hc, c->hcnt.p, sizeof(unsigned long long) * nh, cudaMemcpyDeviceToHost, s));
-    if (weighted) {
-      enqueue_fix_convert(c->hfix.p, nh, nh, nbin, fscale, false, c->hval.p, s);
-      GR_CUDA_TRY(cudaMemcpyAsync(hv, c->hval.p, sizeof(double) * nh, cudaMemcpyDeviceToHost, s));
+    RootParams RT{};
+    if (hash) {
+      TriParams T{};
+      T.nbins = c->nbins;
+      T.nmu = nmu;
+      T.ncfg = ncfg;
+      T.rsd = nmu >= 2;
+      T.equi = equi ? 1 : 0;
+      T.cap = round_cap(c->csr.max_deg, 32, 256);
+      T.normal = c->normal_dev.p;
+      make_rank_tables(T.rank, c->nbins, 3);
+      for (int nr = 0; nr < 4; ++nr) T.fscale[nr] = fscale[nr];
+      launch_tri3(c->index.view(), c->csr.view(), T, weighted, want_counts, c->hcnt.p, c->hfix.p,
+                  c->stats.p, c->work.p, s);
+    } else {
+      RT = root_params(c, equi, ncfg, c->n, box_volume(c->index.box));
+      for (int nr = 0; nr < 4; ++nr) RT.fscale[nr] = fscale[nr];
+      launch_root3(c->index.view(), RT, weighted, want_counts, c->hcnt.p, c->hfix.p, c->stats.p,
+                   c->work.p, c->long_list.p, nullptr, s);
     }
-    GR_CUDA_TRY(cudaMemcpyAsync(st, c->stats.p, sizeof(unsigned long long) * 8, cudaMemcpyDeviceToHost, s));
+    tri_launches = 2;  // with the zero fill
+    GR_CUDA_TRY(cudaEventRecord(c->ev[3], s));
+    read_back();
     std::memset(gctl, 0, sizeof(unsigned long long) * 8);
-    if (spec) {
+    const bool speculated = spec && c->index.speculated;
+    if (spec && hash) {
       GR_CUDA_TRY(cudaMemcpyAsync(gctl, c->csr.ctl.p, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost, s));
       GR_CUDA_TRY(cudaMemcpyAsync(gsts, c->csr.stats.p, sizeof(unsigned long long) * 3, cudaMemcpyDeviceToHost, s));
-      if (c->index.speculated)
-        GR_CUDA_TRY(cudaMemcpyAsync(gflag, c->index.mismatch_flag(), sizeof(unsigned long long),
-                                    cudaMemcpyDeviceToHost, s));
     }
+    if (speculated)
+      GR_CUDA_TRY(cudaMemcpyAsync(gflag, c->index.mismatch_flag(), sizeof(unsigned long long),
+                                  cudaMemcpyDeviceToHost, s));
     GR_CUDA_TRY(cudaStreamSynchronize(s));
     if (spec) {
       if (*gflag != 0 || gctl[1] == 1) {  // repeat with waits
         if (c->cat_gen != c->spec_gen) c->spec_new_ok = false;
         continue;
       }
-      c->csr.settle(gctl, gsts);
-      c->csr_valid = true;
+      if (hash) {
+        c->csr.settle(gctl, gsts);
+        c->csr_valid = true;
+      }
       // a speculative build that needed no second pass: keep it as graphs
       // for the next call of the same configuration
-      if (!replayed) {
-        capture_spec_graph(c, c->spec_graph, 1, true);
-        c->csr_valid = true;
-        c->csr.settle(gctl, gsts);
+      if (!replayed && (hash || speculated)) {
+        capture_spec_graph(c, c->spec_graph, 1, hash);
+        if (hash) {
+          c->csr_valid = true;
+          c->csr.settle(gctl, gsts);
+        }
       }
+      c->index_valid = true;
+    }
+    if (!hash && st[6] > 0) {
+      const RootLong R = long_rows(c, st);
+      launch_root3(c->index.view(), RT, weighted, want_counts, c->hcnt.p, c->hfix.p, c->stats.p,
+                   c->work.p, c->long_list.p, &R, s);
+      tri_launches++;
+      GR_CUDA_TRY(cudaEventRecord(c->ev[3], s));
+      read_back();
+      GR_CUDA_TRY(cudaStreamSynchronize(s));
+      if (st[7] != 0) throw gr::Error{GR_E_CUDA, "3PCF: a row exceeds its own bound"};
     }
     break;
   }
   if (!reuse) c->spec_gen = c->cat_gen;
-  // graph statistics are on the host after the build (or the load)
-  const unsigned long long gst[3] = {(unsigned long long)c->csr.rechecks,
-                                     (unsigned long long)c->csr.candidates,
-                                     (unsigned long long)c->csr.max_deg};
   if (weighted)
     for (int k = 0; k < nh; ++k) hs[k] = hv[k];
   if (!weighted) {
@@ -1228,15 +1322,19 @@ static int count_tri(gr_ctx* c, bool equi, double* N2, double* N3, int64_t* coun
   c->st.ms_query = ev_ms(q0, c->ev[3]);
   c->st.ms_total = c->st.ms_index + c->st.ms_graph + c->st.ms_query;
   c->st.n_points = c->n;
-  c->st.n_edges = 2 * c->csr.n_edges;
-  c->st.tuples = (int64_t)st[0];
-  c->st.rooted = (int64_t)st[1];
-  c->st.probes = (int64_t)st[2];
-  c->st.upper_edges = c->csr.n_edges;
-  c->st.fp64_rechecks = (int64_t)gst[0];
-  c->st.candidates = (int64_t)gst[1];
-  c->st.kernel_launches =
-      (reuse ? 0 : c->index.launches + c->csr.launches) + tri_launches + (weighted ? 1 : 0);
+  if (hash) {
+    c->st.n_edges = 2 * c->csr.n_edges;
+    c->st.tuples = (int64_t)st[0];
+    c->st.rooted = (int64_t)st[1];
+    c->st.probes = (int64_t)st[2];
+    c->st.upper_edges = c->csr.n_edges;
+    c->st.fp64_rechecks = c->csr.rechecks;
+    c->st.candidates = c->csr.candidates;
+  } else {
+    root_stats(c, st);
+  }
+  c->st.kernel_launches = (reuse ? 0 : c->index.launches + (hash ? c->csr.launches : 0)) +
+                          tri_launches + (weighted ? 1 : 0);
   GR_API_END(c)
 }
 
@@ -1865,49 +1963,68 @@ int gr_adjoint_3pcf(gr_ctx* c, const double* cot2, const double* cot3, double* g
   const int nc = ncfg * nmu;
   const int64_t n = c->n;
   const double cmax = max_abs(cot2, nc) + max_abs(cot3, nc);
-  // 2^10 below the per-term bound: the kernel sums up to 1023 terms of one
-  // root per neighbour in signed 64 bits before the 128-bit totals
-  const double gscale = fix_scale(3.0 * cmax * c->wmax * c->wmax * 1024.0);
+  const bool hash = c->clique_mode == 1;
+  // largest term; with 2^10 of headroom where up to 1023 terms of one root
+  // are summed per neighbour in signed 64 bits before the 128-bit totals
+  const double gscale =
+      fix_scale(3.0 * cmax * c->wmax * c->wmax * (hash || nmu >= 2 ? 1024.0 : 1.0));
   ensure_normal(c, nmu, s);
   c->cot.reserve(2 * nc);
   c->gfix.reserve(2 * n + 2);
   c->work.reserve(4);
-  c->stats.reserve(8);
+  c->stats.reserve(kRootStats);
   GR_CUDA_TRY(cudaMemcpyAsync(c->cot.p, cot2, sizeof(double) * nc, cudaMemcpyHostToDevice, s));
   if (cot3)
     GR_CUDA_TRY(cudaMemcpyAsync(c->cot.p + nc, cot3, sizeof(double) * nc, cudaMemcpyHostToDevice, s));
   GR_CUDA_TRY(cudaEventRecord(c->ev[0], s));
-  const bool rebuilt = !c->csr_valid;
+  const bool rebuilt = hash ? !c->csr_valid : !(c->csr_valid || c->index_valid);
   if (rebuilt) {
     build_index(c);
-    build_csr(c);
+    if (hash) build_csr(c);
   }
   GR_CUDA_TRY(cudaEventRecord(c->ev[1], s));
   GR_CUDA_TRY(cudaMemsetAsync(c->gfix.p, 0, sizeof(unsigned long long) * (2 * n + 2), s));
-  GR_CUDA_TRY(cudaMemsetAsync(c->stats.p, 0, sizeof(unsigned long long) * 8, s));
-  TriParams T{};
-  T.nbins = c->nbins;
-  T.nmu = nmu;
-  T.ncfg = ncfg;
-  T.rsd = nmu >= 2;
-  T.cap = round_cap(c->csr.max_deg, 32, 256);
-  T.normal = c->normal_dev.p;
-  make_rank_tables(T.rank, c->nbins, 3);
-  T.P = c->P;
-  T.geo = c->clique_mode == 1 ? 0 : 1;  // faster for the adjoint at every degree measured
-  T.maxdeg = (int)std::min<int64_t>(c->csr.max_deg, 1 << 30);
-  T.long_geo = c->clique_mode != 1;
-  const CSRView G = c->csr.view();
+  GR_CUDA_TRY(cudaMemsetAsync(c->stats.p, 0, sizeof(unsigned long long) * kRootStats, s));
+  const double* dc3 = cot3 ? c->cot.p + nc : nullptr;
   std::memset(&c->st, 0, sizeof(c->st));
-  launch_adj3(c->index.view(), G, T, c->cot.p, cot3 ? c->cot.p + nc : nullptr, gscale, c->gfix.p,
-              c->gfix.p + n, c->stats.p, c->work.p, s);
-  finish_grad(c, gscale, grad_w, c->ev[1]);
+  if (hash) {
+    TriParams T{};
+    T.nbins = c->nbins;
+    T.nmu = nmu;
+    T.ncfg = ncfg;
+    T.rsd = nmu >= 2;
+    T.cap = round_cap(c->csr.max_deg, 32, 256);
+    T.normal = c->normal_dev.p;
+    make_rank_tables(T.rank, c->nbins, 3);
+    launch_adj3(c->index.view(), c->csr.view(), T, c->cot.p, dc3, gscale, c->gfix.p, c->gfix.p + n,
+                c->stats.p, c->work.p, s);
+    finish_grad(c, gscale, grad_w, c->ev[1]);
+    c->st.n_edges = 2 * c->csr.n_edges;
+    c->st.upper_edges = c->csr.n_edges;
+  } else {
+    c->long_list.reserve(n + 1);
+    c->stage.reserve(kRootStats);
+    const RootParams T = root_params(c, false, ncfg, n, box_volume(c->index.box));
+    auto run = [&](const RootLong* R) {
+      launch_root3_adj(c->index.view(), T, c->cot.p, dc3, gscale, c->gfix.p, c->gfix.p + n,
+                       c->stats.p, c->work.p, c->long_list.p, R, s);
+      GR_CUDA_TRY(cudaMemcpyAsync(c->stage.p, c->stats.p, sizeof(unsigned long long) * kRootStats,
+                                  cudaMemcpyDeviceToHost, s));
+      finish_grad(c, gscale, grad_w, c->ev[1]);
+    };
+    run(nullptr);
+    const unsigned long long* st = c->stage.p;
+    if (st[6] > 0) {
+      const RootLong R = long_rows(c, st);
+      run(&R);
+    }
+    if (st[7] != 0) throw gr::Error{GR_E_CUDA, "3PCF: a row exceeds its own bound"};
+    root_stats(c, st);
+  }
   c->st.ms_graph = rebuilt ? ev_ms(c->ev[0], c->ev[1]) : 0.0;
   c->st.ms_total = c->st.ms_graph + c->st.ms_query;
   c->st.n_points = n;
-  c->st.n_edges = 2 * c->csr.n_edges;
-  c->st.upper_edges = c->csr.n_edges;
-  c->st.kernel_launches = (rebuilt ? c->index.launches + c->csr.launches : 0) + 2;
+  c->st.kernel_launches = (rebuilt ? c->index.launches + (hash ? c->csr.launches : 0) : 0) + 2;
   GR_API_END(c)
 }
 
@@ -2226,47 +2343,67 @@ int gr_count_3pcf_batched(gr_ctx* c, double* N2, double* N3, int64_t* counts, do
                                      : fix_scale(std::pow(c->wgmax, 3 - nr) * std::pow(c->wrmax, nr));
   c->hcnt.reserve(nh);
   c->hfix.reserve(2 * nh);
-  c->stats.reserve(8);
+  c->stats.reserve(kRootStats);
   c->work.reserve(4);
   ensure_normal(c, nmu, s);
   c->regions.enqueue_layout(c->xyz.p, c->w.p, s, planned);
   const DevCatalog RC = c->regions.view();
+  const bool hash = c->clique_mode == 1;
   GR_CUDA_TRY(cudaEventRecord(c->ev[1], s));
-  c->csr.build(RC, c->P, s);
-  c->csr_valid = false;  // the graph of the region members, not of the catalogue
+  if (hash) {
+    c->csr.build(RC, c->P, s);
+    c->csr_valid = false;  // the graph of the region members, not of the catalogue
+  }
   GR_CUDA_TRY(cudaEventRecord(c->ev[2], s));
   {
     ZeroList z;
     z.add(c->hcnt.p, sizeof(unsigned long long) * nh);
     z.add(c->hfix.p, sizeof(unsigned long long) * 2 * nh);
-    z.add(c->stats.p, sizeof(unsigned long long) * 8);
+    z.add(c->stats.p, sizeof(unsigned long long) * kRootStats);
     zero_async(z, s);
   }
-  TriParams T{};
-  T.nbins = c->nbins;
-  T.nmu = nmu;
-  T.ncfg = ncfg;
-  T.rsd = nmu >= 2;
-  T.equi = 0;
-  T.cap = round_cap(c->csr.max_deg, 32, 256);
-  T.normal = c->normal_dev.p;
-  make_rank_tables(T.rank, c->nbins, 3);
-  for (int nr = 0; nr < 4; ++nr) T.fscale[nr] = fscale[nr];
-  T.P = c->P;
-  T.geo = tri_geometric(c);
-  T.maxdeg = (int)std::min<int64_t>(c->csr.max_deg, 1 << 30);
-  T.long_geo = c->clique_mode != 1;
-  const int tri_launches = 1 + launch_tri3(RC, c->csr.view(), T, weighted, true, c->hcnt.p,
-                                           c->hfix.p, c->stats.p, c->work.p, s);
-  GR_CUDA_TRY(cudaEventRecord(c->ev[3], s));
   std::vector<unsigned long long> hc(nh), hf(2 * nh, 0ull);
   std::vector<double> hs(nh, 0.0);
-  unsigned long long st[8];
-  GR_CUDA_TRY(cudaMemcpyAsync(hc.data(), c->hcnt.p, sizeof(unsigned long long) * nh, cudaMemcpyDeviceToHost, s));
-  if (weighted)
-    GR_CUDA_TRY(cudaMemcpyAsync(hf.data(), c->hfix.p, sizeof(unsigned long long) * 2 * nh, cudaMemcpyDeviceToHost, s));
-  GR_CUDA_TRY(cudaMemcpyAsync(st, c->stats.p, sizeof(st), cudaMemcpyDeviceToHost, s));
-  GR_CUDA_TRY(cudaStreamSynchronize(s));
+  unsigned long long st[kRootStats];
+  auto read_back = [&]() {
+    GR_CUDA_TRY(cudaEventRecord(c->ev[3], s));
+    GR_CUDA_TRY(cudaMemcpyAsync(hc.data(), c->hcnt.p, sizeof(unsigned long long) * nh, cudaMemcpyDeviceToHost, s));
+    if (weighted)
+      GR_CUDA_TRY(cudaMemcpyAsync(hf.data(), c->hfix.p, sizeof(unsigned long long) * 2 * nh, cudaMemcpyDeviceToHost, s));
+    GR_CUDA_TRY(cudaMemcpyAsync(st, c->stats.p, sizeof(st), cudaMemcpyDeviceToHost, s));
+    GR_CUDA_TRY(cudaStreamSynchronize(s));
+  };
+  if (hash) {
+    TriParams T{};
+    T.nbins = c->nbins;
+    T.nmu = nmu;
+    T.ncfg = ncfg;
+    T.rsd = nmu >= 2;
+    T.cap = round_cap(c->csr.max_deg, 32, 256);
+    T.normal = c->normal_dev.p;
+    make_rank_tables(T.rank, c->nbins, 3);
+    for (int nr = 0; nr < 4; ++nr) T.fscale[nr] = fscale[nr];
+    launch_tri3(RC, c->csr.view(), T, weighted, true, c->hcnt.p, c->hfix.p, c->stats.p, c->work.p, s);
+    read_back();
+  } else {
+    c->long_list.reserve(RC.n + 1);
+    // mocks overlap: each has its share of the points
+    RootParams T = root_params(c, false, ncfg,
+                               c->region_mode == 3 ? c->n / std::max(1, c->regions.nreg) : c->n,
+                               c->regions.volume);
+    for (int nr = 0; nr < 4; ++nr) T.fscale[nr] = fscale[nr];
+    auto run = [&](const RootLong* R) {
+      launch_root3(RC, T, weighted, true, c->hcnt.p, c->hfix.p, c->stats.p, c->work.p,
+                   c->long_list.p, R, s);
+      read_back();
+    };
+    run(nullptr);
+    if (st[6] > 0) {
+      const RootLong R = long_rows(c, st);
+      run(&R);
+    }
+    if (st[7] != 0) throw gr::Error{GR_E_CUDA, "3PCF: a row exceeds its own bound"};
+  }
   if (weighted) {
     for (int k = 0; k < nh; ++k) hs[k] = fix_value(hf[k], hf[nh + k], fscale[k / nbin]);
   } else {
@@ -2289,14 +2426,18 @@ int gr_count_3pcf_batched(gr_ctx* c, double* N2, double* N3, int64_t* counts, do
   c->st.ms_query = ev_ms(c->ev[2], c->ev[3]);
   c->st.ms_total = ev_ms(c->ev[0], c->ev[3]);
   c->st.n_points = c->regions.n_members;
-  c->st.n_edges = 2 * c->csr.n_edges;
-  c->st.upper_edges = c->csr.n_edges;
-  c->st.tuples = (int64_t)st[0];
-  c->st.rooted = (int64_t)st[1];
-  c->st.probes = (int64_t)st[2];
-  c->st.fp64_rechecks = c->csr.rechecks;
-  c->st.candidates = c->csr.candidates;
-  c->st.kernel_launches = c->csr.launches + tri_launches + 9;
+  if (hash) {
+    c->st.n_edges = 2 * c->csr.n_edges;
+    c->st.upper_edges = c->csr.n_edges;
+    c->st.tuples = (int64_t)st[0];
+    c->st.rooted = (int64_t)st[1];
+    c->st.probes = (int64_t)st[2];
+    c->st.fp64_rechecks = c->csr.rechecks;
+    c->st.candidates = c->csr.candidates;
+  } else {
+    root_stats(c, st);
+  }
+  c->st.kernel_launches = (hash ? c->csr.launches : 0) + 2 + 9;
   GR_API_END(c)
 }
 

@@ -354,9 +354,8 @@ __global__ void b_gather_kernel(int64_t m, const int* __restrict__ perm,
     const int i = m_orig[k];
     const double x = xyz[3 * (int64_t)i], y = xyz[3 * (int64_t)i + 1], z = xyz[3 * (int64_t)i + 2];
     const uint8_t f = m_flag[k];
-    // the fourth component marks buffer points (pair sweeps skip pairs of two)
     pos4[p] = make_float4(__double2float_rn(x), __double2float_rn(y), __double2float_rn(z),
-                          (f & FLAG_BUFFER) ? 1.f : 0.f);
+                          pos4_flags(f));
     posd[p] = make_double4(x, y, z, w[i]);
     wl[p] = w[i];
     orig[p] = i;
@@ -412,8 +411,10 @@ void RegionLayout::plan(const double* d_xyz, int64_t n_pts, int64_t n_data_pts,
   count.reserve(nreg);
   SplitGeom sg;
   sg.ns = ns;
+  volume = 1.0;
   for (int d = 0; d < 3; ++d) {
     const double span = box.hi[d] - box.lo[d];
+    volume *= span;
     sg.lo[d] = cat_lo[d] = box.lo[d];
     sg.inv_span[d] = cat_inv_span[d] = span > 0 ? 1.0 / span : 0.0;
     reach[d] = span > 0 ? rmax * ns / span * (1.0 + 1e-6) + 1e-6 : 2.0;

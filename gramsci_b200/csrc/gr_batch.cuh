@@ -43,6 +43,7 @@ struct RegionLayout {
   int ns = 0, nreg = 0;
   int64_t n = 0, n_data = 0, n_members = 0, ncell = 0;
   double rmax = 0.0;
+  double volume = 0.0;  // of the catalogue's box
   // host geometry
   std::vector<double> h_halo, h_glo, h_ginv;
   std::vector<GridParams> h_grid;

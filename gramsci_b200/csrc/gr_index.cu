@@ -154,9 +154,8 @@ __global__ void cell_order_gather_kernel(int64_t ncell, const int64_t* __restric
       const double wi = w[i];
       uint8_t f = (i >= n_data) ? FLAG_RANDOM : 0;
       if (buffer && buffer[i] == 1) f |= FLAG_BUFFER;
-      // the fourth component marks buffer points (pair sweeps skip pairs of two)
       pos4[p] = make_float4(__double2float_rn(x), __double2float_rn(y), __double2float_rn(z),
-                            (f & FLAG_BUFFER) ? 1.0f : 0.0f);
+                            pos4_flags(f));
       posd[p] = make_double4(x, y, z, wi);
       wl[p] = wi;
       orig[p] = i;
@@ -255,7 +254,7 @@ void CellIndex::build(const double* d_xyz, const double* d_w, const int* d_buffe
     GR_CUDA_TRY(cudaMemcpyAsync(bbox_prev.p, prev_raw, sizeof(prev_raw), cudaMemcpyHostToDevice, s));
     GR_CUDA_TRY(cudaMemsetAsync(bbox_prev.p + 7, 0, sizeof(unsigned long long), s));
   }
-  const CatalogBox box = box_of_keys(h, n);
+  box = box_of_keys(h, n);
   coord_max = box.coord_max;
   // cells at least rmax (sub 2: rmax/2) wide; the cell table stays O(N)
   GridGeom g;

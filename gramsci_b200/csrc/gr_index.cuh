@@ -11,11 +11,20 @@
 
 namespace gr {
 
+// Bounding box of a catalogue and its largest |coordinate| (all zero without
+// points), read back with one wait; raises on non-finite coordinates.
+struct CatalogBox {
+  double lo[3], hi[3], coord_max;
+};
+CatalogBox catalog_box(const double* d_xyz, int64_t n, DevBuf<unsigned long long>& raw,
+                       cudaStream_t s);
+
 // Uniform-grid index over the catalogue, points laid out in cell order.
 struct CellIndex {
   int64_t n = 0, n_data = 0;
   int has_buffer = 0;
   double coord_max = 0.0;  // max |coordinate|, bounds the FP32 rounding error
+  CatalogBox box{};        // the box the grid was laid over
   GridParams grid{};
   int launches = 0;
   DevBuf<unsigned long long> bbox_raw;
@@ -48,14 +57,6 @@ struct CellIndex {
   const unsigned long long* mismatch_flag() const { return bbox_prev.p + 7; }
   DevCatalog view() const;
 };
-
-// Bounding box of a catalogue and its largest |coordinate| (all zero without
-// points), read back with one wait; raises on non-finite coordinates.
-struct CatalogBox {
-  double lo[3], hi[3], coord_max;
-};
-CatalogBox catalog_box(const double* d_xyz, int64_t n, DevBuf<unsigned long long>& raw,
-                       cudaStream_t s);
 
 // Upper adjacency: row p lists the neighbours q > p (internal labels) of the
 // (rmin, rmax) graph in increasing label order, with packed bin / mu

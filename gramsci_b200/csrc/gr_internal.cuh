@@ -114,10 +114,10 @@ __device__ __forceinline__ int mu_bin_f64(double th, const PairParams& P) {
   return m;
 }
 
-// Exact reference predicate in FP64 (separate IEEE multiply / add, no FMA),
-// root pi, neighbour pj.  Identical arithmetic to the CPU oracle.
-__device__ __forceinline__ bool edge_f64(const double4 pi, const double4 pj, const PairParams& P,
-                                         int& bin, int& muf, int& mur) {
+// Exact reference membership and radial bin in FP64 (separate IEEE multiply /
+// add, no FMA), the same from either end.
+__device__ __forceinline__ bool edge_radial_f64(const double4 pi, const double4 pj,
+                                                const PairParams& P, int& bin) {
   double dx = __dsub_rn(pj.x, pi.x);
   double dy = __dsub_rn(pj.y, pi.y);
   double dz = __dsub_rn(pj.z, pi.z);
@@ -137,6 +137,14 @@ __device__ __forceinline__ bool edge_f64(const double4 pi, const double4 pj, con
   b = b > P.nbins ? P.nbins : b;
   b = b < 1 ? 1 : b;
   bin = b;
+  return true;
+}
+
+// The whole reference predicate in FP64, root pi, neighbour pj.  Identical
+// arithmetic to the CPU oracle.
+__device__ __forceinline__ bool edge_f64(const double4 pi, const double4 pj, const PairParams& P,
+                                         int& bin, int& muf, int& mur) {
+  if (!edge_radial_f64(pi, pj, P, bin)) return false;
   if (P.rsd) {
     double m0 = __dmul_rn(0.5, __dadd_rn(pi.x, pj.x));
     double m1 = __dmul_rn(0.5, __dadd_rn(pi.y, pj.y));
@@ -266,7 +274,7 @@ __device__ __forceinline__ int pair_row_biased(int k2m1, int t) {
   return (int)(0.5f * ((float)k2m1 - pair_index_sqrt(disc)) + 2.5e-4f);
 }
 
-// Both points of a pair are buffer points (pos4.w = 1 marks them): the pair
+// Both points of a pair are buffer points (see pos4_flags): the pair
 // has no root and adds nothing to any 2PCF histogram or gradient, so the
 // pair sweeps skip it before testing it.  (The neighbour graph keeps such
 // edges: they close triangles and 4-cliques rooted elsewhere.)
@@ -516,7 +524,7 @@ __device__ __forceinline__ int meta_mur(uint32_t m) { return (int)((m >> 16) & 0
 // Points in cell order ("internal labels").  orig[p] is the position in the
 // reference's catalogue order; random = orig >= n_data.
 struct DevCatalog {
-  const float4* pos4;    // float x, y, z, (unused)
+  const float4* pos4;    // float x, y, z, flags (pos4_flags)
   const double4* posd;   // double x, y, z, w
   const double* w;       // weight
   const int* orig;       // original index
@@ -552,6 +560,15 @@ __device__ __forceinline__ void cell_grid(const DevCatalog& C, int cell, GridPar
 }
 
 enum : uint8_t { FLAG_RANDOM = 1, FLAG_BUFFER = 2 };
+
+// The flags in the fourth component of pos4: 1 for a buffer point and 0 for
+// another (pair sweeps compare it with 0), its sign bit for a random.
+__device__ __forceinline__ float pos4_flags(uint8_t f) {
+  return __int_as_float(((f & FLAG_BUFFER) ? 0x3f800000 : 0) |
+                        ((f & FLAG_RANDOM) ? (int)0x80000000u : 0));
+}
+__device__ __forceinline__ bool pos4_random(const float4& p) { return __float_as_int(p.w) < 0; }
+__device__ __forceinline__ bool pos4_buffer(const float4& p) { return p.w != 0.0f; }
 
 // 2PCF weight adjoint: coefficient of the pair (p, q) in dL/dw, the
 // cotangents of the bins the pair lands in from each non-buffer end (cot3

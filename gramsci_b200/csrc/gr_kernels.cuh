@@ -65,11 +65,6 @@ struct TriParams {
   const uint8_t* normal;   // device find_normal table [mu1-1 + nmu*(mu2-1)]
   RankTables rank;         // 3-tuple ranks
   double fscale[4];        // fixed-point scale of the products with 0..3 randoms
-  PairParams P;            // edge predicate and binning of the graph
-  int geo;                 // 1: third edges by the geometric pair test, 0: hash probes of rows
-  int maxdeg;              // longest upper row
-  int long_geo;            // 1: rows beyond cap take a second, geometric launch
-  int kmin, kskip;         // roots handled by one launch: kmin < row length <= kskip
 };
 
 // 3PCF: triangles p < a < c enumerated once over the upper CSR; each adds to
@@ -78,11 +73,51 @@ struct TriParams {
 // words, weighted only) must be zeroed.  stats: [0] distinct triangles binned, [1] rooted
 // incidences, [2] intersection probes.
 // work: one device int used as the dynamic root counter (reset by the launch).
-// Returns the number of kernel launches (2 when long rows take a second one).
-size_t tri3_smem_bytes(const TriParams& T, bool weighted, bool counts);
-int launch_tri3(const DevCatalog& C, const CSRView& G, const TriParams& T, bool weighted,
+void launch_tri3(const DevCatalog& C, const CSRView& G, const TriParams& T, bool weighted,
                  bool counts, unsigned long long* g_cnt, unsigned long long* g_lim,
                  unsigned long long* stats, int* work, cudaStream_t s);
+
+// Rooted triangle kernel (gr_root.cu): the 3PCF and its adjoint straight from
+// a cell index of rmax-wide cells, without a neighbour graph.
+struct RootParams {
+  int nbins, nmu, ncfg, rsd;
+  int equi;               // -equi: only triangles with three equal bins, ncfg = nbins
+  int asym;               // the find_normal table is not symmetric
+  int cap;                // wanted row capacity of a warp; longer rows are listed
+  int group;              // roots taken together, at most
+  int chunk;              // roots per work-counter increment
+  const uint8_t* normal;  // device find_normal table [mu1-1 + nmu*(mu2-1)]
+  RankTables rank;        // 3-tuple ranks
+  double fscale[4];       // fixed-point scale of the products with 0..3 randoms
+  PairParams P;
+};
+// Second launch for the listed rows: n of them, at most cap members each, in
+// global memory, blocks * cap entries per array.
+struct RootLong {
+  int n, cap, blocks;
+  float4* pos;
+  double* w;
+  int *q, *id;
+};
+// cap, group and chunk for a catalogue of n points in a volume.
+void root3_plan(RootParams& T, int64_t n, double volume, double rmax);
+// g_cnt (nh = ncfg*nmu*4, when counts) and g_lim (2*nh: 128-bit fixed-point
+// sums, lo words then hi words, weighted only) must be zeroed, stats (9
+// entries) too.  stats: [0] distinct triangles with a root, [1] rooted
+// triangles, [2] pairs tested, [3] edges, [4] candidates, [5] FP64 evaluations
+// of root edges, [6] rows listed in
+// long_list (n entries), [7] set when a listed row exceeds the capacity of the
+// second launch, [8] the longest listed row's bound.  The caller runs the
+// second launch (R) when rows were listed; it adds to the same outputs.
+void launch_root3(const DevCatalog& C, const RootParams& T, bool weighted, bool counts,
+                  unsigned long long* g_cnt, unsigned long long* g_lim, unsigned long long* stats,
+                  int* work, int* long_list, const RootLong* R, cudaStream_t s);
+// The weight adjoint (see launch_adj3) into g_lo / g_hi (zeroed, label order);
+// with mu bins gscale needs 2^10 of headroom over the largest term.
+void launch_root3_adj(const DevCatalog& C, const RootParams& T, const double* cot2,
+                      const double* cot3, double gscale, unsigned long long* g_lo,
+                      unsigned long long* g_hi, unsigned long long* stats, int* work,
+                      int* long_list, const RootLong* R, cudaStream_t s);
 
 // Weight adjoints: gradient of sum(cot2 * N2) + sum(cot3 * N3) with respect
 // to the weights, as 128-bit fixed-point sums (g_lo, g_hi, label order; the
@@ -92,7 +127,7 @@ int launch_tri3(const DevCatalog& C, const CSRView& G, const TriParams& T, bool 
 void launch_adj2(const DevCatalog& C, const PairParams& P, const double* cot2, const double* cot3,
                  double gscale, unsigned long long* g_lo, unsigned long long* g_hi, int* work,
                  cudaStream_t s, int variant = kPairWarpCell);
-int launch_adj3(const DevCatalog& C, const CSRView& G, const TriParams& T, const double* cot2,
+void launch_adj3(const DevCatalog& C, const CSRView& G, const TriParams& T, const double* cot2,
                  const double* cot3, double gscale, unsigned long long* g_lo,
                  unsigned long long* g_hi, unsigned long long* stats, int* work, cudaStream_t s);
 // The same adjoint with the tile sweep (gr_tile.cu): half stencil, both ends

@@ -205,7 +205,8 @@ __global__ void na_gather_kernel(int n, int n_data, const int* __restrict__ perm
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
     const int i = perm[p];
     const double x = xyz[3 * (int64_t)i], y = xyz[3 * (int64_t)i + 1], z = xyz[3 * (int64_t)i + 2];
-    pos4[p] = make_float4(__double2float_rn(x), __double2float_rn(y), __double2float_rn(z), 0.f);
+    pos4[p] = make_float4(__double2float_rn(x), __double2float_rn(y), __double2float_rn(z),
+                          pos4_flags(i >= n_data ? FLAG_RANDOM : 0));
     posd[p] = make_double4(x, y, z, w[i]);
     wl[p] = w[i];
     orig[p] = i;

@@ -169,15 +169,17 @@ __global__ void __launch_bounds__(kTileThreads, (ADJ && SUB == 2) ? 4 : GR_TILE_
   // A point's code.  Tables: the part of a pair's entry that the point
   // contributes, its sign bit a buffer root (the pair is then seen from the
   // candidate).  One update per root, adjoint: its flags.
-  auto root_code = [&](uint8_t f) -> int {
-    if (ADJ || rooted) return (int)f;
-    const int r = f & FLAG_RANDOM;
-    return (f & FLAG_BUFFER) ? (int)(0x80000000u | (unsigned)(nbm * r + (nt - nh)))
-                             : 2 * nbm * r;
+  auto flag_code = [&](const float4& c) -> int {
+    return (pos4_random(c) ? FLAG_RANDOM : 0) | (pos4_buffer(c) ? FLAG_BUFFER : 0);
   };
-  auto cand_code = [&](uint8_t f) -> int {
-    if (ADJ || rooted) return (int)f;
-    return nbm * (f & FLAG_RANDOM) + ((f & FLAG_BUFFER) ? nt - nh : 0);
+  auto root_code = [&](const float4& c) -> int {
+    if (ADJ || rooted) return flag_code(c);
+    const int r = pos4_random(c) ? 1 : 0;
+    return pos4_buffer(c) ? (int)(0x80000000u | (unsigned)(nbm * r + (nt - nh))) : 2 * nbm * r;
+  };
+  auto cand_code = [&](const float4& c) -> int {
+    if (ADJ || rooted) return flag_code(c);
+    return (pos4_random(c) ? nbm : 0) + (pos4_buffer(c) ? nt - nh : 0);
   };
 
   auto flush = [&]() {
@@ -273,8 +275,8 @@ __global__ void __launch_bounds__(kTileThreads, (ADJ && SUB == 2) ? 4 : GR_TILE_
       float4 pi = C.pos4[act ? p : c0];  // idle lanes: the first root again
       double4 pd = make_double4(0.0, 0.0, 0.0, 0.0);
       if (!F32 && act) pd = C.posd[p];
-      const bool pbuf = pi.w != 0.0f;
-      T.root[lane] = make_float4(pi.x, pi.y, pi.z, __int_as_float(act ? root_code(C.flags[p]) : 0));
+      const bool pbuf = pos4_buffer(pi);
+      T.root[lane] = make_float4(pi.x, pi.y, pi.z, __int_as_float(root_code(pi)));
       if (act && (WEIGHTED || ADJ)) T.wr[lane] = C.w[p];
       // the roots' bounding box; candidates farther than rmax from it (with
       // the guard band) and, when every root is a buffer point, buffer
@@ -307,7 +309,7 @@ __global__ void __launch_bounds__(kTileThreads, (ADJ && SUB == 2) ? 4 : GR_TILE_
             while (kr + 1 < NR && f >= T.rpre[kr + 1]) ++kr;
             q = T.rb[kr] + (f - T.rpre[kr]);
             c = C.pos4[q];
-            qbuf = c.w != 0.0f;
+            qbuf = pos4_buffer(c);
             const float ex = fmaxf(fmaxf(blx - c.x, c.x - bhx), 0.f);
             const float ey = fmaxf(fmaxf(bly - c.y, c.y - bhy), 0.f);
             const float ez = fmaxf(fmaxf(blz - c.z, c.z - bhz), 0.f);
@@ -327,7 +329,7 @@ __global__ void __launch_bounds__(kTileThreads, (ADJ && SUB == 2) ? 4 : GR_TILE_
               T.z[at] = cd.z;
             }
             T.q[at] = q;
-            T.code[at] = cand_code(C.flags[q]);
+            T.code[at] = cand_code(c);
             if (WEIGHTED || ADJ) T.wq[at] = C.w[q];
           }
           nacc += __popc(kept);
