@@ -1347,12 +1347,12 @@ int gr_count_equi(gr_ctx* c, double* N2, double* N3, int64_t* counts, double* ca
 }
 
 // Edges among R+(p) in the 4-clique kernels: the geometric pair test (rows
-// up to 256 members) or hash probes of the members' rows.  Measured on the
+// up to 255 members) or hash probes of the members' rows.  Measured on the
 // 4PCF workload (upper degree 17.5): unit weights 5.0 ms geometric against
 // 6.3 ms, lognormal weighted sums 9.8 against 10.8 ms, adjoint 13.0 against
 // 15.3 ms.
-static int quad_geometric(const gr_ctx* c, int cap, int nbins) {
-  return (cap > 256 || nbins > 255 || c->clique_mode == 1) ? 0 : 1;
+static int quad_geometric(const gr_ctx* c, int64_t max_deg, int nbins) {
+  return (max_deg > 255 || nbins > 255 || c->clique_mode == 1) ? 0 : 1;
 }
 
 static int count_quad(gr_ctx* c, bool tetra, double* N2, double* N3, double* discN, double* discR,
@@ -1411,7 +1411,8 @@ static int count_quad(gr_ctx* c, bool tetra, double* N2, double* N3, double* dis
   Q.cap = round_cap((int64_t)gst[2], 32, 1024);
   make_rank_tables(Q.rank, nb, 4);
   Q.P = c->P;
-  Q.geo = quad_geometric(c, Q.cap, nb);
+  Q.geo = quad_geometric(c, c->csr.max_deg, nb);
+  Q.mean_row = (int)(c->csr.n_edges / std::max<int64_t>(1, c->n));
   const CSRView G = c->csr.view();
   cudaEvent_t q0 = c->ev[4];  // owned by the context
   GR_CUDA_TRY(cudaEventRecord(q0, s));
@@ -2047,12 +2048,9 @@ int gr_adjoint_4pcf(gr_ctx* c, const double* cot2, const double* cot3, const dou
   const double c4 = max_abs(cot2, nbin) + max_abs(cot3, nbin);
   const double cd = max_abs(cotN, 6 * (int64_t)nbin) + max_abs(cotR, 6 * (int64_t)nbin);
   const double gscale = fix_scale(4.0 * (c4 * w * w * w + 3.0 * cd * w));
-  std::vector<double> cot((size_t)14 * nbin, 0.0);
-  std::memcpy(cot.data(), cot2, sizeof(double) * nbin);
-  if (cot3) std::memcpy(cot.data() + nbin, cot3, sizeof(double) * nbin);
-  if (cotN) std::memcpy(cot.data() + 2 * (size_t)nbin, cotN, sizeof(double) * 6 * nbin);
-  if (cotR) std::memcpy(cot.data() + 8 * (size_t)nbin, cotR, sizeof(double) * 6 * nbin);
-  c->cot.reserve(14 * (int64_t)nbin);
+  std::vector<double> cot((size_t)kCotLine * nbin);
+  quad_cot_lines(cot2, cot3, cotN, cotR, nbin, cot.data());
+  c->cot.reserve(cot.size());
   c->gfix.reserve(2 * n + 2);
   c->work.reserve(4);
   c->stats.reserve(8);
@@ -2076,7 +2074,8 @@ int gr_adjoint_4pcf(gr_ctx* c, const double* cot2, const double* cot3, const dou
   Q.cap = round_cap(c->csr.max_deg, 32, 1024);
   make_rank_tables(Q.rank, nb, 4);
   Q.P = c->P;
-  Q.geo = quad_geometric(c, Q.cap, nb);
+  Q.geo = quad_geometric(c, c->csr.max_deg, nb);
+  Q.mean_row = (int)(c->csr.n_edges / std::max<int64_t>(1, c->n));
   std::memset(&c->st, 0, sizeof(c->st));
   Q.order = root_order(c, s, &Q.above, &Q.nclass);
   launch_adj4(c->index.view(), c->csr.view(), Q, c->cot.p, gscale, c->gfix.p, c->gfix.p + n,

@@ -171,6 +171,8 @@ struct QuadParams {
   const int* above;  // with order: above[b] = the number of roots whose row
                      // length class (min(length, nclass - 1)) exceeds b, or null
   int nclass;
+  int mean_row;     // average row length
+  int long_warps, short_cap;  // set by the launch (quadg_shape)
 };
 
 // -tetra histograms (tetra = 1): g_cnt nbins*5, d_cnt nbins*30 (6 terms x 5
@@ -205,9 +207,17 @@ constexpr int kQuadPatterns = 16;
 void quad_expand_patterns(const unsigned long long* H, int nbin, unsigned long long* hc,
                           unsigned long long* dc);
 // 4PCF adjoint: gradient of sum(cot2 N2) + sum(cot3 N3) + sum(cotN discN)
-// + sum(cotR discR), cot = [cot2 nbin | cot3 nbin | cotN 6 nbin | cotR 6 nbin]
-// (nbin = ncfg nbins^2), into g_lo / g_hi (label order, zeroed) at scale
-// gscale.  Q as for launch_quad4 with tetra = 0.
+// + sum(cotR discR) into g_lo / g_hi (label order, zeroed) at scale gscale; cot:
+// the lines of quad_cot_lines on the device.  Q as for launch_quad4 with
+// tetra = 0.
+//
+// One 128-byte line of cotangents per histogram index (nbin = ncfg nbins^2 of
+// them, kCotLine doubles each): cot2; cot2 + cot3; the six cotN; the six
+// cotN + cotR.  A root of a clique reads up to seven of them, which as 14
+// separate arrays lay on as many lines.
+constexpr int kCotLine = 16;
+void quad_cot_lines(const double* cot2, const double* cot3, const double* cotN,
+                    const double* cotR, int nbin, double* out);
 void launch_adj4(const DevCatalog& C, const CSRView& G, const QuadParams& Q, const double* cot,
                  double gscale, unsigned long long* g_lo, unsigned long long* g_hi,
                  unsigned long long* stats, int* work, cudaStream_t s);

@@ -38,64 +38,89 @@ constexpr int kQuadMaxWarpsU = 24;  // unweighted kernels (up to 85 registers)
 #define GR_QUADG_WEIGHTED_WARPS 24
 #endif
 // Weighted geometric kernel: 24 warps (at most 85 registers, a few bytes
-// spilled) measured 4.47 ms on the 4PCF workload against 4.64 ms at 20,
-// 5.04 ms at 16 (106 registers), 4.84 ms at 28 and 5.29 ms at 32 (spills)
-// once its sums had a line per bin; before that the reductions, not the
-// warps, bounded it.  (The high limb in the
-// low limb's line instead of a line of its own: 4.58 ms.)
+// spilled).  (The high limb of a sum in the low limb's line instead of a line of
+// its own made the kernel 2% slower.)
 constexpr int kQuadGWarpsW = GR_QUADG_WEIGHTED_WARPS;
-// Geometric adjoint kernel: 24 warps (at most 85 registers, ~50 bytes
-// spilled) measured 6.13 ms on the 4PCF workload against 6.67 ms at 20 and
-// 7.27 ms at 16 (116 registers), identical gradients.
+// Geometric adjoint kernel: 24 warps too (13 warps: 5.5 against 3.2 ms).
 constexpr int kQuadGWarpsA = 24;
 constexpr size_t kQuadSmemLimit = 227 * 1024;
 constexpr int kQQueue = 96;         // hit queue entries per warp (< 32 left + 64 pushed)
 constexpr int kQMaxOffset = 1 << 22;  // hash entries: (label offset << 10) | position
 constexpr uint8_t kFlagDeg4 = 4;    // staged flag: full row length > 3 (a reference root)
 // The longest rows (a root's cost grows with the cube of its row length) are
-// handed out as kSplitParts work items each, every item staging the root in
-// full and taking every kSplitParts-th share of its cliques: a heavy root on
-// one warp otherwise ends the launch alone (measured on the 4PCF workload:
-// one SM busy for 8.0M cycles while the others were done after 5.1M).  The
-// split roots are the longest ones, at least kSplitRow long, few enough that
-// their items fill at most a quarter of the launch's warps (measured on the
-// 4PCF workload, unit weights: 2.98 ms at an eighth, 2.64 ms at a quarter,
-// 2.62 ms at a half; 16 items per root: 3.01 ms).
-constexpr int kSplitRow = 32;
-constexpr int kSplitParts = 8;
+// handed out as several work items each, every item staging the root in full
+// and taking its share of the member pairs (geometric kernel) or of the first
+// members (hash kernel): a heavy root on one warp otherwise ends the launch
+// alone.  A row of 32 is one unit of work; longer ones take about as many
+// parts as they have units, by the classes below, where the launch's warps
+// outnumber the rows to split (in catalogues with more such rows than warps
+// the shares would only repeat the staging).
+constexpr int kSplitClasses = 5;
+__host__ __device__ constexpr int split_row(int j) {
+  return j == 0 ? 128 : (j == 1 ? 96 : (j == 2 ? 64 : (j == 3 ? 48 : 32)));
+}
+__host__ __device__ constexpr int split_parts(int j) {
+  return j == 0 ? 64 : (j == 1 ? 32 : (j == 2 ? 16 : (j == 3 ? 4 : 2)));
+}
 
-// The root and part of work item `item` (QuadParams::order / nheavy).
-// Items [0, nheavy * parts) are the parts of the heavy roots, then one item
-// per remaining root.  Returns false past the last root.
-__device__ __forceinline__ bool quad_item(const QuadParams& Q, int n, int item, int nh, int parts,
-                                          int& p, int& part) {
-  int slot;
-  part = 0;
-  if (item < nh * parts) {
-    slot = item / parts;
-    part = item - slot * parts;
-  } else {
-    slot = nh + (item - nh * parts);
+// A window of slots (places in QuadParams::order): all rows, or, when some of
+// a block's warps take the long ones (QuadParams::long_warps), those of at
+// least kShortRow members (phase 0) or the others (phase 1); end[j]: slots
+// before which rows of split class j end, relative to start.
+constexpr int kShortRow = 64;
+struct QuadWindow {
+  int start, stop, end[kSplitClasses];
+};
+__device__ __forceinline__ QuadWindow quad_window(const QuadParams& Q, int n, int phase) {
+  QuadWindow W;
+  W.start = 0;
+  W.stop = n;
+#pragma unroll
+  for (int j = 0; j < kSplitClasses; ++j) W.end[j] = 0;
+  if (!Q.order || !Q.above) return W;
+  // above[b]: the number of rows with at least b members
+  if (Q.long_warps > 0) {
+    const int nlong = Q.above[kShortRow];
+    if (phase == 0)
+      W.stop = nlong;
+    else
+      W.start = nlong;
   }
-  if (slot >= n) return false;
+  const int limit = (int)gridDim.x * (int)(blockDim.x >> 5);
+#pragma unroll
+  for (int j = 0; j < kSplitClasses; ++j)
+    if (split_row(j) < Q.nclass)
+      W.end[j] = max(0, min(min(Q.above[split_row(j)], W.stop) - W.start, limit));
+  return W;
+}
+// The root, part and number of parts of work item `item`; false past the
+// last root.
+__device__ __forceinline__ bool quad_item(const QuadParams& Q, const QuadWindow& W, int item,
+                                          int& p, int& part, int& nparts) {
+  int slot = 0, first = 0;  // first slot of the class, and its first item
+  part = 0;
+  nparts = 1;
+  bool done = false;
+#pragma unroll
+  for (int j = 0; j < kSplitClasses; ++j) {
+    const int rows = W.end[j] - slot, items = rows * split_parts(j);
+    if (!done && item < first + items) {
+      const int i = (item - first) / split_parts(j);
+      part = item - first - i * split_parts(j);
+      nparts = split_parts(j);
+      slot += i;
+      done = true;
+    }
+    if (!done) {
+      slot = W.end[j];
+      first += items;
+    }
+  }
+  if (!done) slot += item - first;
+  slot += W.start;
+  if (slot >= W.stop) return false;
   p = Q.order ? Q.order[slot] : slot;
   return true;
-}
-__device__ __forceinline__ int quad_split_parts(const QuadParams& Q, int& nh) {
-  nh = 0;
-  if (!Q.order || !Q.above || Q.nclass <= kSplitRow) return 1;
-  const int limit = (int)gridDim.x * (int)(blockDim.x >> 5) / (4 * kSplitParts);
-  // above[] does not increase with b: the smallest b >= kSplitRow - 1 with
-  // above[b] <= limit
-  int lo = kSplitRow - 1, hi = Q.nclass - 1;
-  if (Q.above[hi] > limit) return 1;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (Q.above[mid] <= limit) hi = mid;
-    else lo = mid + 1;
-  }
-  nh = Q.above[lo];
-  return nh > 0 ? kSplitParts : 1;
 }
 
 __host__ __device__ inline size_t qalign8(size_t x) { return (x + 7) & ~(size_t)7; }
@@ -152,8 +177,7 @@ struct QuadCtx {
   int counts;                       // 0: weighted sums only, no integer counts
   double fscale;  // scale of the 4-point products
   double dscale;  // scale of the pair products of the disconnected terms
-  // adjoint: cotangents of N2, N3 (nbin each), discN, discR (6 nbin each)
-  const double *c2, *c3, *cN, *cR;
+  const double* cot;  // adjoint: a line of cotangents per histogram index (quad_cot_lines)
 };
 
 // Logical entry i of a global fixed-point array: one entry per kFixStride
@@ -367,17 +391,37 @@ __device__ __forceinline__ unsigned id_order(const QVerts& V) {
   return a0 | (a1 << 2) | (a2 << 4) | (a3 << 6);
 }
 
-// Gradient of the cotangent-weighted sums with respect to the four vertex
-// weights of one clique (g[v] = d/dw_v, vertices as in quad_contrib).  The
-// sums are multilinear: a 4-product contributes its cotangent times the
-// product of the other three weights, a pair term its cotangent times the
-// partner's weight.  The valid roots' cotangents are gathered into one
-// 4-product coefficient c4 and one coefficient per clique edge D[e] (edges
-// 0 (0,1) 1 (0,2) 2 (0,3) 3 (1,2) 4 (1,3) 5 (2,3)); the roots are a loop
-// that is not unrolled (fully unrolled, the gradient code overflowed the
-// instruction cache).
+// Gradient of one root's cotangent-weighted sums with respect to the weights
+// of its four roles (0 = root, 1..3 = the other vertices in catalogue-id
+// order; rb: whether each is a random): the sums are multilinear, so the
+// 4-product contributes its cotangent times the product of the other three
+// weights, a pair term its cotangent times the partner's weight.  Both
+// 4-clique kernels round these four numbers to the fixed point, so their
+// gradients are identical.
+__device__ __forceinline__ void quad_root_grad(const QuadCtx& X, int kr, const unsigned rb[4],
+                                               const double w[4], double g[4]) {
+  const double* c = X.cot + (size_t)kr * kCotLine;
+  const double c4 = __ldg(c + (rb[0] && rb[1] && rb[2] && rb[3] ? 1 : 0));
+  double D[6];
+#pragma unroll
+  for (int tt = 0; tt < 6; ++tt) {
+    D[tt] = 0.0;
+    if (rb[term_gate(tt)]) D[tt] = __ldg(c + (rb[term_pu(tt)] && rb[term_pv(tt)] ? 8 : 2) + tt);
+  }
+  // terms: 0 (0,1) 1 (0,2) 2 (0,3) 3 (1,2) 4 (3,2) 5 (3,1)
+  g[0] = c4 * (w[1] * w[2] * w[3]) + D[0] * w[1] + D[1] * w[2] + D[2] * w[3];
+  g[1] = c4 * (w[0] * w[2] * w[3]) + D[0] * w[0] + D[3] * w[2] + D[5] * w[3];
+  g[2] = c4 * (w[0] * w[1] * w[3]) + D[1] * w[0] + D[3] * w[1] + D[4] * w[3];
+  g[3] = c4 * (w[0] * w[1] * w[2]) + D[2] * w[0] + D[5] * w[1] + D[4] * w[2];
+}
+
+// The weight gradient of one clique (vertices as in quad_contrib) from each
+// of its valid roots: vertex 0's to racc, the others' to the accumulators at
+// positions ya, yb, yd.  The roots are a loop that is not unrolled (unrolled,
+// the code overflowed the instruction cache).  Returns the number of roots.
 __device__ __forceinline__ int quad_grad_c(const QuadCtx& X, const QVerts& V, const uint32_t m[6],
-                                           double g[4]) {
+                                           double gscale, Fix128& racc, unsigned* s_grad, int gcap,
+                                           int ya, int yb, int yd) {
   unsigned long long packed = 0;
 #pragma unroll
   for (int e = 0; e < 6; ++e) packed |= (unsigned long long)meta_bin(m[e]) << (8 * e);
@@ -387,9 +431,7 @@ __device__ __forceinline__ int quad_grad_c(const QuadCtx& X, const QVerts& V, co
     rndm |= (unsigned)(V.fl[k] & FLAG_RANDOM) << k;
     flw |= (unsigned)V.fl[k] << (8 * k);
   }
-  const int nr = __popc(rndm);
   const unsigned perm = id_order(V);
-  double c4 = 0.0, D[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   int n = 0;
 #pragma unroll 1
   for (int R = 0; R < 4; ++R) {
@@ -411,27 +453,24 @@ __device__ __forceinline__ int quad_grad_c(const QuadCtx& X, const QVerts& V, co
     const int d1 = qbin(packed, R, u1), d2 = qbin(packed, u0, u2);
     const int kk = (cfg - 1) + X.ncfg * ((d1 - 1) + X.nbins * (d2 - 1));
     ++n;
-    c4 += __ldg(&X.c2[kk]) + (nr == 4 ? __ldg(&X.c3[kk]) : 0.0);
-    const unsigned rp = (unsigned)R | ((unsigned)u0 << 2) | ((unsigned)u1 << 4) | ((unsigned)u2 << 6);
+    const int v[4] = {R, u0, u1, u2};
+    unsigned rb[4];
+    double w[4], g[4];
 #pragma unroll
-    for (int tt = 0; tt < 6; ++tt) {
-      const int ga = (int)((rp >> (2 * term_gate(tt))) & 3u);
-      if (!((rndm >> ga) & 1u)) continue;
-      const int u = (int)((rp >> (2 * term_pu(tt))) & 3u), vv = (int)((rp >> (2 * term_pv(tt))) & 3u);
-      const int kt = kk + X.nbin * tt;
-      const bool both = ((rndm >> u) & 1u) && ((rndm >> vv) & 1u);
-      const double cd = __ldg(&X.cN[kt]) + (both ? __ldg(&X.cR[kt]) : 0.0);
-      const int e = qedge(u, vv);
+    for (int j = 0; j < 4; ++j) {
+      rb[j] = (rndm >> v[j]) & 1u;
+      w[j] = qsel(v[j], V);
+    }
+    quad_root_grad(X, kk, rb, w, g);
 #pragma unroll
-      for (int ee = 0; ee < 6; ++ee)
-        if (ee == e) D[ee] += cd;
+    for (int j = 0; j < 4; ++j) {
+      if (v[j] == 0)
+        fix_acc(racc, g[j], gscale);
+      else
+        smem_fix_add(s_grad + (v[j] == 1 ? ya : (v[j] == 2 ? yb : yd)), gcap,
+                     __double2ll_rn(g[j] * gscale));
     }
   }
-  const double w0 = V.w[0], w1 = V.w[1], w2 = V.w[2], w3 = V.w[3];
-  g[0] = c4 * (w1 * w2 * w3) + D[0] * w1 + D[1] * w2 + D[2] * w3;
-  g[1] = c4 * (w0 * w2 * w3) + D[0] * w0 + D[3] * w2 + D[4] * w3;
-  g[2] = c4 * (w0 * w1 * w3) + D[1] * w0 + D[3] * w1 + D[5] * w3;
-  g[3] = c4 * (w0 * w1 * w2) + D[2] * w0 + D[4] * w1 + D[5] * w2;
   return n;
 }
 
@@ -474,10 +513,7 @@ __device__ __forceinline__ void quad_setup(QuadCtx& X, const QuadParams& Q, unsi
   }
   X.fscale = fscale;
   X.dscale = dscale;
-  X.c2 = cot;
-  X.c3 = ADJ ? cot + X.nbin : nullptr;
-  X.cN = ADJ ? cot + 2 * (size_t)X.nbin : nullptr;
-  X.cR = ADJ ? cot + 8 * (size_t)X.nbin : nullptr;
+  X.cot = cot;
 }
 
 // Weighted 4PCF contributions of the warp's cliques, flattened: every lane
@@ -593,15 +629,7 @@ __device__ __forceinline__ int quad_emit(const QuadCtx& X, const QVerts& V, cons
                                          double gscale, Fix128& racc, unsigned* s_grad, int gcap,
                                          int ya, int yb, int yd) {
   if constexpr (ADJ) {
-    double g[4];
-    const int nroot = quad_grad_c(X, V, m, g);
-    if (nroot) {
-      fix_acc(racc, g[0], gscale);
-      smem_fix_add(s_grad + ya, gcap, __double2ll_rn(g[1] * gscale));
-      smem_fix_add(s_grad + yb, gcap, __double2ll_rn(g[2] * gscale));
-      smem_fix_add(s_grad + yd, gcap, __double2ll_rn(g[3] * gscale));
-    }
-    return nroot;
+    return quad_grad_c(X, V, m, gscale, racc, s_grad, gcap, ya, yb, yd);
   } else if constexpr (TETRA) {
     return tetra_contrib<WEIGHTED, SHC>(X, V, m);
   } else {
@@ -673,15 +701,13 @@ __global__ void __launch_bounds__((WEIGHTED || ADJ ? kQuadMaxWarps : kQuadMaxWar
     return hit ? (int)(e & 0x3ffu) : -1;
   };
 
-  int nheavy;
-  const int parts = quad_split_parts(Q, nheavy);
+  const QuadWindow win = quad_window(Q, C.n, 1);
   for (;;) {
     int item = 0;
     if (lane == 0) item = atomicAdd(work, 1);
     item = __shfl_sync(0xffffffffu, item, 0);
-    int p, part;
-    if (!quad_item(Q, C.n, item, nheavy, parts, p, part)) break;
-    const int nparts = item < nheavy * parts ? parts : 1;
+    int p, part, nparts;
+    if (!quad_item(Q, win, item, p, part, nparts)) break;
     const int64_t b0 = G.start[p];
     const int k = G.len[p];
     if (k < 3 && Q.order) break;  // longest rows first: every later root is as short
@@ -922,44 +948,83 @@ __global__ void __launch_bounds__((WEIGHTED || ADJ ? kQuadMaxWarps : kQuadMaxWar
 // member (bits of the later members).  The 4-cliques p < a < b < d are then
 // the set bits d of row(a) AND row(b) for every edge (a, b): the edges are
 // queued 32 at a time, each lane ANDs its two rows word by word and emits one
-// clique per set bit into the clique queue.  The bins of (a, b), (a, d) and
-// (b, d) are computed from the positions as the graph build computes them
-// (edge_rbin), the bin of (a, b) once per edge.  No row other than R+(p) is
-// read; the tests are k(k-1)/2 per root instead of the sum over R+(p) of the
-// members' row lengths.  Rows up to 256 members (8-bit positions).
+// clique per set bit into the clique queue, which is drained 32 at a time.  No
+// row other than R+(p) is read; the tests are k(k-1)/2 per root instead of the
+// sum over R+(p) of the members' row lengths.  Rows up to 255 members (8-bit
+// positions, one for the root).
+//
+// What a clique adds depends on its six radial bins, on the catalogue-id order
+// of its vertices and on their flags.  Three things are therefore done once
+// per row instead of once per clique: the members are sorted by catalogue id,
+// so that only the root's place among the three members of a clique is open
+// (three comparisons with its rank in the row, and at most three exchanges
+// bring the bins into id order); the bins of all pairs are kept from the
+// membership test (rows up to kMatCap members; else computed again); and
+// the perimeter's rank and canonical order come from two tables over pairs of
+// bins.  Each of the four roots is then a fixed formula of the ordered bins.
+// Sorting ids, comparing perimeters and summing rank differences for every
+// root of every clique took 1,600 warp instructions per 32 cliques, four fifths
+// of the unit-weight kernel; it takes 420 now, with as much again for the
+// enumeration.  4PCF workload (120,000 points, 42M cliques, rows up to 120):
+// unit weights 2.70 -> 1.41 ms, issue-bound; weighted sums 4.2 -> 2.9 ms, bound
+// by the L1 traffic of the reductions (71%); adjoint 7.2 -> 3.2 ms.
+//
+// Unit weights: one count per valid root (see quad_root).  Weighted sums and
+// the adjoint take the valid (clique, root) pairs of the warp 32 at a time,
+// every lane one root, whose role order makes all of its terms fixed formulas
+// again.
 constexpr int kQEdgeQueue = 64;  // edge queue entries per warp (< 32 left + 32 pushed)
+constexpr int kMatCap = 128;
+constexpr int kNoPerimeter = 1 << 29;  // table entry of two bins out of order
 
 struct QuadGLayout {
-  size_t off_rank, off_cnt, off_warp, warp_bytes, total;
-  size_t o_pos, o_w, o_mo, o_g, o_col, o_adj, o_q, o_eq;
+  size_t off_rank, off_tab, off_cnt, off_warp;
+};
+// One warp's area for rows of up to cap members.
+struct QuadGWarp {
+  size_t pos, w, g, col, code, tb, adj, bin, q, eq, bytes;
 };
 
-__host__ __device__ inline QuadGLayout quadg_layout(int nbins, int cap, int nwarps, int ncounts,
-                                                    bool adj, bool lw) {
+// position of the root beside the members' (its weight is staged there)
+__host__ __device__ inline int quad_root_slot(int cap) { return cap < 255 ? cap : 255; }
+// pairs whose bins a warp can keep
+__host__ __device__ inline int quad_bins(int cap) {
+  const int c = cap < kMatCap ? cap : kMatCap;
+  return c * (c - 1) / 2;
+}
+
+__host__ __device__ inline QuadGLayout quadg_layout(int nbins, int ncounts) {
   QuadGLayout L;
   size_t o = 0;
   L.off_rank = o;
   o = qalign8(o + sizeof(int) * 4 * (size_t)(nbins + 2));
+  L.off_tab = o;
+  o = qalign8(o + sizeof(int) * 2 * (size_t)nbins * nbins);
   L.off_cnt = o;
   o = o + sizeof(unsigned int) * (size_t)ncounts;
-  o = (o + 15) & ~(size_t)15;
-  L.off_warp = o;
-  const size_t nwd = (size_t)(cap + 31) / 32;
-  size_t w = 0;
-  L.o_pos = w;  w += (size_t)cap * 16;              // float4 position of each member
-  L.o_w = w;    w += lw ? (size_t)cap * 8 : 0;      // weight
-  L.o_mo = w;   w += (size_t)cap * 8;               // (catalogue id << 32) | flags << 24 | meta(p, a)
-  L.o_g = w;    w += adj ? (size_t)cap * 16 : 0;    // 128-bit gradient of each neighbour
-  L.o_col = w;  w += (size_t)cap * 4;               // label
-  L.o_adj = w;  w += (size_t)cap * nwd * 4;         // adjacency rows
-  L.o_q = w;    w += (size_t)kQQueue * 4;           // cliques: a | b << 8 | d << 16 | bin(a,b) << 24
-  L.o_eq = w;   w += (size_t)kQEdgeQueue * 4;       // edges: a | b << 8
-  L.warp_bytes = (w + 15) & ~(size_t)15;
-  L.total = o + L.warp_bytes * nwarps;
+  L.off_warp = (o + 15) & ~(size_t)15;
   return L;
 }
 
-template <bool WEIGHTED, bool SHC, bool ADJ, bool COMPACT, bool TETRA>
+__host__ __device__ inline QuadGWarp quadg_warp(int cap, bool adj, bool lw) {
+  QuadGWarp W;
+  const size_t nwd = (size_t)(cap + 31) / 32;
+  size_t w = 0;
+  W.pos = w;  w += (size_t)cap * 16;              // float4 position of each member
+  W.tb = w;   w += (size_t)cap * 4;               // catalogue id, then pair index base
+  W.w = w;    w += lw ? ((size_t)cap + 1) * 8 : 0;  // weight, and the root's
+  W.g = w;    w += adj ? (size_t)cap * 16 : 0;    // 128-bit gradient of each neighbour
+  W.col = w;  w += (size_t)cap * 4;               // label
+  W.code = w; w += (size_t)cap * 4;               // bin of (p, a) from 0 | random << 8 | root << 9
+  W.adj = w;  w += (size_t)cap * nwd * 4;         // adjacency rows
+  W.q = w;    w += (size_t)kQQueue * 4;           // cliques: a | b << 8 | d << 16 | bin(a,b) << 24
+  W.eq = w;   w += (size_t)kQEdgeQueue * 4;       // edges: a | b << 8
+  W.bin = w;  w += (size_t)quad_bins(cap);        // bins of the pairs
+  W.bytes = (w + 15) & ~(size_t)15;
+  return W;
+}
+
+template <bool WEIGHTED, bool SHC, bool ADJ, bool TETRA>
 __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW : kQuadMaxWarpsU)) * 32)
     quad4g_kernel(
     DevCatalog C, CSRView G, QuadParams Q, unsigned long long* __restrict__ g_cnt,
@@ -970,137 +1035,295 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
     unsigned long long* __restrict__ g_hi) {
   constexpr bool LW = WEIGHTED || ADJ;
   extern __shared__ __align__(16) unsigned char smem[];
-  const QuadGLayout L = quadg_layout(Q.nbins, Q.cap, blockDim.x >> 5, SHC ? nh + nd : 0, ADJ, LW);
+  const QuadGLayout L = quadg_layout(Q.nbins, SHC ? nh + nd : 0);
   QuadCtx X;
   quad_setup<SHC, ADJ>(X, Q, smem + L.off_rank, smem + L.off_cnt, g_cnt, g_fix, d_cnt, d_fix, nh,
                        nd, fscale, dscale, cot);
   const PairParams& P = Q.P;
+  const int nb = Q.nbins;
+  // rank - 1 of the perimeter b1 <= b2 <= b3 <= b4 is s_t12[b1, b2] +
+  // s_t34[b3, b4] (bins from 0)
+  int* const s_t12 = reinterpret_cast<int*>(smem + L.off_tab);
+  int* const s_t34 = s_t12 + nb * nb;
+  for (int k = threadIdx.x; k < nb * nb; k += blockDim.x) {
+    const int i = k / nb + 1, j = k % nb + 1, n2 = nb + 2;
+    const int* F = X.F;
+    s_t12[k] = i <= j ? (F[i] - F[1]) + (F[n2 + j] - F[n2 + i]) - F[2 * n2 + j] : kNoPerimeter;
+    s_t34[k] = i <= j ? F[2 * n2 + i] + (F[3 * n2 + j] - F[3 * n2 + i]) : kNoPerimeter;
+  }
+  __syncthreads();
 
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  unsigned char* wb = smem + L.off_warp + L.warp_bytes * (threadIdx.x >> 5);
-  float4* s_pos = reinterpret_cast<float4*>(wb + L.o_pos);
-  double* s_w = reinterpret_cast<double*>(wb + L.o_w);
-  unsigned long long* s_mo = reinterpret_cast<unsigned long long*>(wb + L.o_mo);
-  unsigned* s_grad = reinterpret_cast<unsigned*>(wb + L.o_g);  // four words per neighbour, cap apart
-  int* s_col = reinterpret_cast<int*>(wb + L.o_col);
-  uint32_t* s_adj = reinterpret_cast<uint32_t*>(wb + L.o_adj);
-  uint32_t* s_q = reinterpret_cast<uint32_t*>(wb + L.o_q);
-  uint32_t* s_eq = reinterpret_cast<uint32_t*>(wb + L.o_eq);
+  // the first long_warps warps hold rows of up to cap members, the others of
+  // up to short_cap
+  const int wid = threadIdx.x >> 5;
+  const bool big = wid < Q.long_warps;
+  const int cap = big || Q.long_warps == 0 ? Q.cap : Q.short_cap;
+  const QuadGWarp A = quadg_warp(cap, ADJ, LW);
+  unsigned char* wb = smem + L.off_warp;
+  if (big || Q.long_warps == 0)
+    wb += A.bytes * wid;
+  else
+    wb += quadg_warp(Q.cap, ADJ, LW).bytes * Q.long_warps + A.bytes * (wid - Q.long_warps);
+  float4* const s_pos = reinterpret_cast<float4*>(wb + A.pos);
+  double* const s_w = reinterpret_cast<double*>(wb + A.w);
+  unsigned* const s_grad = reinterpret_cast<unsigned*>(wb + A.g);  // four words per neighbour, cap apart
+  int* const s_col = reinterpret_cast<int*>(wb + A.col);
+  int* const s_code = reinterpret_cast<int*>(wb + A.code);
+  int* const s_tb = reinterpret_cast<int*>(wb + A.tb);
+  uint32_t* const s_adj = reinterpret_cast<uint32_t*>(wb + A.adj);
+  uint32_t* const s_q = reinterpret_cast<uint32_t*>(wb + A.q);
+  uint32_t* const s_eq = reinterpret_cast<uint32_t*>(wb + A.eq);
+  uint8_t* const s_bin = wb + A.bin;
+  const int slot = quad_root_slot(cap);
   unsigned long long quads = 0, rooted = 0, probes = 0;
+  const float guard = P.f32 ? P.tguard : INFINITY;
+  // edge test and radial bin (from 0) of members x, y (see bin_pair_f32)
+  auto pair_bin = [&](int x, int y, int& b0) -> bool {
+    const float4 px = s_pos[x], py = s_pos[y];
+    const float dx = py.x - px.x, dy = py.y - px.y, dz = py.z - px.z;
+    const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+    const float t = fmaf(d2 * rsqrt_approx(d2), P.f_inv_dr, P.f_t0);
+    const float tr = __fadd_rn(t, 12582912.0f);
+    const float tn = __fadd_rn(tr, -12582912.0f);
+    b0 = __float_as_int(tr) - 0x4B400000 - (t < tn ? 1 : 0);
+    bool in = (unsigned)b0 < (unsigned)nb;
+    if (!(fabsf(t - tn) >= guard)) {
+      int b = 1;
+      in = d2 < P.rmax2_hi && d2 > P.rmin2_lo &&
+           edge_radial_f64(C.posd[s_col[x]], C.posd[s_col[y]], P, b);
+      b0 = b - 1;
+    }
+    return in;
+  };
 
-  int nheavy;
-  const int parts = quad_split_parts(Q, nheavy);
+  int phase = big ? 0 : 1;  // long rows first, then the others (work[1], work[0])
+  QuadWindow win = quad_window(Q, C.n, phase);
   for (;;) {
     int item = 0;
-    if (lane == 0) item = atomicAdd(work, 1);
+    if (lane == 0) item = atomicAdd(work + (1 - phase), 1);
     item = __shfl_sync(0xffffffffu, item, 0);
-    int p, part;
-    if (!quad_item(Q, C.n, item, nheavy, parts, p, part)) break;
-    const int nparts = item < nheavy * parts ? parts : 1;
+    int p, part, nparts;
+    if (!quad_item(Q, win, item, p, part, nparts)) {
+      if (phase == 1) break;
+      phase = 1;
+      win = quad_window(Q, C.n, 1);
+      continue;
+    }
     const int64_t b0 = G.start[p];
     const int k = G.len[p];
     if (k < 3 && Q.order) break;  // longest rows first: every later root is as short
-    if (k < 3 || k > Q.cap) continue;  // rows longer than cap are rejected on the host
-    const uint8_t fp = C.flags[p] | (G.deg_full[p] > 3 ? kFlagDeg4 : 0);
+    if (k < 3 || k > cap) continue;  // rows longer than cap are rejected on the host
+    // a vertex is a root unless it is a buffer point or (not -tetra) its full
+    // row is too short
+    auto root_bit = [&](int v, uint8_t f) {
+      return !(f & FLAG_BUFFER) && (TETRA || G.deg_full[v] > 3) ? 1u : 0u;
+    };
+    const uint8_t fp = C.flags[p];
+    const unsigned prnd = fp & FLAG_RANDOM, proot = root_bit(p, fp);
     const int op = C.orig[p];
-    const double wp = LW ? C.w[p] : 0.0;
     Fix128 racc = {0ull, 0ull};
     const int nwk = (k + 31) >> 5;  // adjacency words per row for this root
     __syncwarp();
-    for (int x = lane; x < k; x += 32) {
-      const unsigned long long r = G.rec[b0 + x];
-      const int a = rec_col(r);
-      s_col[x] = a;
-      s_pos[x] = C.pos4[a];
-      const uint8_t fa = C.flags[a] | (G.deg_full[a] > 3 ? kFlagDeg4 : 0);
-      s_mo[x] = ((unsigned long long)(uint32_t)C.orig[a] << 32) | (rec_meta(r) | ((uint32_t)fa << 24));
-      if (LW) s_w[x] = C.w[a];
-      if (ADJ) {
-        s_grad[x] = s_grad[Q.cap + x] = s_grad[2 * Q.cap + x] = s_grad[3 * Q.cap + x] = 0u;
-      }
+    // the members sorted by catalogue id
+    int below = 0;
+    const int k4 = (k + 3) & ~3;
+    for (int x = lane; x < k4; x += 32) {
+      const int id = x < k ? C.orig[rec_col(G.rec[b0 + x])] : 0x7fffffff;
+      s_tb[x] = id;
+      below += id < op ? 1 : 0;
     }
+    const int rank_p = (int)__reduce_add_sync(0xffffffffu, (unsigned)below);
     for (int i = lane; i < k * nwk; i += 32) s_adj[i] = 0u;
     __syncwarp();
-    // pass 1: adjacency among the members of R+(p)
+    for (int x = lane; x < k; x += 32) {
+      const int id = s_tb[x];
+      int at = 0;
+      for (int j = 0; j < k4; j += 4) {
+        const int4 v = *reinterpret_cast<const int4*>(&s_tb[j]);
+        at += (v.x < id ? 1 : 0) + (v.y < id ? 1 : 0) + (v.z < id ? 1 : 0) + (v.w < id ? 1 : 0);
+      }
+      const unsigned long long r = G.rec[b0 + x];
+      const int a = rec_col(r);
+      const uint8_t fa = C.flags[a];
+      s_col[at] = a;
+      s_pos[at] = C.pos4[a];
+      s_code[at] = (meta_bin(rec_meta(r)) - 1) | ((fa & FLAG_RANDOM) << 8) | (int)(root_bit(a, fa) << 9);
+      if (LW) s_w[at] = C.w[a];
+      if (ADJ) {
+        s_grad[at] = s_grad[cap + at] = s_grad[2 * cap + at] = s_grad[3 * cap + at] = 0u;
+      }
+    }
+    if (LW && lane == 0) s_w[slot] = C.w[p];
+    __syncwarp();
+    // pass 1: adjacency among the members of R+(p), and their bins
     const int npair = k * (k - 1) / 2;
     const int k2m1 = 2 * k - 1;
+    const bool mat = npair <= quad_bins(cap);  // their bins are kept
+    // index of the pair (x, y) is s_tb[x] + y
+    for (int x = lane; x < k; x += 32) s_tb[x] = x * (k2m1 - x) / 2 - x - 1;
     if (lane == 0 && part == 0) probes += (unsigned long long)npair;  // once per root
     auto pair_of = [&](int t, int& x, int& y) {
       // x: the largest row with x (2k - 1 - x) / 2 <= t pairs before it
-      // (exact up to kPairRowExact members, else one adjustment each way)
+      // (exact for every k up to kPairRowExact)
       x = pair_row_biased(k2m1, t);
-      if (k > kPairRowExact) {
-        x = max(0, min(x, k - 2));
-        if ((x + 1) * (k2m1 - x - 1) / 2 <= t) ++x;
-        if (x * (k2m1 - x) / 2 > t) --x;
-      }
       y = t - (int)((unsigned)(x * (k2m1 - x)) >> 1) + x + 1;
     };
     for (int t = lane; t < npair; t += 32) {
-      int x, y;
+      int x, y, bin;
       pair_of(t, x, y);
-      int r = P.f32 ? member_f32(s_pos[x], s_pos[y], P) : 2;
-      if (r == 2) {
-        int b, mf, mr;
-        r = edge_f64(C.posd[s_col[x]], C.posd[s_col[y]], P, b, mf, mr) ? 1 : 0;
+      if (pair_bin(x, y, bin)) {
+        atomicOr(&s_adj[x * nwk + (y >> 5)], 1u << (y & 31));
+        if (mat) s_bin[t] = (uint8_t)bin;
       }
-      if (r == 1) atomicOr(&s_adj[x * nwk + (y >> 5)], 1u << (y & 31));
     }
     __syncwarp();
     int qn = 0, en = 0;
-    // one queued clique: (p, a = member x, b = member y, d = member z), one
-    // per lane (act: the lane holds entry e).  The weighted 4PCF bins the
-    // warp's cliques together (quad_contrib_flat): every lane takes part, a
-    // lane without a clique reads nothing and holds no valid root.
+    // one queued clique: (p, members x < y < z), one per lane (act: the lane
+    // holds entry e; every lane takes part, one without a clique has no root)
     auto drain_one = [&](int e, bool act) {
-      constexpr bool FLAT = WEIGHTED && COMPACT && !ADJ && !TETRA;
-      if (!act && !FLAT) return;
-      QVerts V;
-      uint32_t m[6] = {0u, 0u, 0u, 0u, 0u, 0u};
-      int x = 0, y = 0, z = 0;
-      V.fl[0] = V.fl[1] = V.fl[2] = V.fl[3] = 0;
-      V.og[0] = V.og[1] = V.og[2] = V.og[3] = 0;
-      V.w[0] = V.w[1] = V.w[2] = V.w[3] = 0.0;
+      const uint32_t qe = act ? s_q[e] : 0u;
+      const int x = (int)(qe & 0xffu), y = (int)((qe >> 8) & 0xffu), z = (int)((qe >> 16) & 0xffu);
+      const int cx = s_code[x], cy = s_code[y], cz = s_code[z];
+      int bxz = 0, byz = 0;
       if (act) {
-        const uint32_t qe = s_q[e];
-        x = (int)(qe & 0xffu);
-        y = (int)((qe >> 8) & 0xffu);
-        z = (int)((qe >> 16) & 0xffu);
-        const int bxy = (int)(qe >> 24);
-        const int bxz = edge_rbin(C.posd, P, s_col[x], s_col[z], s_pos[x], s_pos[z]);
-        const int byz = edge_rbin(C.posd, P, s_col[y], s_col[z], s_pos[y], s_pos[z]);
-        const unsigned long long ma = s_mo[x], mb = s_mo[y], md = s_mo[z];
-        V.fl[0] = fp;
-        V.fl[1] = (uint8_t)((uint32_t)ma >> 24);
-        V.fl[2] = (uint8_t)((uint32_t)mb >> 24);
-        V.fl[3] = (uint8_t)((uint32_t)md >> 24);
-        V.og[0] = op;
-        V.og[1] = (int)(ma >> 32);
-        V.og[2] = (int)(mb >> 32);
-        V.og[3] = (int)(md >> 32);
-        V.w[0] = wp;
-        V.w[1] = LW ? s_w[x] : 0.0;
-        V.w[2] = LW ? s_w[y] : 0.0;
-        V.w[3] = LW ? s_w[z] : 0.0;
-        // m: (p,a) (p,b) (p,d) (a,b) (a,d) (b,d)
-        m[0] = (uint32_t)ma & 0xffffffu;
-        m[1] = (uint32_t)mb & 0xffffffu;
-        m[2] = (uint32_t)md & 0xffffffu;
-        m[3] = pack_meta(bxy, 1, 1);
-        m[4] = pack_meta(bxz, 1, 1);
-        m[5] = pack_meta(byz, 1, 1);
+        if (mat) {
+          bxz = s_bin[s_tb[x] + z];
+          byz = s_bin[s_tb[y] + z];
+        } else {
+          pair_bin(x, z, bxz);
+          pair_bin(y, z, byz);
+        }
       }
-      int nroot;
-      if constexpr (FLAT)
-        nroot = quad_contrib_flat<SHC>(X, V, m, act,
-                                       (unsigned)x | ((unsigned)y << 10) | ((unsigned)z << 20), s_w,
-                                       wp);
-      else
-        nroot = quad_emit<WEIGHTED, SHC, ADJ, COMPACT, TETRA>(X, V, m, gscale, racc, s_grad, Q.cap,
-                                                              x, y, z);
-      quads += nroot > 0;
-      rooted += nroot;
+      // bins b_ij between the i-th and j-th vertex in catalogue-id order: the
+      // root first, then moved behind the members of smaller id
+      int b01 = cx & 0xff, b02 = cy & 0xff, b03 = cz & 0xff, b12 = (int)(qe >> 24), b13 = bxz, b23 = byz;
+      auto swap_if = [](bool c, int& u, int& v) {
+        const int t = c ? v : u;
+        v = c ? u : v;
+        u = t;
+      };
+      const bool r1 = x < rank_p, r2 = y < rank_p, r3 = z < rank_p;  // r3 implies r2 implies r1
+      swap_if(r1, b02, b12);
+      swap_if(r1, b03, b13);
+      swap_if(r2, b01, b02);
+      swap_if(r2, b13, b23);
+      swap_if(r3, b02, b03);
+      swap_if(r3, b12, b13);
+      const int r = (r1 ? 1 : 0) + (r2 ? 1 : 0) + (r3 ? 1 : 0);
+      // one bit per vertex in that order: randoms, and possible roots
+      auto insert = [&](unsigned three, unsigned own) {
+        const unsigned low = (1u << r) - 1u;
+        return (three & low) | (own << r) | ((three & ~low) << 1);
+      };
+      const unsigned rnd = insert((unsigned)(((cx >> 8) & 1) | ((cy >> 7) & 2) | ((cz >> 6) & 4)), prnd);
+      unsigned vm = insert((unsigned)(((cx >> 9) & 1) | ((cy >> 8) & 2) | ((cz >> 7) & 4)), proot);
+      if (!act) vm = 0u;
+      // histogram index of each root, or none when its perimeter is not
+      // canonical
+      int kk[4] = {0, 0, 0, 0};
+      if (TETRA) {
+        if (!(b01 == b02 && b01 == b03 && b01 == b12 && b01 == b13 && b01 == b23)) vm = 0u;
+        kk[0] = kk[1] = kk[2] = kk[3] = b01;
+      } else {
+        auto root = [&](int i, int b1, int b2, int b3, int b4, int d1, int d2) {
+          const int cfg = s_t12[b1 * nb + b2] + s_t34[b3 * nb + b4];
+          if (!((unsigned)cfg < (1u << 28) && b2 <= b3)) vm &= ~(1u << i);
+          kk[i] = cfg + X.ncfg * (d1 + nb * d2);
+        };
+        root(0, b01, b12, b23, b03, b02, b13);
+        root(1, b01, b02, b23, b13, b12, b03);
+        root(2, b02, b01, b13, b23, b12, b03);
+        root(3, b03, b01, b12, b23, b13, b02);
+      }
+      quads += vm ? 1 : 0;
+      rooted += (unsigned)__popc(vm);
+      if constexpr (!LW && !TETRA) {
+        // the pattern of root i: its randomness, then that of the others
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const unsigned low = (1u << i) - 1u;
+          const unsigned pat = ((rnd >> i) & 1u) | ((rnd & low) << 1) | (rnd & ~(2u * low + 1u));
+          if ((vm >> i) & 1u) qcount<SHC>(X, kk[i] + X.nbin * (int)pat);
+        }
+      } else {
+        // the warp's valid roots, ordered by vertex, then lane
+        const unsigned three = (unsigned)(x | (y << 8) | (z << 16));
+        const unsigned lowb = r == 0 ? 0u : (0xffffffu >> (24 - 8 * r));
+        const unsigned vpos = (three & lowb) | ((unsigned)slot << (8 * r)) |
+                              (r == 3 ? 0u : (three & ~lowb) << 8);
+        unsigned mr[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mr[i] = __ballot_sync(0xffffffffu, (vm >> i) & 1u);
+        const int c0 = __popc(mr[0]), c1 = c0 + __popc(mr[1]), c2 = c1 + __popc(mr[2]),
+                  total = c2 + __popc(mr[3]);
+        for (int i0 = 0; i0 < total; i0 += 32) {
+          const int i = i0 + lane;
+          const int R = i < c0 ? 0 : (i < c1 ? 1 : (i < c2 ? 2 : 3));
+          const int base = R == 0 ? 0 : (R == 1 ? c0 : (R == 2 ? c1 : c2));
+          const unsigned mR = R == 0 ? mr[0] : (R == 1 ? mr[1] : (R == 2 ? mr[2] : mr[3]));
+          const int o = i < total ? (int)__fns(mR, 0, i - base + 1) : 0;
+          // every lane takes part in each shuffle; the select comes after
+          const unsigned ornd = __shfl_sync(0xffffffffu, rnd, o);
+          const unsigned opos = __shfl_sync(0xffffffffu, vpos, o);
+          const int q0 = __shfl_sync(0xffffffffu, kk[0], o), q1 = __shfl_sync(0xffffffffu, kk[1], o),
+                    q2 = __shfl_sync(0xffffffffu, kk[2], o), q3 = __shfl_sync(0xffffffffu, kk[3], o);
+          if (i >= total) continue;
+          const int kr = R == 0 ? q0 : (R == 1 ? q1 : (R == 2 ? q2 : q3));
+          // roles: the root, then the other three in id order
+          const int v[4] = {R, R == 0 ? 1 : 0, R <= 1 ? 2 : 1, R <= 2 ? 3 : 2};
+          int pos[4];
+          unsigned rb[4];
+          double w[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            pos[j] = (int)((opos >> (8 * v[j])) & 0xffu);
+            rb[j] = (ornd >> v[j]) & 1u;
+            w[j] = LW ? s_w[pos[j]] : 0.0;
+          }
+          const int onr = (int)(rb[0] + rb[1] + rb[2] + rb[3]);
+          if constexpr (ADJ) {
+            double g[4];
+            quad_root_grad(X, kr, rb, w, g);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              if (pos[j] == slot)
+                fix_acc(racc, g[j], gscale);
+              else
+                smem_fix_add(s_grad + pos[j], cap, __double2ll_rn(g[j] * gscale));
+            }
+          } else if constexpr (TETRA) {
+            qcount<SHC>(X, kr + nb * onr);
+            if (WEIGHTED)
+              qfix(X, qfx(X.fix, kr + nb * onr), qfx(X.fix, kr + nb * (onr + 5)),
+                   ((w[0] * w[1]) * w[2]) * w[3], X.fscale);
+#pragma unroll
+            for (int tt = 0; tt < 6; ++tt) {
+              const int ua = term_gate(tt), ub = term_pu(tt), uc = term_pv(tt);
+              if (!rb[ua]) continue;
+              const int nr3 = (int)(rb[ua] + rb[ub] + rb[uc]);
+              const int kt = kr + nb * tt + nb * 6 * nr3;
+              // discR (all three random) equals category 3 and is copied on the host
+              qdcount<SHC>(X, kt);
+              if (WEIGHTED)
+                qfix(X, qfx(X.dfix, kt), qfx(X.dfix, kt + X.dhi), (w[ua] * w[ub]) * w[uc], X.dscale);
+            }
+          } else {
+            qcount<SHC>(X, kr + X.nbin * onr);
+            qfix(X, qfx(X.fix, kr + X.nbin * onr), qfx(X.fix, kr + X.nbin * (onr + 5)),
+                 ((w[0] * w[1]) * w[2]) * w[3], X.fscale);
+#pragma unroll
+            for (int tt = 0; tt < 6; ++tt) {
+              if (!rb[term_gate(tt)]) continue;
+              const int u = term_pu(tt), vv = term_pv(tt);
+              const int kt = kr + X.nbin * tt + X.nbin * 6 * (int)(rb[u] + rb[vv]);
+              qdcount<SHC>(X, kt);
+              qfix(X, qfx(X.dfix, kt), qfx(X.dfix, kt + X.dhi), w[u] * w[vv], X.dscale);
+            }
+          }
+        }
+      }
     };
     // the cliques of up to 32 queued edges (entry e, or none when e < 0);
     // every lane takes part.  fin: also drain the cliques still queued.
@@ -1115,7 +1338,10 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
         y = (int)((ent >> 8) & 0xffu);
         cw = y >> 5;
         cm = s_adj[x * nwk + cw] & s_adj[y * nwk + cw];
-        bxy = edge_rbin(C.posd, P, s_col[x], s_col[y], s_pos[x], s_pos[y]);
+        if (mat)
+          bxy = s_bin[s_tb[x] + y];
+        else
+          pair_bin(x, y, bxy);
       }
       for (;;) {
         if (live)
@@ -1128,7 +1354,7 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
         if (has) {
           const int z = cw * 32 + __ffs(cm) - 1;
           cm &= cm - 1u;
-          s_q[qn + __popc(hm & lt)] = (uint32_t)(x | (y << 8) | (z << 16) | (bxy << 24));
+          s_q[qn + __popc(hm & lt)] = (uint32_t)(x | (y << 8) | (z << 16)) | ((uint32_t)bxy << 24);
         }
         qn += __popc(hm);
         if (qn >= 32 || (fin && hm == 0u && qn > 0)) {
@@ -1170,7 +1396,7 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
     if (ADJ) {
       for (int x = lane; x < k; x += 32) {
         unsigned long long lo, hi;
-        hist_fix_value(reinterpret_cast<const unsigned long long*>(s_grad), Q.cap, x, lo, hi);
+        hist_fix_value(reinterpret_cast<const unsigned long long*>(s_grad), cap, x, lo, hi);
         if (lo | hi) fix_merge(&g_lo[s_col[x]], &g_hi[s_col[x]], lo, hi);
       }
       racc = fix_warp_sum(racc);
@@ -1206,11 +1432,35 @@ int quad4_warps(int nbins, int cap, int ncounts, bool adj = false, int maxw = kQ
 
 }  // namespace
 
-// Warps per block of the geometric kernel (at most maxw).
-static int quadg_warps(int nbins, int cap, int ncounts, bool adj, bool lw, int maxw) {
-  int nw = maxw;
-  while (nw > 1 && quadg_layout(nbins, cap, nw, ncounts, adj, lw).total > kQuadSmemLimit) nw -= 1;
-  return nw;
+// Block shape of the geometric kernel: rows beyond kShortRow members go to the
+// first few warps of each block, with the capacity they need, and the others
+// hold short rows only, which leaves room for 24 warps beside the pair bins.
+// (4PCF workload, rows up to 120, unit weights: one capacity for all, 13
+// warps, 1.97 ms; the long rows, 9% of the work, in a launch of their own
+// 1.46 ms; this way 1.41 ms, and at a tenth of the size 0.21, 0.36 and 0.22.)  Catalogues whose
+// average row is half of kShortRow or more take one capacity.
+constexpr int kLongWarps = 4;
+static QuadParams quadg_shape(const QuadParams& Q0, int ncounts, bool adj, bool lw, int maxw, int& nw,
+                              size_t& smem) {
+  QuadParams Q = Q0;
+  const size_t fixed = quadg_layout(Q.nbins, ncounts).off_warp;
+  const size_t big = quadg_warp(Q.cap, adj, lw).bytes;
+  Q.long_warps = 0;
+  Q.short_cap = kShortRow;
+  if (Q.cap > kShortRow && Q.order && Q.above && Q.nclass > kShortRow && 2 * Q.mean_row < kShortRow) {
+    const size_t small = quadg_warp(kShortRow, adj, lw).bytes;
+    nw = maxw;
+    while (nw > kLongWarps && fixed + kLongWarps * big + (nw - kLongWarps) * small > kQuadSmemLimit) --nw;
+    smem = fixed + kLongWarps * big + (nw - kLongWarps) * small;
+    if (nw >= 3 * kLongWarps) {
+      Q.long_warps = kLongWarps;
+      return Q;
+    }
+  }
+  nw = maxw;
+  while (nw > 1 && fixed + nw * big > kQuadSmemLimit) --nw;
+  smem = fixed + nw * big;
+  return Q;
 }
 
 // Launch of either 4-clique kernel: grid of resident blocks, dynamic roots.
@@ -1231,7 +1481,7 @@ static void launch_quad_grid(K kfn, int nw, size_t smem, int n, int* work, cudaS
   const int64_t need = ((int64_t)n + nw - 1) / nw;
   if (blocks > need) blocks = need;
   if (blocks < 1) blocks = 1;
-  GR_CUDA_TRY(cudaMemsetAsync(work, 0, sizeof(int), s));
+  GR_CUDA_TRY(cudaMemsetAsync(work, 0, 2 * sizeof(int), s));
   kfn<<<(unsigned)blocks, nw * 32, smem, s>>>(C, G, Q, g_cnt, g_fix, d_cnt, d_fix, nh, nd, fscale,
                                               dscale, stats, work, cot, gscale, g_lo, g_hi);
   GR_CHECK_LAUNCH();
@@ -1242,46 +1492,49 @@ bool launch_quad4(const DevCatalog& C, const CSRView& G, const QuadParams& Q, bo
                   unsigned long long* d_fix, int nh, int nd, double fscale, double dscale,
                   bool shared_counts, unsigned long long* stats, int* work, cudaStream_t s) {
   if (C.n <= 0) return false;
-  const bool geo = Q.geo != 0;
-  const int maxw = weighted ? (geo ? kQuadGWarpsW : kQuadMaxWarps) : kQuadMaxWarpsU;
-  auto warps = [&](int ncounts, int mw) {
-    return geo ? quadg_warps(Q.nbins, Q.cap, ncounts, false, weighted, mw)
-               : quad4_warps(Q.nbins, Q.cap, ncounts, false, mw);
+  const int ncnt = nh + nd;
+  int nw = 0;
+  size_t smem = 0;
+  QuadParams S = Q;
+  auto go = [&](auto kfn) {
+    launch_quad_grid(kfn, nw, smem, C.n, work, s, C, G, S, g_cnt, g_fix, d_cnt, d_fix, nh, nd,
+                     fscale, dscale, stats, nullptr, 1.0, nullptr, nullptr);
   };
   // integer counts in block-private counters when they leave room for at
   // least 8 warps (weighted sums without counts need none)
-  const int ncnt = nh + nd;
-  if ((weighted && !Q.counts) || warps(ncnt, kQuadMaxWarps) < 8) shared_counts = false;
+  if (weighted && !Q.counts) shared_counts = false;
+  if (Q.geo) {
+    const int maxw = weighted ? kQuadGWarpsW : kQuadMaxWarpsU;
+    if (shared_counts) {
+      S = quadg_shape(Q, ncnt, false, weighted, maxw, nw, smem);
+      if (nw < 8) shared_counts = false;
+    }
+    if (!shared_counts) S = quadg_shape(Q, 0, false, weighted, maxw, nw, smem);
+    auto pick = [&](auto tetra_t) {
+      constexpr bool TT = decltype(tetra_t)::value;
+      if (weighted && shared_counts) go(quad4g_kernel<true, true, false, TT>);
+      else if (weighted) go(quad4g_kernel<true, false, false, TT>);
+      else if (shared_counts) go(quad4g_kernel<false, true, false, TT>);
+      else go(quad4g_kernel<false, false, false, TT>);
+    };
+    Q.tetra ? pick(std::true_type{}) : pick(std::false_type{});
+    return shared_counts;
+  }
+  S.long_warps = 0;
+  if (quad4_warps(Q.nbins, Q.cap, ncnt) < 8) shared_counts = false;
   const int nc = shared_counts ? ncnt : 0;
-  const int nw = warps(nc, maxw);
-  const size_t smem = geo ? quadg_layout(Q.nbins, Q.cap, nw, nc, false, weighted).total
-                          : quad_layout(Q.nbins, Q.cap, nw, nc).total;
+  nw = quad4_warps(Q.nbins, Q.cap, nc, false, weighted ? kQuadMaxWarps : kQuadMaxWarpsU);
+  smem = quad_layout(Q.nbins, Q.cap, nw, nc).total;
   // weighted: the compact contribution code (the unrolled form of its long
   // fixed-point updates overflows the instruction cache); unweighted: unrolled
-  auto go = [&](auto kfn) {
-    launch_quad_grid(kfn, nw, smem, C.n, work, s, C, G, Q, g_cnt, g_fix, d_cnt, d_fix, nh, nd,
-                     fscale, dscale, stats, nullptr, 1.0, nullptr, nullptr);
+  auto pick = [&](auto tetra_t) {
+    constexpr bool TT = decltype(tetra_t)::value;
+    if (weighted && shared_counts) go(quad4_kernel<true, true, false, true, TT>);
+    else if (weighted) go(quad4_kernel<true, false, false, true, TT>);
+    else if (shared_counts) go(quad4_kernel<false, true, false, false, TT>);
+    else go(quad4_kernel<false, false, false, false, TT>);
   };
-  auto pick = [&](auto geo_t, auto tetra_t) {
-    constexpr bool GEO = decltype(geo_t)::value, TT = decltype(tetra_t)::value;
-    if constexpr (GEO) {
-      if (weighted && shared_counts) go(quad4g_kernel<true, true, false, true, TT>);
-      else if (weighted) go(quad4g_kernel<true, false, false, true, TT>);
-      else if (shared_counts) go(quad4g_kernel<false, true, false, false, TT>);
-      else go(quad4g_kernel<false, false, false, false, TT>);
-    } else {
-      if (weighted && shared_counts) go(quad4_kernel<true, true, false, true, TT>);
-      else if (weighted) go(quad4_kernel<true, false, false, true, TT>);
-      else if (shared_counts) go(quad4_kernel<false, true, false, false, TT>);
-      else go(quad4_kernel<false, false, false, false, TT>);
-    }
-  };
-  using T1 = std::true_type;
-  using T0 = std::false_type;
-  if (geo)
-    Q.tetra ? pick(T1{}, T1{}) : pick(T1{}, T0{});
-  else
-    Q.tetra ? pick(T0{}, T1{}) : pick(T0{}, T0{});
+  Q.tetra ? pick(std::true_type{}) : pick(std::false_type{});
   return shared_counts;
 }
 
@@ -1289,18 +1542,21 @@ void launch_adj4(const DevCatalog& C, const CSRView& G, const QuadParams& Q, con
                  double gscale, unsigned long long* g_lo, unsigned long long* g_hi,
                  unsigned long long* stats, int* work, cudaStream_t s) {
   if (C.n <= 0) return;
+  int nw = 0;
+  size_t smem = 0;
+  QuadParams S = Q;
+  auto go = [&](auto kfn) {
+    launch_quad_grid(kfn, nw, smem, C.n, work, s, C, G, S, nullptr, nullptr, nullptr, nullptr, 0, 0,
+                     1.0, 1.0, stats, cot, gscale, g_lo, g_hi);
+  };
   if (Q.geo) {
-    const int nw = quadg_warps(Q.nbins, Q.cap, 0, true, true, kQuadGWarpsA);
-    const size_t smem = quadg_layout(Q.nbins, Q.cap, nw, 0, true, true).total;
-    launch_quad_grid(quad4g_kernel<false, false, true, true, false>, nw, smem, C.n, work, s, C, G, Q,
-                     nullptr, nullptr, nullptr, nullptr, 0, 0, 1.0, 1.0, stats, cot, gscale, g_lo,
-                     g_hi);
+    S = quadg_shape(Q, 0, true, true, kQuadGWarpsA, nw, smem);
+    go(quad4g_kernel<false, false, true, false>);
   } else {
-    const int nw = quad4_warps(Q.nbins, Q.cap, 0, true);
-    const size_t smem = quad_layout(Q.nbins, Q.cap, nw, 0, true).total;
-    launch_quad_grid(quad4_kernel<false, false, true, true, false>, nw, smem, C.n, work, s, C, G, Q,
-                     nullptr, nullptr, nullptr, nullptr, 0, 0, 1.0, 1.0, stats, cot, gscale, g_lo,
-                     g_hi);
+    S.long_warps = 0;
+    nw = quad4_warps(Q.nbins, Q.cap, 0, true);
+    smem = quad_layout(Q.nbins, Q.cap, nw, 0, true).total;
+    go(quad4_kernel<false, false, true, true, false>);
   }
 }
 
@@ -1320,6 +1576,21 @@ void quad_expand_patterns(const unsigned long long* H, int nbin, unsigned long l
         dc[k + (size_t)nbin * tt + (size_t)nbin * 6 * npr] += v;
       }
     }
+  }
+}
+
+void quad_cot_lines(const double* cot2, const double* cot3, const double* cotN,
+                    const double* cotR, int nbin, double* out) {
+  for (int k = 0; k < nbin; ++k) {
+    double* c = out + (size_t)k * kCotLine;
+    c[0] = cot2[k];
+    c[1] = cot2[k] + (cot3 ? cot3[k] : 0.0);
+    for (int tt = 0; tt < 6; ++tt) {
+      const size_t kt = k + (size_t)nbin * tt;
+      c[2 + tt] = cotN ? cotN[kt] : 0.0;
+      c[8 + tt] = c[2 + tt] + (cotR ? cotR[kt] : 0.0);
+    }
+    c[14] = c[15] = 0.0;
   }
 }
 
