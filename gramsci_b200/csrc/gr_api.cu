@@ -20,24 +20,6 @@
 
 using namespace gr;
 
-// The speculative rebuild of the last configuration (index and graph
-// phases) as two instantiated CUDA graphs, replayed by the next 3PCF count
-// whose configuration is the same: every pointer, capacity and size the two
-// phases read, the binning and the previous bounding box (`key`).  A replay
-// launches the phases' 18 kernels and copies at once instead of one host
-// launch each.
-struct SpecGraph {
-  std::vector<unsigned long long> key;
-  cudaGraphExec_t idx = nullptr, csr = nullptr;
-  void release() {
-    if (idx) cudaGraphExecDestroy(idx);
-    if (csr) cudaGraphExecDestroy(csr);
-    idx = csr = nullptr;
-    key.clear();
-  }
-  ~SpecGraph() { release(); }
-};
-
 struct gr_ctx {
   int device = 0;
   cudaStream_t own = nullptr;
@@ -65,9 +47,9 @@ struct gr_ctx {
   bool csr_valid = false;
   bool index_valid = false;  // index: the current catalogue and bins on rmax-wide cells
   int clique_mode = 0;  // GR_OPT_CLIQUE_MODE
-  // speculative rebuilds (count_tri): catalogue generation (set_catalog),
+  // speculative graphs (count_tri): catalogue generation (set_catalog),
   // generation of the last verified build, and whether speculating on a new
-  // catalogue is still worth it (off after it once found a changed grid)
+  // catalogue is still worth it (off after one ran out of room)
   uint64_t cat_gen = 0, spec_gen = ~0ull;
   bool spec_new_ok = true;
   bool keep_graph = false;    // GR_OPT_KEEP_GRAPH
@@ -80,17 +62,17 @@ struct gr_ctx {
   DevBuf<unsigned long long> hfix, dfix;  // fixed-point sums (lo words, then hi words)
   double wmax = 0.0;                      // max |w| over the catalogue
   double wgmax = 0.0, wrmax = 0.0;        // max |w| over galaxies / randoms
-  DevBuf<unsigned char> uniform_flag;
+  CatalogBox box;                         // of the current catalogue
+  HostBuf<CatalogScan> scan;              // pinned result of the catalogue scan
+  DevBuf<unsigned long long> scan_part;   // its blocks' partial results
+  DevBuf<unsigned long long> fingerprint;
   DevBuf<int> work;
   HostBuf<unsigned long long> stage;     // pinned read-back of a call's results
-  DevBuf<double> hval;                   // fixed-point sums converted on the device
   DevBuf<int> qorder;                    // 4-clique root order (n) + its class counts
   DevBuf<int> long_list;                 // 3PCF: roots with rows beyond a warp's capacity
   DevBuf<float4> row_pos;                // their rows (second launch)
   DevBuf<double> row_w;
   DevBuf<int> row_q, row_id;
-  SpecGraph spec_graph;                  // captured speculative rebuild (count_tri)
-  SpecGraph spec_index;                  // captured speculative index (gr_count_2pcf)
   DevBuf<double> cot, grad;              // adjoint inputs / output
   DevBuf<unsigned long long> gfix;       // adjoint fixed-point gradients (lo[n], hi[n])
   // batched regions: 0 none, 1 nsplit^3 subcubes, 2 region ids, 3 mocks
@@ -351,99 +333,6 @@ int set_err(gr_ctx* c, int code, const std::string& m) {
   }                                                \
   return GR_OK;
 
-// The 128-bit fixed-point sums of a histogram in FP64, on the device: value
-// k of (lo[k], hi[k]) times inv_scale[k / per] (inverses of powers of two,
-// so one rounding, as the host's fix_value).  split: (lo, hi) are the split
-// limbs of fix_red, worth hi * 2^32 + lo (fix_split_value).  The host then
-// reads n doubles instead of 2n words and converts nothing.
-__global__ void fix_convert_kernel(const unsigned long long* __restrict__ lo,
-                                   const unsigned long long* __restrict__ hi, int64_t n,
-                                   int64_t per, double4 inv_scale, int split, int stride,
-                                   double* __restrict__ out) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t c = i / per;
-    const double is = c == 0 ? inv_scale.x : (c == 1 ? inv_scale.y : (c == 2 ? inv_scale.z : inv_scale.w));
-    unsigned long long l = lo[i * stride], h = hi[i * stride];
-    if (split) {
-      // (signed h) << 32 as 128 bits, plus l
-      const long long hs = (long long)h;
-      const unsigned long long L = (unsigned long long)hs << 32;
-      unsigned long long H = (unsigned long long)(hs >> 32);
-      const unsigned long long L2 = L + l;
-      H += L2 < L ? 1ull : 0ull;
-      l = L2;
-      h = H;
-    }
-    out[i] = fix_to_double(l, h, is);
-  }
-}
-
-// Queue fix_convert_kernel: n values from (lo, lo + hi_off) entries of
-// `stride` words each, categories of `per` values with scales sc[0..3].
-static void enqueue_fix_convert(const unsigned long long* lo, int64_t hi_off, int64_t n,
-                                int64_t per, const double sc[4], bool split, double* out,
-                                cudaStream_t s, int stride = 1) {
-  if (n <= 0) return;
-  const double4 inv = make_double4(1.0 / sc[0], 1.0 / sc[1], 1.0 / sc[2], 1.0 / sc[3]);
-  const int blocks = (int)std::min<int64_t>((n + 255) / 256, 2 * (int64_t)sm_count());
-  fix_convert_kernel<<<blocks, 256, 0, s>>>(lo, lo + hi_off * stride, n, per, inv, split ? 1 : 0,
-                                            stride, out);
-  GR_CHECK_LAUNCH();
-}
-
-// Clears *flag unless all galaxy weights are equal and all random weights are
-// equal; writes max |w| over galaxies to wmax[0] and over randoms to wmax[1]
-// (as the bits of non-negative doubles) and sets *nonfinite when a weight is
-// not finite (tested directly, not through the maxima).  Reduced per block
-// first, so each block makes at most four global updates.
-__global__ void uniform_check_kernel(const double* __restrict__ w, int64_t n_data, int64_t n,
-                                     unsigned char* flag, unsigned long long* wmax,
-                                     int* nonfinite) {
-  __shared__ unsigned long long s_mg[32], s_mr[32];
-  __shared__ int s_bad[32];
-  unsigned long long mg = 0, mr = 0;
-  bool bad = false, nf = false;
-  const double refg = n_data > 0 ? w[0] : 0.0;
-  const double refr = n > n_data ? w[n_data] : 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const double v = w[i];
-    nf = nf || !isfinite(v);
-    const double ref = i < n_data ? refg : refr;
-    bad = bad || __double_as_longlong(v) != __double_as_longlong(ref);
-    const unsigned long long a = (unsigned long long)__double_as_longlong(fabs(v));
-    if (i < n_data) mg = a > mg ? a : mg;
-    else mr = a > mr ? a : mr;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    unsigned long long u = __shfl_xor_sync(0xffffffffu, mg, o);
-    mg = u > mg ? u : mg;
-    u = __shfl_xor_sync(0xffffffffu, mr, o);
-    mr = u > mr ? u : mr;
-  }
-  bad = __any_sync(0xffffffffu, bad);
-  if (__any_sync(0xffffffffu, nf) && (threadIdx.x & 31) == 0) atomicOr(nonfinite, 1);
-  const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    s_mg[wid] = mg;
-    s_mr[wid] = mr;
-    s_bad[wid] = bad ? 1 : 0;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int b = 0;
-    for (int k = 0; k < nw; ++k) {
-      mg = s_mg[k] > mg ? s_mg[k] : mg;
-      mr = s_mr[k] > mr ? s_mr[k] : mr;
-      b |= s_bad[k];
-    }
-    if (mg) atomicMax(&wmax[0], mg);
-    if (mr) atomicMax(&wmax[1], mr);
-    if (b) *flag = 0;
-  }
-}
-
 unsigned long long mix_host(unsigned long long z) {
   z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
   z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
@@ -490,36 +379,23 @@ float ev_ms(cudaEvent_t a, cudaEvent_t b) {
   return ms;
 }
 
-// Index build + pair parameters (shared by every query).
-// speculate: see CellIndex / UpperCSR; the caller checks the flags
-// sub: cell grid of the index (1: cells at least rmax wide, 2: rmax/2,
-// 0: chosen by density, see CellIndex::build)
 void set_pair_params(gr_ctx* c, double coord_max) {
   make_pair_params(c->P, c->rmin, c->rmax, c->nbins, c->nmu, c->logbins, coord_max,
                    c->precision == 1);
 }
 
-// Host state of a replayed index build that other calls may have changed
-// since it was captured (a batched call sets the pair parameters without a
-// build, another catalogue its own flags); the replay's key holds the rest.
-void restore_index(gr_ctx* c) {
-  c->index.n_data = c->n_data;
-  c->index.has_buffer = c->has_buffer ? 1 : 0;
-  c->index.speculated = true;
-  set_pair_params(c, c->index.coord_max);
-  c->csr_valid = false;
-  c->index_valid = false;
-}
-
-void build_index(gr_ctx* c, bool speculate = false, int sub = 1) {
+// Index build + pair parameters (shared by every query); z is cleared in the
+// same launches.
+// sub: cell grid of the index (1: cells at least rmax wide, 2: rmax/2,
+// 0: chosen by density, see CellIndex::build)
+void build_index(gr_ctx* c, int sub = 1, const ZeroList& z = ZeroList()) {
   cudaStream_t s = c->stream();
   c->csr_valid = false;
   c->index_valid = false;
-  c->index.build(c->xyz.p, c->w.p, c->has_buffer ? c->buffer.p : nullptr, c->n, c->n_data, c->rmax, s,
-                 speculate, sub, kDenseCellPoints);
+  c->index.build(c->xyz.p, c->w.p, c->has_buffer ? c->buffer.p : nullptr, c->n, c->n_data, c->box,
+                 c->rmax, s, z, sub, kDenseCellPoints);
   set_pair_params(c, c->index.coord_max);
-  // a speculative index is valid once its flag has been read
-  c->index_valid = !c->index.speculated && c->index.grid.sub == 1;
+  c->index_valid = c->index.grid.sub == 1;
 }
 
 void build_csr(gr_ctx* c, bool speculate = false) {
@@ -559,123 +435,6 @@ double uniform_product(double wg, double wr, int ng, int nr) {
 
 }  // namespace
 
-// Everything the speculative index and graph phases read from the host:
-// the catalogue's device pointers and sizes, the binning and precision, the
-// previous bounding box, and every buffer's address and capacity.
-static std::vector<unsigned long long> spec_key(const gr_ctx* c) {
-  std::vector<unsigned long long> k;
-  auto add = [&](auto v) {
-    unsigned long long u = 0;
-    std::memcpy(&u, &v, std::min(sizeof(v), sizeof(u)));
-    k.push_back(u);
-  };
-  auto buf = [&](const auto& b) {
-    add(b.p);
-    add(b.n);
-  };
-  add(c->xyz.p);
-  add(c->w.p);
-  add(c->has_buffer ? c->buffer.p : nullptr);
-  add(c->n);
-  add(c->n_data);
-  add(c->rmin);
-  add(c->rmax);
-  add(c->nbins);
-  add(c->nmu);
-  add(c->logbins);
-  add(c->precision);
-  const CellIndex& I = c->index;
-  add(I.have_prev);
-  add(I.prev_n);
-  add(I.prev_rmax);
-  add(I.prev_sub);
-  for (int i = 0; i < 7; ++i) add(I.prev_raw[i]);
-  buf(I.bbox_raw);
-  buf(I.bbox_prev);
-  buf(I.cell_count);
-  buf(I.key_orig);
-  buf(I.slot);
-  buf(I.tmp_perm);
-  buf(I.cell_start);
-  buf(I.orig);
-  buf(I.cell_key);
-  buf(I.cell_start64);
-  buf(I.scan_tmp);
-  buf(I.pos4);
-  buf(I.posd);
-  buf(I.w);
-  buf(I.flags);
-  const UpperCSR& G = c->csr;
-  buf(G.deg_up);
-  buf(G.deg_full);
-  buf(G.work);
-  buf(G.scan_tmp);
-  buf(G.rstart);
-  buf(G.cbound);
-  buf(G.cbase);
-  buf(G.scratch);
-  buf(G.stats);
-  buf(G.ctl);
-  return k;
-}
-
-// Capture the speculative index and graph phases of the current
-// configuration (the call has just run them with success) on the context's
-// own stream.  A capture that fails leaves no graph: the next call runs the
-// phases eagerly.
-static std::vector<unsigned long long> spec_key(const gr_ctx* c, int sub, bool with_csr) {
-  std::vector<unsigned long long> k = spec_key(c);
-  k.push_back((unsigned long long)sub);
-  k.push_back(with_csr ? 1ull : 0ull);
-  return k;
-}
-
-// Capture the speculative index phase (grid choice `sub`) and, with_csr, the
-// graph phase of the current configuration into G (the call has just run
-// them with success) on the context's own stream.  A capture that fails
-// leaves no graph: the next call runs the phases eagerly.
-static void capture_spec_graph(gr_ctx* c, SpecGraph& G, int sub, bool with_csr) {
-  G.release();
-  // the configuration as this call leaves it (a successful speculative build
-  // changes none of it; buffers it grew have their new addresses)
-  const std::vector<unsigned long long> key = spec_key(c, sub, with_csr);
-  cudaStream_t user = c->user;
-  c->user = nullptr;  // build_index / build_csr enqueue on c->stream()
-  cudaStream_t s = c->own;
-  cudaGraph_t g[2] = {nullptr, nullptr};
-  cudaGraphExec_t e[2] = {nullptr, nullptr};
-  bool ok = true;
-  const int phases = with_csr ? 2 : 1;
-  for (int phase = 0; phase < phases && ok; ++phase) {
-    if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-      ok = false;
-      break;
-    }
-    try {
-      if (phase == 0)
-        build_index(c, true, sub);
-      else
-        build_csr(c, true);
-    } catch (...) {
-      ok = false;
-    }
-    if (cudaStreamEndCapture(s, &g[phase]) != cudaSuccess || !g[phase]) ok = false;
-    if (ok && cudaGraphInstantiate(&e[phase], g[phase], 0) != cudaSuccess) ok = false;
-  }
-  for (int k = 0; k < 2; ++k)
-    if (g[k]) cudaGraphDestroy(g[k]);
-  c->user = user;
-  cudaGetLastError();  // a failed capture leaves nothing behind
-  if (!ok || !c->index.speculated || spec_key(c, sub, with_csr) != key) {
-    for (int k = 0; k < 2; ++k)
-      if (e[k]) cudaGraphExecDestroy(e[k]);
-    return;
-  }
-  G.idx = e[0];
-  G.csr = e[1];
-  G.key = key;
-}
-
 extern "C" {
 
 const char* gr_version(void) { return "gramsci_b200 0.1 (sm_100a)"; }
@@ -709,8 +468,6 @@ int gr_destroy(gr_ctx* c) {
   for (int k = 0; k < 2; ++k)
     if (c->bev[k]) cudaEventDestroy(c->bev[k]);
   c->regions.release_graph();
-  c->spec_graph.release();
-  c->spec_index.release();
   if (c->own) cudaStreamDestroy(c->own);
   delete c;
   return GR_OK;
@@ -735,65 +492,35 @@ static int set_catalog_impl(gr_ctx* c, const double* xyz, const double* w, const
   c->cat_gen++;
   c->xyz.reserve(3 * n + 1);
   c->w.reserve(n + 1);
-  if (n > 0) {
-    GR_CUDA_TRY(cudaMemcpyAsync(c->xyz.p, xyz, sizeof(double) * 3 * n, kind, s));
-    GR_CUDA_TRY(cudaMemcpyAsync(c->w.p, w, sizeof(double) * n, kind, s));
-  }
   c->has_buffer = buffer != nullptr;
-  if (buffer) {
-    c->buffer.reserve(n + 1);
-    GR_CUDA_TRY(cudaMemcpyAsync(c->buffer.p, buffer, sizeof(int32_t) * n, kind, s));
-  }
+  if (buffer) c->buffer.reserve(n + 1);
   c->n = n;
   c->n_data = n_data;
   c->n_rand = n_rand;
-  // Uniform weights (all galaxies equal, all randoms equal) let the kernels
-  // keep integer counts only; sums are then count x product.
-  // [0] uniform flag, [4] non-finite weight flag (int), [8] max |w| galaxies,
-  // [16] max |w| randoms, [24] fingerprint
-  c->uniform_flag.reserve(32);
-  // pinned stage: [0..3) the 24 bytes below, [3] first galaxy weight,
-  // [4] first random weight
-  c->stage.reserve(8);
-  unsigned char* init = reinterpret_cast<unsigned char*>(c->stage.p);
-  std::memset(init, 0, 24);
-  init[0] = 1;
-  GR_CUDA_TRY(cudaMemcpyAsync(c->uniform_flag.p, init, 24, cudaMemcpyHostToDevice, s));
-  unsigned long long* d_wmax = reinterpret_cast<unsigned long long*>(c->uniform_flag.p + 8);
-  if (n > 0) {
-    int blocks = (int)std::min<int64_t>((n + 255) / 256, (int64_t)2 * sm_count());
-    uniform_check_kernel<<<blocks, 256, 0, s>>>(c->w.p, n_data, n, c->uniform_flag.p, d_wmax,
-                                                reinterpret_cast<int*>(c->uniform_flag.p + 4));
-    GR_CHECK_LAUNCH();
+  c->scan.reserve(1);
+  CatalogScan& h = *c->scan.p;
+  std::memset(&h, 0, sizeof(h));
+  const bool host = kind == cudaMemcpyHostToDevice;
+  if (host && n > 0) {
+    GR_CUDA_TRY(cudaMemcpyAsync(c->xyz.p, xyz, sizeof(double) * 3 * n, kind, s));
+    GR_CUDA_TRY(cudaMemcpyAsync(c->w.p, w, sizeof(double) * n, kind, s));
+    if (buffer) GR_CUDA_TRY(cudaMemcpyAsync(c->buffer.p, buffer, sizeof(int32_t) * n, kind, s));
   }
-  // the read-back lands in the stage after the upload above has read it
-  unsigned char* out = reinterpret_cast<unsigned char*>(c->stage.p);
-  double* wgr = reinterpret_cast<double*>(c->stage.p + 3);
-  wgr[0] = 0.0;
-  wgr[1] = 0.0;
-  GR_CUDA_TRY(cudaMemcpyAsync(out, c->uniform_flag.p, 24, cudaMemcpyDeviceToHost, s));
-  if (n_data > 0) GR_CUDA_TRY(cudaMemcpyAsync(&wgr[0], c->w.p, sizeof(double), cudaMemcpyDeviceToHost, s));
-  if (n_rand > 0)
-    GR_CUDA_TRY(cudaMemcpyAsync(&wgr[1], c->w.p + n_data, sizeof(double), cudaMemcpyDeviceToHost, s));
-  GR_CUDA_TRY(cudaStreamSynchronize(s));
-  const double wg = wgr[0], wr = wgr[1];
-  unsigned char flag = out[0];
-  int nonfinite = 0;
-  std::memcpy(&nonfinite, out + 4, 4);
-  if (nonfinite) {
+  // device arrays are copied by the scan itself
+  scan_catalog(host ? c->xyz.p : xyz, host ? c->w.p : w, buffer, n_data, n, c->xyz.p, c->w.p,
+               c->buffer.p, c->scan_part, c->scan.p, c->box, s);
+  if (h.word[8] & kScanWeightBad) {
     c->cat_set = false;  // nothing may be counted on a half-set catalogue
     return set_err(c, GR_E_ARG, "non-finite weights");
   }
-  std::memcpy(&c->wgmax, out + 8, 8);
-  std::memcpy(&c->wrmax, out + 16, 8);
+  std::memcpy(&c->wgmax, &h.word[6], 8);
+  std::memcpy(&c->wrmax, &h.word[7], 8);
   c->wmax = std::max(c->wgmax, c->wrmax);
-  if (!std::isfinite(c->wmax)) {
-    c->cat_set = false;
-    return set_err(c, GR_E_ARG, "non-finite weights");
-  }
-  c->uniform = flag != 0;
-  c->w_gal = wg;
-  c->w_ran = wr;
+  // Uniform weights (all galaxies equal, all randoms equal) let the kernels
+  // keep integer counts only; sums are then count x product.
+  c->uniform = (h.word[8] & kScanWeightsDiffer) == 0;
+  c->w_gal = h.w0[0];
+  c->w_ran = h.w0[1];
   c->cat_set = true;
   c->csr_valid = false;
   c->index_valid = false;
@@ -884,10 +611,11 @@ struct ScopedEvents {
 };
 
 // Pair-sweep variant for a catalogue layout: cached per workload class or
-// timed now (histograms are reset by the caller afterwards).
+// timed now (the results, z, are clear before and after).
 static int pick_pair2_variant(gr_ctx* c, const DevCatalog& C, bool weighted, double fscale,
                               unsigned long long* hcnt, unsigned long long* hfix,
-                              unsigned long long* stats, int* work, cudaStream_t s) {
+                              unsigned long long* stats, int* work, cudaStream_t s,
+                              const ZeroList& z) {
   // a grid of rmax/2 cells is read by the tile sweep only
   if (C.grid.sub == 2) return kPairTile2;
   if (c->autotune == 0) return kPairWarpCell;
@@ -916,7 +644,6 @@ static int pick_pair2_variant(gr_ctx* c, const DevCatalog& C, bool weighted, dou
     auto it = T.choice.find(key);
     if (it != T.choice.end()) return it->second;
   }
-  const int nh = c->nbins * c->nmu * 4;
   ScopedEvents ev;
   cudaEvent_t a = ev.a, b = ev.b;
   // every variant once untimed (its first launch loads its code), then the
@@ -928,8 +655,7 @@ static int pick_pair2_variant(gr_ctx* c, const DevCatalog& C, bool weighted, dou
   }
   for (int round = 0; round < 3; ++round) {
     for (int v = 0; v < nvar; ++v) {
-      GR_CUDA_TRY(cudaMemsetAsync(hcnt, 0, sizeof(unsigned long long) * nh, s));
-      GR_CUDA_TRY(cudaMemsetAsync(hfix, 0, sizeof(unsigned long long) * 2 * nh, s));
+      zero_async(z, s);
       GR_CUDA_TRY(cudaEventRecord(a, s));
       launch_pair2(C, c->P, weighted, hcnt, hfix, fscale, stats, work, s, v);
       GR_CUDA_TRY(cudaEventRecord(b, s));
@@ -939,6 +665,7 @@ static int pick_pair2_variant(gr_ctx* c, const DevCatalog& C, bool weighted, dou
       t[v] = std::min(t[v], ms);
     }
   }
+  zero_async(z, s);
   int best = kPairWarpCell;
   for (int v = 1; v < nvar; ++v)
     if (t[v] < t[best]) best = v;
@@ -959,72 +686,41 @@ int gr_count_2pcf(gr_ctx* c, double* N2, double* N3, int64_t* counts, double* ca
   c->hcnt.reserve(nh);
   c->hfix.reserve(2 * nh);
   c->stats.reserve(8);
+  c->work.reserve(4);
   // read-back in the pinned stage: counts (nh), fixed-point sums (2 nh),
-  // stats (8), the speculative grid's bounding-box flag (1)
-  c->stage.reserve(3 * (size_t)nh + 9);
+  // stats (8)
+  c->stage.reserve(3 * (size_t)nh + 8);
   unsigned long long* hc = c->stage.p;
   unsigned long long* hf = hc + nh;
   unsigned long long* st = hf + 2 * (size_t)nh;
-  unsigned long long* gflag = st + 8;
   std::vector<double> hs(nh, 0.0);
   // dense catalogues: cells of rmax/2 and the tile sweep
   int sub = 1;
   if (c->autotune == 1) sub = 0;
   if (c->autotune == 2 + kPairTile2) sub = 2;
-  // A catalogue seen before (or a new one while that has worked) is indexed
-  // on the grid of the last bounding box without waiting for the new one;
-  // a device flag read with the histograms repeats the call with waits when
-  // the box changed (as for the 3PCF).
   const bool reuse = reuse_graph(c);
-  const bool can_spec =
-      !reuse && c->index.have_prev && (c->cat_gen == c->spec_gen || c->spec_new_ok);
-  int variant = 0;
-  bool replayed = false;
-  for (int attempt = 0; attempt < 2; ++attempt) {
-    const bool spec = can_spec && attempt == 0;
-    replayed = spec && c->spec_index.idx && spec_key(c, sub, false) == c->spec_index.key;
-    GR_CUDA_TRY(cudaEventRecord(c->ev[0], s));
-    if (!reuse) {
-      if (replayed) {
-        restore_index(c);
-        GR_CUDA_TRY(cudaGraphLaunch(c->spec_index.idx, s));
-      } else {
-        build_index(c, spec, sub);
-      }
-    }
-    GR_CUDA_TRY(cudaEventRecord(c->ev[1], s));
-    c->work.reserve(4);
-    variant = pick_pair2_variant(c, c->index.view(), weighted, fscale, c->hcnt.p, c->hfix.p,
-                                 c->stats.p, c->work.p, s);
-    c->last_variant = variant;
-    GR_CUDA_TRY(cudaEventRecord(c->ev[1], s));
-    GR_CUDA_TRY(cudaMemsetAsync(c->hcnt.p, 0, sizeof(unsigned long long) * nh, s));
-    GR_CUDA_TRY(cudaMemsetAsync(c->hfix.p, 0, sizeof(unsigned long long) * 2 * nh, s));
-    GR_CUDA_TRY(cudaMemsetAsync(c->stats.p, 0, sizeof(unsigned long long) * 8, s));
-    launch_pair2(c->index.view(), c->P, weighted, c->hcnt.p, c->hfix.p, fscale, c->stats.p,
-                 c->work.p, s, variant);
-    GR_CUDA_TRY(cudaEventRecord(c->ev[2], s));
-    GR_CUDA_TRY(cudaMemcpyAsync(hc, c->hcnt.p, sizeof(unsigned long long) * nh, cudaMemcpyDeviceToHost, s));
-    if (weighted)
-      GR_CUDA_TRY(cudaMemcpyAsync(hf, c->hfix.p, sizeof(unsigned long long) * 2 * nh, cudaMemcpyDeviceToHost, s));
-    GR_CUDA_TRY(cudaMemcpyAsync(st, c->stats.p, sizeof(unsigned long long) * 8, cudaMemcpyDeviceToHost, s));
-    *gflag = 0;
-    const bool speculated = spec && c->index.speculated;
-    if (speculated)
-      GR_CUDA_TRY(cudaMemcpyAsync(gflag, c->index.mismatch_flag(), sizeof(unsigned long long),
-                                  cudaMemcpyDeviceToHost, s));
-    GR_CUDA_TRY(cudaEventRecord(c->ev[3], s));
-    GR_CUDA_TRY(cudaStreamSynchronize(s));
-    if (speculated && *gflag != 0) {  // the bounding box changed: repeat with waits
-      if (c->cat_gen != c->spec_gen) c->spec_new_ok = false;
-      continue;
-    }
-    // a speculative index that held: kept as a graph for the next call of
-    // the same configuration
-    if (speculated && !replayed) capture_spec_graph(c, c->spec_index, sub, false);
-    break;
-  }
-  if (!reuse) c->spec_gen = c->cat_gen;
+  ZeroList z;
+  z.add(c->hcnt.p, sizeof(unsigned long long) * nh);
+  z.add(c->hfix.p, sizeof(unsigned long long) * 2 * nh);
+  z.add(c->stats.p, sizeof(unsigned long long) * 8);
+  GR_CUDA_TRY(cudaEventRecord(c->ev[0], s));
+  if (reuse)
+    zero_async(z, s);
+  else
+    build_index(c, sub, z);
+  const int variant = pick_pair2_variant(c, c->index.view(), weighted, fscale, c->hcnt.p, c->hfix.p,
+                                         c->stats.p, c->work.p, s, z);
+  c->last_variant = variant;
+  GR_CUDA_TRY(cudaEventRecord(c->ev[1], s));
+  launch_pair2(c->index.view(), c->P, weighted, c->hcnt.p, c->hfix.p, fscale, c->stats.p, c->work.p,
+               s, variant);
+  GR_CUDA_TRY(cudaEventRecord(c->ev[2], s));
+  ResultList r;
+  r.copy(c->hcnt.p, nh, hc);
+  if (weighted) r.copy(c->hfix.p, 2 * (int64_t)nh, hf);
+  r.copy(c->stats.p, 8, st);
+  results_async(r, s);
+  GR_CUDA_TRY(cudaStreamSynchronize(s));
   if (weighted)
     for (int k = 0; k < nh; ++k) hs[k] = fix_value(hf[k], hf[nh + k], fscale);
   if (!weighted) {
@@ -1055,7 +751,7 @@ int gr_count_2pcf(gr_ctx* c, double* N2, double* N3, int64_t* counts, double* ca
   c->st.rooted = rooted;
   c->st.fp64_rechecks = (int64_t)st[0];
   c->st.candidates = (int64_t)st[1];
-  c->st.kernel_launches = c->index.launches + 1;
+  c->st.kernel_launches = c->index.launches + 2;
   GR_API_END(c)
 }
 
@@ -1160,78 +856,52 @@ static int count_tri(gr_ctx* c, bool equi, double* N2, double* N3, int64_t* coun
   c->stats.reserve(kRootStats);
   ensure_normal(c, nmu, s);
   const bool reuse = hash ? reuse_graph(c) : reuse_index(c);
-  // A rebuild of a catalogue seen before runs without waiting on the host:
-  // the grid is taken from the last bounding box and, for the hash probes, the
-  // graph is filled in the scratch area as it is and the kernel's row capacity
-  // taken from the last graph (longer rows take its global-memory path, so any
-  // capacity gives the same result).  A device flag records a changed
-  // bounding box and the graph build one that ran out of room; both are
-  // read with the results, and the call is then repeated with waits.
-  const bool can_spec =
-      !reuse && c->index.have_prev && (c->cat_gen == c->spec_gen || c->spec_new_ok);
+  // For the hash probes the graph of a catalogue seen before is built without
+  // waiting on the host: filled in the scratch area as it is, the kernel's row
+  // capacity taken from the last graph (longer rows take its global-memory
+  // path, so any capacity gives the same result).  A build that ran out of
+  // room is recorded and read with the results, and the call is then repeated
+  // with waits.
+  const bool can_spec = hash && !reuse && c->csr.max_deg > 0 &&
+                        (c->cat_gen == c->spec_gen || c->spec_new_ok);
   // read-back layout in the pinned stage: counts (nh), the sums converted
-  // on the device (nh doubles), kernel stats, graph control (4) and stats
-  // (3), bbox flag (1)
-  c->stage.reserve(2 * (size_t)nh + kRootStats + 8);
-  c->hval.reserve(nh);
+  // on the device (nh doubles), kernel stats, graph control (4) and stats (3)
+  c->stage.reserve(2 * (size_t)nh + kRootStats + 7);
   unsigned long long* hc = c->stage.p;
   double* hv = reinterpret_cast<double*>(hc + nh);
   unsigned long long* st = hc + 2 * (size_t)nh;
   unsigned long long* gctl = st + kRootStats;
   unsigned long long* gsts = gctl + 4;
-  unsigned long long* gflag = gsts + 3;
   std::vector<double> hs(nh, 0.0);
   cudaEvent_t q0 = c->ev[4];  // owned by the context
   c->work.reserve(4);
   if (!hash) c->long_list.reserve(c->n + 1);
   int tri_launches = 0;
-  std::vector<unsigned long long> key;
-  bool replayed = false;
+  ZeroList z;
+  z.add(c->hcnt.p, sizeof(unsigned long long) * nh);
+  z.add(c->hfix.p, sizeof(unsigned long long) * 2 * nh);
+  z.add(c->stats.p, sizeof(unsigned long long) * kRootStats);
   // results to the stage
-  auto read_back = [&]() {
-    if (want_counts)
-      GR_CUDA_TRY(cudaMemcpyAsync(hc, c->hcnt.p, sizeof(unsigned long long) * nh, cudaMemcpyDeviceToHost, s));
-    if (weighted) {
-      enqueue_fix_convert(c->hfix.p, nh, nh, nbin, fscale, false, c->hval.p, s);
-      GR_CUDA_TRY(cudaMemcpyAsync(hv, c->hval.p, sizeof(double) * nh, cudaMemcpyDeviceToHost, s));
+  auto read_back = [&](bool spec) {
+    ResultList r;
+    if (want_counts) r.copy(c->hcnt.p, nh, hc);
+    if (weighted) r.sums(c->hfix.p, nh, nbin, fscale, hv);
+    r.copy(c->stats.p, kRootStats, st);
+    if (spec) {
+      r.copy(c->csr.ctl.p, 4, gctl);
+      r.copy(c->csr.stats.p, 3, gsts);
     }
-    GR_CUDA_TRY(cudaMemcpyAsync(st, c->stats.p, sizeof(unsigned long long) * kRootStats,
-                                cudaMemcpyDeviceToHost, s));
+    results_async(r, s);
   };
   for (int attempt = 0; attempt < 2; ++attempt) {
     const bool spec = can_spec && attempt == 0;
-    bool replay = false;
-    if (spec) {
-      key = spec_key(c, 1, hash);
-      replay = c->spec_graph.idx && (c->spec_graph.csr || !hash) && key == c->spec_graph.key;
-    }
-    replayed = replay;
     GR_CUDA_TRY(cudaEventRecord(c->ev[0], s));
-    if (!reuse) {
-      if (replay) {
-        restore_index(c);
-        GR_CUDA_TRY(cudaGraphLaunch(c->spec_graph.idx, s));
-      } else {
-        build_index(c, spec);
-      }
-    }
-    GR_CUDA_TRY(cudaEventRecord(c->ev[1], s));
-    if (!reuse && hash) {
-      if (replay) {
-        GR_CUDA_TRY(cudaGraphLaunch(c->spec_graph.csr, s));
-        c->csr.compacted = false;
-      } else {
-        build_csr(c, spec);
-      }
-    }
-    GR_CUDA_TRY(cudaEventRecord(c->ev[2], s));
-    {
-      ZeroList z;
-      z.add(c->hcnt.p, sizeof(unsigned long long) * nh);
-      z.add(c->hfix.p, sizeof(unsigned long long) * 2 * nh);
-      z.add(c->stats.p, sizeof(unsigned long long) * kRootStats);
+    if (reuse)
       zero_async(z, s);
-    }
+    else
+      build_index(c, 1, z);
+    GR_CUDA_TRY(cudaEventRecord(c->ev[1], s));
+    if (!reuse && hash) build_csr(c, spec);
     GR_CUDA_TRY(cudaEventRecord(q0, s));
     RootParams RT{};
     if (hash) {
@@ -1253,38 +923,17 @@ static int count_tri(gr_ctx* c, bool equi, double* N2, double* N3, int64_t* coun
       launch_root3(c->index.view(), RT, weighted, want_counts, c->hcnt.p, c->hfix.p, c->stats.p,
                    c->work.p, c->long_list.p, nullptr, s);
     }
-    tri_launches = 2;  // with the zero fill
+    tri_launches = 1;
     GR_CUDA_TRY(cudaEventRecord(c->ev[3], s));
-    read_back();
-    std::memset(gctl, 0, sizeof(unsigned long long) * 8);
-    const bool speculated = spec && c->index.speculated;
-    if (spec && hash) {
-      GR_CUDA_TRY(cudaMemcpyAsync(gctl, c->csr.ctl.p, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost, s));
-      GR_CUDA_TRY(cudaMemcpyAsync(gsts, c->csr.stats.p, sizeof(unsigned long long) * 3, cudaMemcpyDeviceToHost, s));
-    }
-    if (speculated)
-      GR_CUDA_TRY(cudaMemcpyAsync(gflag, c->index.mismatch_flag(), sizeof(unsigned long long),
-                                  cudaMemcpyDeviceToHost, s));
+    read_back(spec);
     GR_CUDA_TRY(cudaStreamSynchronize(s));
     if (spec) {
-      if (*gflag != 0 || gctl[1] == 1) {  // repeat with waits
+      if (gctl[1] == 1) {  // repeat with waits
         if (c->cat_gen != c->spec_gen) c->spec_new_ok = false;
         continue;
       }
-      if (hash) {
-        c->csr.settle(gctl, gsts);
-        c->csr_valid = true;
-      }
-      // a speculative build that needed no second pass: keep it as graphs
-      // for the next call of the same configuration
-      if (!replayed && (hash || speculated)) {
-        capture_spec_graph(c, c->spec_graph, 1, hash);
-        if (hash) {
-          c->csr_valid = true;
-          c->csr.settle(gctl, gsts);
-        }
-      }
-      c->index_valid = true;
+      c->csr.settle(gctl, gsts);
+      c->csr_valid = true;
     }
     if (!hash && st[6] > 0) {
       const RootLong R = long_rows(c, st);
@@ -1292,7 +941,7 @@ static int count_tri(gr_ctx* c, bool equi, double* N2, double* N3, int64_t* coun
                    c->work.p, c->long_list.p, &R, s);
       tri_launches++;
       GR_CUDA_TRY(cudaEventRecord(c->ev[3], s));
-      read_back();
+      read_back(false);
       GR_CUDA_TRY(cudaStreamSynchronize(s));
       if (st[7] != 0) throw gr::Error{GR_E_CUDA, "3PCF: a row exceeds its own bound"};
     }
@@ -1318,7 +967,7 @@ static int count_tri(gr_ctx* c, bool equi, double* N2, double* N3, int64_t* coun
     for (int k = 0; k < nh; ++k) catsum[k] = hs[k];
   std::memset(&c->st, 0, sizeof(c->st));
   c->st.ms_index = ev_ms(c->ev[0], c->ev[1]);
-  c->st.ms_graph = ev_ms(c->ev[1], c->ev[2]);
+  c->st.ms_graph = hash ? ev_ms(c->ev[1], q0) : 0.0;
   c->st.ms_query = ev_ms(q0, c->ev[3]);
   c->st.ms_total = c->st.ms_index + c->st.ms_graph + c->st.ms_query;
   c->st.n_points = c->n;
@@ -1334,7 +983,7 @@ static int count_tri(gr_ctx* c, bool equi, double* N2, double* N3, int64_t* coun
     root_stats(c, st);
   }
   c->st.kernel_launches = (reuse ? 0 : c->index.launches + (hash ? c->csr.launches : 0)) +
-                          tri_launches + (weighted ? 1 : 0);
+                          tri_launches + 1;
   GR_API_END(c)
 }
 
@@ -1383,21 +1032,26 @@ static int count_quad(gr_ctx* c, bool tetra, double* N2, double* N3, double* dis
   c->dfix.reserve((size_t)2 * ndv * kFixStride);
   c->stats.reserve(8);
   const bool reuse = reuse_graph(c);
+  c->work.reserve(4);
+  ZeroList z;
+  z.add(c->hcnt.p, sizeof(unsigned long long) * nhk);
+  z.add(c->dcnt.p, sizeof(unsigned long long) * ndk);
+  if (weighted) {
+    z.add(c->hfix.p, sizeof(unsigned long long) * 2 * nh * kFixStride);
+    z.add(c->dfix.p, sizeof(unsigned long long) * 2 * ndv * kFixStride);
+  }
+  z.add(c->stats.p, sizeof(unsigned long long) * 8);
   GR_CUDA_TRY(cudaEventRecord(c->ev[0], s));
-  if (!reuse) build_index(c);
+  if (reuse)
+    zero_async(z, s);
+  else
+    build_index(c, 1, z);
   GR_CUDA_TRY(cudaEventRecord(c->ev[1], s));
   if (!reuse) build_csr(c);
   GR_CUDA_TRY(cudaEventRecord(c->ev[2], s));
   const unsigned long long gst[3] = {(unsigned long long)c->csr.rechecks,
                                      (unsigned long long)c->csr.candidates,
                                      (unsigned long long)c->csr.max_deg};
-  GR_CUDA_TRY(cudaMemsetAsync(c->hcnt.p, 0, sizeof(unsigned long long) * nhk, s));
-  if (ndk) GR_CUDA_TRY(cudaMemsetAsync(c->dcnt.p, 0, sizeof(unsigned long long) * ndk, s));
-  if (weighted) {
-    GR_CUDA_TRY(cudaMemsetAsync(c->hfix.p, 0, sizeof(unsigned long long) * 2 * nh * kFixStride, s));
-    GR_CUDA_TRY(cudaMemsetAsync(c->dfix.p, 0, sizeof(unsigned long long) * 2 * ndv * kFixStride, s));
-  }
-  GR_CUDA_TRY(cudaMemsetAsync(c->stats.p, 0, sizeof(unsigned long long) * 8, s));
   if ((int64_t)gst[2] > 1024)
     return set_err(c, GR_E_CAPACITY, "4PCF: a point has more than 1024 larger-label neighbours");
   QuadParams Q{};
@@ -1424,7 +1078,6 @@ static int count_quad(gr_ctx* c, bool tetra, double* N2, double* N3, double* dis
   // counts, fewer), the sums converted on the device (nh, ndv doubles),
   // kernel stats (8)
   c->stage.reserve(2 * ((size_t)nh + ndv) + 8);
-  c->hval.reserve((size_t)nh + ndv);
   unsigned long long* sc = c->stage.p;
   unsigned long long* sd = sc + nh;
   double* sv = reinterpret_cast<double*>(sd + ndv);
@@ -1437,13 +1090,7 @@ static int count_quad(gr_ctx* c, bool tetra, double* N2, double* N3, double* dis
   // launch is repeated with 64-bit counters and carried 128-bit sums.
   for (int attempt = 0; attempt < 2; ++attempt) {
     if (attempt > 0) {
-      GR_CUDA_TRY(cudaMemsetAsync(c->hcnt.p, 0, sizeof(unsigned long long) * nhk, s));
-      if (ndk) GR_CUDA_TRY(cudaMemsetAsync(c->dcnt.p, 0, sizeof(unsigned long long) * ndk, s));
-      if (weighted) {
-        GR_CUDA_TRY(cudaMemsetAsync(c->hfix.p, 0, sizeof(unsigned long long) * 2 * nh * kFixStride, s));
-        GR_CUDA_TRY(cudaMemsetAsync(c->dfix.p, 0, sizeof(unsigned long long) * 2 * ndv * kFixStride, s));
-      }
-      GR_CUDA_TRY(cudaMemsetAsync(c->stats.p, 0, sizeof(unsigned long long) * 8, s));
+      zero_async(z, s);
       GR_CUDA_TRY(cudaEventRecord(q0, s));
     }
     Q.split = (weighted && attempt == 0) ? 1 : 0;
@@ -1451,19 +1098,19 @@ static int count_quad(gr_ctx* c, bool tetra, double* N2, double* N3, double* dis
                                      c->dcnt.p, c->dfix.p, nhk, ndk, fscale, dscale, attempt == 0,
                                      c->stats.p, c->work.p, s);
     GR_CUDA_TRY(cudaEventRecord(c->ev[3], s));
+    ResultList r;
     if (Q.counts) {
-      GR_CUDA_TRY(cudaMemcpyAsync(sc, c->hcnt.p, sizeof(unsigned long long) * nhk, cudaMemcpyDeviceToHost, s));
-      if (ndk)
-        GR_CUDA_TRY(cudaMemcpyAsync(sd, c->dcnt.p, sizeof(unsigned long long) * ndk, cudaMemcpyDeviceToHost, s));
+      r.copy(c->hcnt.p, nhk, sc);
+      r.copy(c->dcnt.p, ndk, sd);
     }
     if (weighted) {
       const double fs[4] = {fscale, fscale, fscale, fscale};
       const double ds4[4] = {dscale, dscale, dscale, dscale};
-      enqueue_fix_convert(c->hfix.p, nh, nh, nh, fs, Q.split != 0, c->hval.p, s, kFixStride);
-      enqueue_fix_convert(c->dfix.p, ndv, ndv, ndv, ds4, Q.split != 0, c->hval.p + nh, s, kFixStride);
-      GR_CUDA_TRY(cudaMemcpyAsync(sv, c->hval.p, sizeof(double) * ((size_t)nh + ndv), cudaMemcpyDeviceToHost, s));
+      r.sums(c->hfix.p, nh, nh, fs, sv, kFixStride, Q.split != 0);
+      r.sums(c->dfix.p, ndv, ndv, ds4, sv + nh, kFixStride, Q.split != 0);
     }
-    GR_CUDA_TRY(cudaMemcpyAsync(st, c->stats.p, sizeof(unsigned long long) * 8, cudaMemcpyDeviceToHost, s));
+    r.copy(c->stats.p, 8, st);
+    results_async(r, s);
     GR_CUDA_TRY(cudaStreamSynchronize(s));
     if (!(shared || Q.split) || st[1] < (1ull << 32)) break;
   }
@@ -1530,8 +1177,7 @@ static int count_quad(gr_ctx* c, bool tetra, double* N2, double* N3, double* dis
   c->st.upper_edges = c->csr.n_edges;
   c->st.fp64_rechecks = (int64_t)gst[0];
   c->st.candidates = (int64_t)gst[1];
-  c->st.kernel_launches = c->index.launches + c->csr.launches + 1 + (Q.order ? kRootOrderLaunches : 0) +
-                          (weighted ? 2 : 0);
+  c->st.kernel_launches = c->index.launches + c->csr.launches + 2 + (Q.order ? kRootOrderLaunches : 0);
   GR_API_END(c)
 }
 
@@ -1580,8 +1226,8 @@ unsigned long long fnv1a(unsigned long long h, const void* p, size_t bytes) {
 
 unsigned long long coord_fingerprint(gr_ctx* c) {
   cudaStream_t s = c->stream();
-  c->uniform_flag.reserve(32);
-  unsigned long long* d = reinterpret_cast<unsigned long long*>(c->uniform_flag.p + 24);
+  c->fingerprint.reserve(1);
+  unsigned long long* d = c->fingerprint.p;
   GR_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(unsigned long long), s));
   if (c->n > 0) {
     int blocks = (int)std::min<int64_t>((c->n + 255) / 256, (int64_t)8 * sm_count());
@@ -1922,7 +1568,7 @@ int gr_adjoint_2pcf(gr_ctx* c, const double* cot2, const double* cot3, double* g
     int sub = 1;
     if (c->autotune == 1) sub = 0;
     if (c->autotune == 2 + kPairTile2) sub = 2;
-    build_index(c, false, sub);
+    build_index(c, sub);
   }
   GR_CUDA_TRY(cudaEventRecord(c->ev[1], s));
   std::memset(&c->st, 0, sizeof(c->st));
@@ -2137,7 +1783,8 @@ int gr_set_mocks(gr_ctx* c, int32_t nmocks, const int64_t* n_data, const int64_t
 static bool ensure_regions(gr_ctx* c, cudaStream_t s, bool rmax_cells) {
   if (c->regions.valid && (!rmax_cells || c->regions.grid_sub == 1)) return false;
   // pair parameters from the catalogue's coordinate bound
-  const CatalogBox box = catalog_box(c->xyz.p, c->n, c->index.bbox_raw, s);
+  const CatalogBox& box = c->box;
+  if (!box.finite) throw gr::Error{GR_E_ARG, "catalogue has non-finite coordinates"};
   set_pair_params(c, box.coord_max);
   c->csr_valid = false;
   // dense regions: cells of rmax/2 and the tile sweep
@@ -2155,11 +1802,17 @@ static bool ensure_regions(gr_ctx* c, cudaStream_t s, bool rmax_cells) {
 }
 
 // Histogram reset and pair sweep of one batched call.
-static void enqueue_batched_sweep(gr_ctx* c, cudaStream_t s) {
+static ZeroList batched_zeros(const gr_ctx* c) {
   const int nh = c->nbins * c->nmu * 4;
-  GR_CUDA_TRY(cudaMemsetAsync(c->bcnt.p, 0, sizeof(unsigned long long) * nh, s));
-  GR_CUDA_TRY(cudaMemsetAsync(c->bfix.p, 0, sizeof(unsigned long long) * 2 * nh, s));
-  GR_CUDA_TRY(cudaMemsetAsync(c->bstats.p, 0, sizeof(unsigned long long) * 8, s));
+  ZeroList z;
+  z.add(c->bcnt.p, sizeof(unsigned long long) * nh);
+  z.add(c->bfix.p, sizeof(unsigned long long) * 2 * nh);
+  z.add(c->bstats.p, sizeof(unsigned long long) * 8);
+  return z;
+}
+
+static void enqueue_batched_sweep(gr_ctx* c, cudaStream_t s) {
+  zero_async(batched_zeros(c), s);
   launch_pair2(c->regions.view(), c->P, c->batch_weighted, c->bcnt.p, c->bfix.p, c->batch_fscale,
                c->bstats.p, c->bwork.p, s, c->batch_variant);
 }
@@ -2218,7 +1871,8 @@ int gr_count_2pcf_batched(gr_ctx* c, double* N2, double* N3, int64_t* counts, do
     c->regions.enqueue_layout(c->xyz.p, c->w.p, s, planned);
     GR_CUDA_TRY(cudaEventRecord(c->ev[2], s));
     c->batch_variant = pick_pair2_variant(c, c->regions.view(), c->batch_weighted, c->batch_fscale,
-                                          c->bcnt.p, c->bfix.p, c->bstats.p, c->bwork.p, s);
+                                          c->bcnt.p, c->bfix.p, c->bstats.p, c->bwork.p, s,
+                                          batched_zeros(c));
     GR_CUDA_TRY(cudaEventRecord(c->ev[3], s));
     enqueue_batched_sweep(c, s);
     c->regions.swept = true;
@@ -2243,16 +1897,17 @@ int gr_count_2pcf_batched(gr_ctx* c, double* N2, double* N3, int64_t* counts, do
     GR_CUDA_TRY(cudaGraphLaunch(c->regions.exec, s));
   }
   GR_CUDA_TRY(cudaEventRecord(c->ev[1], s));
-  std::vector<unsigned long long> hc(nh), hf(2 * nh, 0ull);
-  unsigned long long st[8];
-  GR_CUDA_TRY(cudaMemcpyAsync(hc.data(), c->bcnt.p, sizeof(unsigned long long) * nh, cudaMemcpyDeviceToHost, s));
-  if (c->batch_weighted)
-    GR_CUDA_TRY(cudaMemcpyAsync(hf.data(), c->bfix.p, sizeof(unsigned long long) * 2 * nh, cudaMemcpyDeviceToHost, s));
-  GR_CUDA_TRY(cudaMemcpyAsync(st, c->bstats.p, sizeof(st), cudaMemcpyDeviceToHost, s));
+  c->stage.reserve(3 * (size_t)nh + 8);
+  unsigned long long *hc = c->stage.p, *hf = hc + nh, *st = hf + 2 * (size_t)nh;
+  ResultList r;
+  r.copy(c->bcnt.p, nh, hc);
+  if (c->batch_weighted) r.copy(c->bfix.p, 2 * (int64_t)nh, hf);
+  r.copy(c->bstats.p, 8, st);
+  results_async(r, s);
   GR_CUDA_TRY(cudaEventRecord(c->bev[1], s));
   GR_CUDA_TRY(cudaStreamWaitEvent(us, c->bev[1], 0));
   GR_CUDA_TRY(cudaStreamSynchronize(s));
-  pair_outputs(c, c->batch_weighted, c->batch_fscale, hc.data(), hf.data(), N2, N3, counts, catsum);
+  pair_outputs(c, c->batch_weighted, c->batch_fscale, hc, hf, N2, N3, counts, catsum);
   int64_t rooted = 0;
   for (int k = 0; k < nh; ++k) rooted += (int64_t)hc[k];
   std::memset(&c->st, 0, sizeof(c->st));
@@ -2295,17 +1950,18 @@ int gr_count_2pcf_regions(gr_ctx* c, double* N2, double* N3, int64_t* counts, do
   launch_pair2_tile(c->regions.view(), c->P, c->batch_weighted, c->rcnt.p, c->rfix.p,
                     c->batch_fscale, c->bstats.p, c->bwork.p, s, true);
   GR_CUDA_TRY(cudaEventRecord(c->ev[2], s));
-  std::vector<unsigned long long> hc(tot), hf(2 * tot, 0ull);
-  unsigned long long st[8];
-  GR_CUDA_TRY(cudaMemcpyAsync(hc.data(), c->rcnt.p, sizeof(unsigned long long) * tot, cudaMemcpyDeviceToHost, s));
-  if (c->batch_weighted)
-    GR_CUDA_TRY(cudaMemcpyAsync(hf.data(), c->rfix.p, sizeof(unsigned long long) * 2 * tot, cudaMemcpyDeviceToHost, s));
-  GR_CUDA_TRY(cudaMemcpyAsync(st, c->bstats.p, sizeof(st), cudaMemcpyDeviceToHost, s));
+  c->stage.reserve(3 * tot + 8);
+  unsigned long long *hc = c->stage.p, *hf = hc + tot, *st = hf + 2 * tot;
+  ResultList r;
+  r.copy(c->rcnt.p, (int64_t)tot, hc);
+  if (c->batch_weighted) r.copy(c->rfix.p, 2 * (int64_t)tot, hf);
+  r.copy(c->bstats.p, 8, st);
+  results_async(r, s);
   GR_CUDA_TRY(cudaStreamSynchronize(s));
   int64_t rooted = 0;
   for (int r = 0; r < nreg; ++r) {
     const size_t o = (size_t)r * nh;
-    pair_outputs(c, c->batch_weighted, c->batch_fscale, hc.data() + o, hf.data() + 2 * o,
+    pair_outputs(c, c->batch_weighted, c->batch_fscale, hc + o, hf + 2 * o,
                  N2 ? N2 + (size_t)r * nbm : nullptr, N3 ? N3 + (size_t)r * nbm : nullptr,
                  counts ? counts + o : nullptr, catsum ? catsum + o : nullptr);
   }

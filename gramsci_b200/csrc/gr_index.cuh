@@ -12,12 +12,28 @@
 namespace gr {
 
 // Bounding box of a catalogue and its largest |coordinate| (all zero without
-// points), read back with one wait; raises on non-finite coordinates.
+// points).
 struct CatalogBox {
-  double lo[3], hi[3], coord_max;
+  double lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0}, coord_max = 0.0;
+  bool finite = true;  // false: a coordinate is not
 };
-CatalogBox catalog_box(const double* d_xyz, int64_t n, DevBuf<unsigned long long>& raw,
-                       cudaStream_t s);
+
+// One pass over a catalogue, as the kernel leaves it in pinned memory:
+// word[0..2] / [3..5] order keys of the least and largest coordinates, [6] /
+// [7] bits of the largest |weight| of galaxies / randoms, [8] kScan* flags;
+// w0: the first weight of either.
+constexpr int kCatalogScanWords = 9;
+struct CatalogScan {
+  unsigned long long word[kCatalogScanWords];
+  double w0[2];
+};
+constexpr unsigned int kScanCoordBad = 1u, kScanWeightBad = 2u, kScanWeightsDiffer = 4u;
+
+// Scan (and, when the outputs differ from the inputs, copy) a catalogue; waits
+// for the result.  `out` is pinned.
+void scan_catalog(const double* xyz, const double* w, const int* buffer, int64_t n_data, int64_t n,
+                  double* xyz_out, double* w_out, int* buffer_out, DevBuf<unsigned long long>& part,
+                  CatalogScan* out, CatalogBox& box, cudaStream_t s);
 
 // Uniform-grid index over the catalogue, points laid out in cell order.
 struct CellIndex {
@@ -27,19 +43,6 @@ struct CellIndex {
   CatalogBox box{};        // the box the grid was laid over
   GridParams grid{};
   int launches = 0;
-  DevBuf<unsigned long long> bbox_raw;
-  // Speculative build: the grid depends only on the bounding box, the point
-  // count and rmax, so a build may take the previous build's bounding box
-  // without waiting for the new one and let a device check record whether
-  // it differs (bbox_prev[7] = 1); the caller reads the flag with its results
-  // and rebuilds without speculation when it is set.
-  bool have_prev = false, speculated = false;
-  int64_t prev_n = -1;
-  double prev_rmax = 0.0;
-  int prev_sub = 0;
-  bool prev_auto = false;  // the previous build chose sub itself
-  unsigned long long prev_raw[7] = {0, 0, 0, 0, 0, 0, 0};
-  DevBuf<unsigned long long> bbox_prev;  // previous raw bounding box [0..6], mismatch flag [7]
   DevBuf<int> cell_count, key_orig, slot, tmp_perm, cell_start, orig, cell_key;
   DevBuf<int64_t> cell_start64, scan_tmp;
   DevBuf<float4> pos4;
@@ -50,11 +53,12 @@ struct CellIndex {
   // sub = 1: cells at least rmax wide; sub = 2: at least rmax/2 wide (for
   // the tile pair sweep); sub = 0: 2 when an rmax-wide grid would hold at
   // least dense_per_cell points per cell, else 1.
+  // The grid is laid over cat_box (throws when that is not finite); z is
+  // cleared in the same launches.
   void build(const double* d_xyz, const double* d_w, const int* d_buffer, int64_t n, int64_t n_data,
-             double rmax, cudaStream_t s, bool speculate = false, int sub = 1,
-             double dense_per_cell = 0.0);
+             const CatalogBox& cat_box, double rmax, cudaStream_t s, ZeroList z = ZeroList(),
+             int sub = 1, double dense_per_cell = 0.0);
   double per_cell_rmax = 0.0;  // points per cell of an rmax-wide grid (last build)
-  const unsigned long long* mismatch_flag() const { return bbox_prev.p + 7; }
   DevCatalog view() const;
 };
 

@@ -791,6 +791,8 @@ struct ZeroList {
   size_t bytes[8];
   int n = 0;
   void add(void* ptr, size_t b) {
+    if ((reinterpret_cast<uintptr_t>(ptr) & 15) != 0 || (b & 3) != 0 || n == 8)
+      throw Error{-2, "zero list: buffer not 16-byte aligned, size not a multiple of 4, or too many"};
     if (b > 0) {
       p[n] = ptr;
       bytes[n] = b;
@@ -799,6 +801,35 @@ struct ZeroList {
   }
 };
 void zero_async(const ZeroList& z, cudaStream_t s);
+
+// What a call reads back, written to pinned host memory by one launch (a
+// copy of its own costs 2.5 us of stream time for each array, whatever its
+// size): words as they are, or fixed-point sums (entries of `stride` words,
+// low words then high words) as doubles, `per` values for each scale.
+struct ResultList {
+  struct Part {
+    const unsigned long long *lo, *hi;
+    unsigned long long* out;
+    int64_t n, per;  // per == 0: copied as it is
+    double inv[4];
+    int stride, split;
+  } part[6];
+  int n = 0;
+  void copy(const unsigned long long* src, int64_t count, unsigned long long* out) {
+    if (count <= 0) return;
+    part[n] = Part{src, nullptr, out, count, 0, {0, 0, 0, 0}, 1, 0};
+    ++n;
+  }
+  void sums(const unsigned long long* lo, int64_t count, int64_t per, const double scale[4],
+            double* out, int stride = 1, bool split = false) {
+    if (count <= 0) return;
+    part[n] = Part{lo, lo + count * stride, reinterpret_cast<unsigned long long*>(out), count, per,
+                   {1.0 / scale[0], 1.0 / scale[1], 1.0 / scale[2], 1.0 / scale[3]}, stride,
+                   split ? 1 : 0};
+    ++n;
+  }
+};
+void results_async(const ResultList& r, cudaStream_t s);
 
 // Exclusive scan of n int32 values into n+1 int64 values (out[n] = total).
 // out32 (optional): the scan also as 32-bit integers (values below 2^31)
