@@ -148,7 +148,6 @@ void make_pair_params(PairParams& P, double rmin, double rmax, int nbins, int nm
   double in_lo = rmin + 2.0 * d0;
   in_lo = in_lo * in_lo * (1.0 + 16.0 * u);
   P.rmin2_hi = std::nextafter((float)in_lo, std::numeric_limits<float>::infinity());
-  P.f_rmin = (float)rmin;
   P.f_inv_dr = (float)P.inv_dr;
   P.f_mu_scale = (float)P.mu_scale;
   const double tmax = nbins + 1.0;
@@ -166,6 +165,20 @@ void make_pair_params(PairParams& P, double rmin, double rmax, int nbins, int nm
   P.mB = (float)(8.0 * X * u + 1e-30);
   P.k1 = (float)((eA + eB) * P.mu_scale);
   P.k2 = (float)(128.0 * u * P.mu_scale + 8.0 * u * nmu);
+  // Logarithmic bins: log10(d) moves by at most |d_f - d| / ((d - d0) ln 10),
+  // and 1 / (d - d0) is below 1.2 / d_f when d is above 8 d0; lg2.approx (2^-22
+  // of max(1, |log2 d2|)) and the roundings of the two constants, the sum and
+  // the coordinate make the constant part.  Doubled as above.
+  if (logbins && !force_fp64 && rmin > 8.0 * d0 && std::isfinite(X)) {
+    const double c1 = 0.5 * std::log10(2.0) * P.inv_dr, c0 = -P.log_rmin * P.inv_dr;
+    const double lmax = 2.0 * std::max(std::fabs(std::log2(rmin)), std::fabs(std::log2(rmax))) + 1.0;
+    const double g1 = c1 * lmax * (4.0 * u + 2.0 * u) + u * std::fabs(c0) + 4.0 * u * tmax;
+    P.f_inv_dr = (float)c1;
+    P.f_t0 = (float)c0;
+    P.tguard = (float)(2.0 * g1 + 1e-9 * tmax);
+    P.tguard_d = (float)(2.0 * 1.2 * d0 / std::log(10.0) * P.inv_dr);
+    if ((double)P.tguard + (double)P.tguard_d / rmin < 0.05) P.logbins = 2;
+  }
   P.f32 = (!force_fp64 && !logbins && std::isfinite(tg) && tg < 0.05 && std::isfinite(X)) ? 1 : 0;
 }
 
@@ -610,6 +623,11 @@ struct ScopedEvents {
   ScopedEvents& operator=(const ScopedEvents&) = delete;
 };
 
+// The arithmetic of the tuned pair sweeps, a part of the tuner's keys.
+static const char* pair_form(const PairParams& P) {
+  return P.f32 ? "f32" : (P.logbins == 2 ? "f32log" : "f64");
+}
+
 // Pair-sweep variant for a catalogue layout: cached per workload class or
 // timed now (the results, z, are clear before and after).
 static int pick_pair2_variant(gr_ctx* c, const DevCatalog& C, bool weighted, double fscale,
@@ -635,7 +653,7 @@ static int pick_pair2_variant(gr_ctx* c, const DevCatalog& C, bool weighted, dou
   int cb = 0;
   while (cb < 20 && ((int64_t)4 << (2 * cb)) <= C.grid.ncell) ++cb;
   char key[128];
-  std::snprintf(key, sizeof(key), "pair2v10|%s|%s|dens%d|hist%d|cells%d", c->P.f32 ? "f32" : "f64",
+  std::snprintf(key, sizeof(key), "pair2v10|%s|%s|dens%d|hist%d|cells%d", pair_form(c->P),
                 weighted ? "w" : "u", dens, hb, cb);
   Tuner& T = tuner();
   {
@@ -1500,7 +1518,7 @@ static int pick_adj2_layout(gr_ctx* c, const DevCatalog& C, const double* c2, co
   int cb = 0;
   while (cb < 20 && ((int64_t)4 << (2 * cb)) <= C.grid.ncell) ++cb;
   char key[128];
-  std::snprintf(key, sizeof(key), "adj2v3|%s|dens%d|hist%d|cells%d", c->P.f32 ? "f32" : "f64", dens,
+  std::snprintf(key, sizeof(key), "adj2v3|%s|dens%d|hist%d|cells%d", pair_form(c->P), dens,
                 hb, cb);
   Tuner& T = tuner();
   {

@@ -83,10 +83,12 @@ struct HostBuf {
 struct PairParams {
   // exact FP64 form (src/gramsci.F90:136-147, 295-340)
   double rmin, rmax, rmin2, rmax2, inv_dr, log_rmin, mu_scale;
+  // logbins 2: logarithmic bins, and the tile pair sweep may take its FP32 form
+  // (f32 stays 0): t = lg2(d2) * f_inv_dr + f_t0, guard tguard + tguard_d / d
   int nbins, nmu, logbins, rsd;
   // FP32 fast path with guard band
   int f32;           // 1 = FP32 path enabled
-  float f_rmin, f_inv_dr, f_mu_scale;
+  float tguard_d, f_inv_dr, f_mu_scale;
   float f_t0;        // -rmin / dr
   float rmax2_hi;    // d2 >= rmax2_hi: certainly d >= rmax
   float rmin2_lo;    // d2 <= rmin2_lo: certainly d <= rmin (or -1)
@@ -179,6 +181,13 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   return r;
 }
 
+// log2(x): absolute error 2^-22 for x in (0.5, 2), relative 2^-22 outside.
+__device__ __forceinline__ float lg2_approx(float x) {
+  float r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // FP32 binning of a pair, the radial bin b0 and mu bin m0 from 0 (mu seen from
 // pi; from pj it is nmu - 1 - m0).  Returns 0: not an edge; 1: an edge with
 // these bins; 2: inside the guard band, re-evaluate with edge_f64.  There are
@@ -191,6 +200,11 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 // origin) is decided in FP64 too.  make_pair_params sizes the guards for these
 // operations: t with one rounding of c - rmin/dr and one of the sum beside
 // the error of d, and a cosine within 16 units of 2^-24.
+// LOG: logarithmic bins, the radial coordinate from the base-2 logarithm of
+// d2 (lg2.approx: 2^-22, absolute below 1 and relative above) with a guard
+// that falls with d, since an error of d moves the logarithm by its relative
+// size.
+template <bool LOG = false>
 __device__ __forceinline__ int bin_pair_f32(const float4 pi, const float4 pj, const PairParams& P,
                                             int& b0, int& m0) {
   constexpr float kRound = 12582912.0f;
@@ -201,10 +215,10 @@ __device__ __forceinline__ int bin_pair_f32(const float4 pi, const float4 pj, co
   const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
   const float rd = rsqrt_approx(d2);
   const float d = d2 * rd;
-  const float t = fmaf(d, P.f_inv_dr, P.f_t0);
+  const float t = LOG ? fmaf(lg2_approx(d2), P.f_inv_dr, P.f_t0) : fmaf(d, P.f_inv_dr, P.f_t0);
   const float tr = __fadd_rn(t, kRound);
   const float tn = __fadd_rn(tr, -kRound);
-  bool near_edge = !(fabsf(t - tn) >= P.tguard);
+  bool near_edge = !(fabsf(t - tn) >= (LOG ? fmaf(P.tguard_d, rd, P.tguard) : P.tguard));
   b0 = __float_as_int(tr) - kRoundBits - (t < tn ? 1 : 0);
   m0 = 0;
   if (P.rsd) {

@@ -38,7 +38,11 @@
 //
 // The FP64 form (precision mode 1) stages the candidates' FP64 positions and
 // tests membership with the reference arithmetic; every hit is binned by the
-// exact FP64 predicate.
+// exact FP64 predicate.  It is also what logarithmic bins take when the FP32
+// form's guard would be wide (rmin below a few hundred units of the last place
+// of the coordinates).  Logarithmic bins in FP32: 240,000 weighted points, 10
+// children per parent, 12 bins, sweep 119 -> 89 us (an FP64 square root and
+// log10 per pair before).
 //
 // Bound by instruction issue (about 80% of the slots, DRAM idle).  The binning
 // of a hit took 183 warp instructions per 32 pairs with two updates, two
@@ -107,6 +111,7 @@ __device__ __forceinline__ float warp_max(float v) {
   return __int_as_float(i ^ ((i >> 31) & 0x7fffffff));
 }
 
+enum : int { kTileF64 = 0, kTileF32 = 1, kTileF32Log = 2 };
 // Tables of a launch (see the head of this file).
 enum : int {
   kTabMirror = 0,  // first table only (no buffer points)
@@ -114,7 +119,8 @@ enum : int {
   kTabRooted = 2   // second table only, one update per root
 };
 
-// F32: FP32 membership tests and binning with the guard band (else FP64).
+// MODE: kTileF64, or FP32 membership tests and binning with the guard band,
+// on linear or logarithmic bins.
 // WHIST: tables private to each warp in shared memory, of kind `tab` (else
 // the result in global memory, one update per root).
 // SUB: 1 (cells >= rmax, 5 ranges) or 2 (cells >= rmax/2, 13 ranges).
@@ -122,13 +128,14 @@ enum : int {
 // g_cnt + r*nh and fixed-point words at g_fix + 2*r*nh.
 // ADJ: the 2PCF weight adjoint instead of histograms: each edge adds
 // coef * w_q to dL/dw_p and coef * w_p to dL/dw_q (pair_coef).
-template <bool F32, bool WEIGHTED, bool WHIST, int SUB, bool PERREG, bool ADJ>
+template <int MODE, bool WEIGHTED, bool WHIST, int SUB, bool PERREG, bool ADJ>
 __global__ void __launch_bounds__(kTileThreads, (ADJ && SUB == 2) ? 4 : GR_TILE_MIN_BLOCKS)
     pair2_tile_kernel(DevCatalog C, PairParams P, unsigned long long* __restrict__ g_cnt,
                       unsigned long long* __restrict__ g_fix, double fscale,
                       unsigned long long* __restrict__ stats, int* __restrict__ work, int tab,
                       int parts, TileAdj A) {
   extern __shared__ __align__(16) unsigned char smem[];
+  constexpr bool F32 = MODE != kTileF64;
   typedef TileWarp<F32, WEIGHTED || ADJ, ADJ> Tile;
   __shared__ __align__(16) Tile s_tw[kTileWarps];
   const int lane = threadIdx.x & 31;
@@ -408,7 +415,7 @@ __global__ void __launch_bounds__(kTileThreads, (ADJ && SUB == 2) ? 4 : GR_TILE_
             const int cr = __float_as_int(a.w), cq = T.code[j];
             int st = 2, b0 = 0, m0 = 0;
             if constexpr (F32)
-              st = bin_pair_f32(a, make_float4(T.x[j], T.y[j], T.z[j], 0.f), P, b0, m0);
+              st = bin_pair_f32<MODE == kTileF32Log>(a, make_float4(T.x[j], T.y[j], T.z[j], 0.f), P, b0, m0);
             bool mirrored = true;
             int mrev = 0;  // mu bin from the candidate when it does not mirror m0
             if (st == 2) {
@@ -555,9 +562,11 @@ void launch_pair2_tile(const DevCatalog& C, const PairParams& P, bool weighted,
     if (whist) GR_TILE_S(F, W, true); else GR_TILE_S(F, W, false);                            \
   } while (0)
   if (P.f32) {
-    if (weighted) GR_TILE_H(true, true); else GR_TILE_H(true, false);
+    if (weighted) GR_TILE_H(kTileF32, true); else GR_TILE_H(kTileF32, false);
+  } else if (P.logbins == 2) {
+    if (weighted) GR_TILE_H(kTileF32Log, true); else GR_TILE_H(kTileF32Log, false);
   } else {
-    if (weighted) GR_TILE_H(false, true); else GR_TILE_H(false, false);
+    if (weighted) GR_TILE_H(kTileF64, true); else GR_TILE_H(kTileF64, false);
   }
 #undef GR_TILE_H
 #undef GR_TILE_S
@@ -598,9 +607,11 @@ void launch_adj2_tile(const DevCatalog& C, const PairParams& P, const double* co
                                                 0, parts, A);                                 \
   } while (0)
   if (P.f32) {
-    if (sub == 2) GR_ADJT_LAUNCH(true, 2); else GR_ADJT_LAUNCH(true, 1);
+    if (sub == 2) GR_ADJT_LAUNCH(kTileF32, 2); else GR_ADJT_LAUNCH(kTileF32, 1);
+  } else if (P.logbins == 2) {
+    if (sub == 2) GR_ADJT_LAUNCH(kTileF32Log, 2); else GR_ADJT_LAUNCH(kTileF32Log, 1);
   } else {
-    if (sub == 2) GR_ADJT_LAUNCH(false, 2); else GR_ADJT_LAUNCH(false, 1);
+    if (sub == 2) GR_ADJT_LAUNCH(kTileF64, 2); else GR_ADJT_LAUNCH(kTileF64, 1);
   }
 #undef GR_ADJT_LAUNCH
   GR_CHECK_LAUNCH();
