@@ -5,14 +5,15 @@ the device-resident catalogue to the binned histograms): 100,000 Neyman-Scott
 galaxies (10,000 parents, Poisson(10) children, Gaussian sigma 4 Mpc/h) and
 300,000 uniform randoms in [0,1000]^3, lognormal(0, 0.3) weights, rmin 5,
 rmax 25, 8 radial bins, 5 mu bins (line-of-sight binning on).  Each step
-builds the cell index, the CSR neighbour graph and counts every triangle.
+builds the cell index and counts every triangle from it.
 
 value      distinct triangles binned / second of device time (inputs in HBM)
 e2e        the same through the public API with host inputs: pinned host ->
            device copy of the catalogue, the count, and the histogram read back
 roofline   the triangle kernel: algorithmic bytes / its CUDA-event time, with
            its instruction-issue and shared-atomic rates (`issue`, `atomics`)
-           from the committed ncu summary; `graph_roofline` the graph build
+           from the committed ncu summary; `graph_roofline` the neighbour
+           graph's build (4PCF, exports), timed beside the step
 cpu_baseline  the CPU restatement of the reference algorithm (kd-tree range
            search, id-sorted rows, the reference's 3PCF loop) on the host cores
 parity     the GPU result on the full catalogue against that CPU result
@@ -321,6 +322,13 @@ def _ev():
     return torch.cuda.Event(enable_timing=True)
 
 
+def graph_build_ms(ctx, st, stream, flush):
+    """Device time (ms) of the neighbour graph's build: the build call less the
+    index it starts with (`st`: the statistics of a count on this catalogue)."""
+    ms = timed(lambda: ctx._check(ctx._lib.gr_graph_build(ctx._h)), 8, stream, flush)
+    return max(1e-3, statistics.median(ms) - st["ms_index"])
+
+
 def timed(fn, steps, stream, flush=None):
     """Device time (ms) of `fn` per call, CUDA events on `stream`, L2 flushed
     before each call when `flush` is given."""
@@ -409,7 +417,7 @@ def run_ours(args):
     torch.cuda.synchronize()
     t_region0 = time.monotonic()
     ev = [(_ev(), _ev()) for _ in range(args.steps)]
-    q_ms, g_ms, tri, launches = [], [], 0, 0
+    q_ms, tri, launches = [], 0, 0
     st = None
     for k in range(args.steps):
         flush.zero_()
@@ -418,7 +426,6 @@ def run_ours(args):
         ev[k][1].record(stream)
         st = ctx.stats()
         q_ms.append(st["ms_query"])
-        g_ms.append(st["ms_graph"])
         tri += st["tuples"]
         launches += st["kernel_launches"]
     torch.cuda.synchronize()
@@ -449,17 +456,18 @@ def run_ours(args):
     # roofline of the triangle kernel (algorithmic bytes over its event time)
     # with its issue and shared-atomic rates, and of the graph build
     pk = roofline.peaks()
-    rf = roofline.tri3_roofline(ctx, q_ms, pk)
-    rf["traffic"] = roofline.profiled_traffic("tri3_kernel", args.scale)
+    ctx.count_3pcf(counts=False)
+    rf = roofline.root3_roofline(ctx, q_ms, pk)
+    rf["traffic"] = roofline.profiled_traffic("root3_kernel", args.scale)
     dev = device_info()
     sm_mhz = clocks.get("sm_mhz")
-    prof = roofline.profile("tri3_kernel", "c2") if args.scale == 1.0 else None
+    prof = roofline.profile("root3_kernel", "c2") if args.scale == 1.0 else None
     rf["issue"] = roofline.issue_roofline(prof, st["tuples"], rf["ms_per_launch"], sm_mhz, dev["sms"])
     rf["atomics"] = roofline.atomic_roofline(prof, st["tuples"], rf["ms_per_launch"], sm_mhz,
                                              dev["sms"])
     gprof = roofline.profile("csr_fill_kernel", "c2") if args.scale == 1.0 else None
     gtraffic = (float(gprof["dram_bytes_read"]) + float(gprof["dram_bytes_write"])) if gprof else None
-    grf = roofline.graph_roofline(st, float(np.mean(g_ms)), pk, gtraffic)
+    grf = roofline.graph_roofline(st, graph_build_ms(ctx, st, stream, flush), pk, gtraffic)
     grf["issue"] = roofline.issue_roofline(gprof, st["upper_edges"], grf["ms_per_launch"], sm_mhz,
                                            dev["sms"])
 
@@ -985,7 +993,7 @@ def run_shard(args):
     # call on the whole catalogue; every rank takes this step
     chk = step(counts=True)
     pk = roofline.peaks()
-    rf = roofline.tri3_roofline(ctx, q_ms, pk)
+    rf = roofline.root3_roofline(ctx, q_ms, pk)
     rf["of"] = "rank 0's slab"
     line = None
     if rank == 0:

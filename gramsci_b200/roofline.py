@@ -18,7 +18,8 @@ def peaks():
 
 
 def tri3_bytes(stats):
-    """Algorithmic bytes of one triangle-kernel launch.
+    """Algorithmic bytes of one launch of the hash-probe triangle kernel
+    (tri3_kernel, clique mode 1).
 
     Per upper edge (p, a): the root row entry (col + meta, 8 B) and the two
     row offsets of a (16 B).  Per probe (an entry c of the row of a looked up
@@ -36,6 +37,26 @@ def tri3_roofline(ctx, q_ms, pk):
     b = tri3_bytes(st)
     achieved = b / (ms * 1e-3) / 1e9
     return {"bound": "hbm", "kernel": "tri3_kernel", "achieved": achieved, "peak": pk["hbm_gbs"],
+            "unit": "GB/s", "frac": achieved / pk["hbm_gbs"], "traffic": None,
+            "bytes_per_launch": b, "ms_per_launch": ms, "peak_source": pk["source"]}
+
+
+def root3_bytes(stats):
+    """Algorithmic bytes of one rooted-triangle launch (root3_kernel).
+
+    Per candidate of a root's row: its FP32 position (16 B).  Per member kept
+    (upper edge): its weight, catalogue id and label (16 B).  The triangles run
+    on the row in shared memory.
+    """
+    return 16 * stats["candidates"] + 16 * stats["upper_edges"]
+
+
+def root3_roofline(ctx, q_ms, pk):
+    st = ctx.stats()
+    ms = sum(q_ms) / len(q_ms)
+    b = root3_bytes(st)
+    achieved = b / (ms * 1e-3) / 1e9
+    return {"bound": "hbm", "kernel": "root3_kernel", "achieved": achieved, "peak": pk["hbm_gbs"],
             "unit": "GB/s", "frac": achieved / pk["hbm_gbs"], "traffic": None,
             "bytes_per_launch": b, "ms_per_launch": ms, "peak_source": pk["source"]}
 
