@@ -270,25 +270,33 @@ class Context:
         self._check(self._lib.gr_regions_export(self._h, _ptr(off), _ptr(orig), _ptr(buf)))
         return [(orig[off[r]:off[r + 1]], buf[off[r]:off[r + 1]]) for r in range(nr.value)]
 
-    def _adjoint(self, fn, cot2, cot3, shape):
+    def _grad_out(self, out):
+        """Where a gradient goes: a new NumPy array, or `out`, a contiguous FP64
+        CUDA tensor of n entries on the context's device with no work pending."""
+        if out is None:
+            g = np.zeros(self.n)
+            return g, _ptr(g)
+        return out, ctypes.c_void_p(out.data_ptr())
+
+    def _adjoint(self, fn, cot2, cot3, shape, out=None):
         c2 = np.ascontiguousarray(np.asarray(cot2, np.float64).reshape(shape).T.ravel())
         c3 = None if cot3 is None else np.ascontiguousarray(
             np.asarray(cot3, np.float64).reshape(shape).T.ravel())
-        g = np.zeros(self.n)
-        self._check(fn(self._h, _ptr(c2), _ptr(c3), _ptr(g)))
+        g, p = self._grad_out(out)
+        self._check(fn(self._h, _ptr(c2), _ptr(c3), p))
         return g
 
-    def adjoint_2pcf(self, cot2, cot3=None):
+    def adjoint_2pcf(self, cot2, cot3=None, _out=None):
         """Gradient of sum(cot2*N2) + sum(cot3*N3) of the 2PCF with respect to
         the weights (catalogue order)."""
-        return self._adjoint(self._lib.gr_adjoint_2pcf, cot2, cot3, (self.nbins, self.nmu))
+        return self._adjoint(self._lib.gr_adjoint_2pcf, cot2, cot3, (self.nbins, self.nmu), _out)
 
-    def adjoint_3pcf(self, cot2, cot3=None):
+    def adjoint_3pcf(self, cot2, cot3=None, _out=None):
         """Gradient of sum(cot2*N2) + sum(cot3*N3) of the 3PCF with respect to
         the weights (catalogue order)."""
-        return self._adjoint(self._lib.gr_adjoint_3pcf, cot2, cot3, (ncfg3(self.nbins), self.nmu))
+        return self._adjoint(self._lib.gr_adjoint_3pcf, cot2, cot3, (ncfg3(self.nbins), self.nmu), _out)
 
-    def adjoint_4pcf(self, cot2, cot3=None, cotN=None, cotR=None):
+    def adjoint_4pcf(self, cot2, cot3=None, cotN=None, cotR=None, _out=None):
         """Gradient of sum(cot2*N2) + sum(cot3*N3) + sum(cotN*discN) +
         sum(cotR*discR) of the 4PCF with respect to the weights (catalogue
         order); cotangents in the shapes count_4pcf returns."""
@@ -302,9 +310,8 @@ class Context:
 
         c2, c3 = f(cot2, nc, nb, nb), f(cot3, nc, nb, nb)
         cN, cR = f(cotN, nc, nb, nb, 6), f(cotR, nc, nb, nb, 6)
-        g = np.zeros(self.n)
-        self._check(self._lib.gr_adjoint_4pcf(self._h, _ptr(c2), _ptr(c3), _ptr(cN), _ptr(cR),
-                                              _ptr(g)))
+        g, p = self._grad_out(_out)
+        self._check(self._lib.gr_adjoint_4pcf(self._h, _ptr(c2), _ptr(c3), _ptr(cN), _ptr(cR), p))
         return g
 
     def set_clique_mode(self, mode):

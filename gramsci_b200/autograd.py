@@ -79,7 +79,13 @@ class _PCF(torch.autograd.Function):
         if cots[0] is None:
             cots[0] = np.zeros(ctx.shapes[0])
         fn = {2: c.adjoint_2pcf, 3: c.adjoint_3pcf, 4: c.adjoint_4pcf}[ctx.order]
-        g = fn(*cots)
+        out = None
+        if w.is_cuda:
+            # the kernels write the gradient where it is needed; the library's
+            # stream is not torch's, so whatever last used this memory ends first
+            out = torch.empty(w.numel(), dtype=torch.float64, device=w.device)
+            torch.cuda.current_stream(w.device).synchronize()
+        g = fn(*cots, _out=out)
         return torch.as_tensor(g, dtype=w.dtype, device=w.device), None, None, None, None
 
 

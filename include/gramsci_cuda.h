@@ -97,11 +97,7 @@ const char* gr_last_error(const gr_ctx* ctx);
 
 /* Use a caller-owned CUDA stream (cudaStream_t passed as void*); NULL
  * restores the context's own stream.  Count calls wait on the stream for
- * their results, so they cannot be captured into a caller's CUDA graph.
- * Internally, a 2PCF or 3PCF count of a catalogue of the same size, box and
- * binning as the previous one replays that call's index (and graph)
- * phases as a CUDA graph the library captured on the context's own stream;
- * the replay is launched on the stream in use. */
+ * their results, so they cannot be captured into a caller's CUDA graph. */
 int gr_set_stream(gr_ctx* ctx, void* stream);
 
 /* Catalogue.  Replaces read_files_2's result (src/gramsci.F90:1364-1396):
@@ -247,7 +243,8 @@ int gr_regions_export(gr_ctx* ctx, int64_t* member_off, int32_t* member_orig,
 
 /* Weight adjoints.  Gradient of L = sum(cot2 * N2) + sum(cot3 * N3) with
  * respect to every signed normalised weight w_k (grad_w has N entries,
- * catalogue order).  cot2/cot3 have the shapes of N2/N3 of the matching
+ * catalogue order; host memory, or memory of the context's device, which is
+ * complete on return).  cot2/cot3 have the shapes of N2/N3 of the matching
  * count call; cot3 may be NULL.  The reference has no derivatives; these
  * differentiate the sums of query_graph_2pcf (src/gramsci.F90:362-379) and
  * query_graph_3pcf_all (:475-510): N2 and N3 are multilinear in the weights
