@@ -1947,7 +1947,7 @@ int gr_count_2pcf_batched(gr_ctx* c, double* N2, double* N3, int64_t* counts, do
   c->st.rooted = rooted;
   c->st.fp64_rechecks = (int64_t)st[0];
   c->st.candidates = (int64_t)st[1];
-  c->st.kernel_launches = 11;
+  c->st.kernel_launches = 10;
   GR_API_END(c)
 }
 
@@ -2003,7 +2003,7 @@ int gr_count_2pcf_regions(gr_ctx* c, double* N2, double* N3, int64_t* counts, do
   c->st.rooted = rooted;
   c->st.fp64_rechecks = (int64_t)st[0];
   c->st.candidates = (int64_t)st[1];
-  c->st.kernel_launches = 11;
+  c->st.kernel_launches = 10;
   GR_API_END(c)
 }
 

@@ -314,17 +314,27 @@ __global__ void b_members_kernel(const double* __restrict__ xyz, int n, int n_da
   }
 }
 
+// A member's point and flags at its cell's next place (any order in a cell).
 __global__ void b_scatter_kernel(int64_t m, const int* __restrict__ key, const int* __restrict__ slot,
-                                 const int64_t* __restrict__ start, int* __restrict__ tmp) {
+                                 const int* __restrict__ m_orig, const uint8_t* __restrict__ m_flag,
+                                 const int64_t* __restrict__ start, int2* __restrict__ tmp) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < m;
        k += (int64_t)gridDim.x * blockDim.x)
-    tmp[start[key[k]] + slot[k]] = (int)k;
+    tmp[start[key[k]] + slot[k]] = make_int2(m_orig[k], m_flag[k]);
 }
 
-// members of a cell ordered by catalogue index (deterministic layout)
-__global__ void b_order_kernel(int64_t ncell, const int64_t* __restrict__ start,
-                               const int* __restrict__ tmp, const int* __restrict__ m_orig,
-                               int* __restrict__ perm) {
+// One warp per cell: each member's rank by its point, then the member's data
+// at its place.  The record scattered above holds all that the ranking needs,
+// so the only reads out of order are the point's coordinates and weight, 80
+// bytes of sectors; with the members' indices scattered and ranked instead,
+// a permutation and four more arrays were read through it.  Bound by these
+// reads: 22.9M members, with the scatter, 3.4 -> 2.1 ms.
+__global__ void b_order_gather_kernel(int64_t ncell, const int64_t* __restrict__ start,
+                                      const int2* __restrict__ tmp, const double* __restrict__ xyz,
+                                      const double* __restrict__ w, float4* __restrict__ pos4,
+                                      double4* __restrict__ posd, double* __restrict__ wl,
+                                      int* __restrict__ orig, uint8_t* __restrict__ flags,
+                                      int* __restrict__ cell_key) {
   const int lane = threadIdx.x & 31;
   int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -332,43 +342,24 @@ __global__ void b_order_kernel(int64_t ncell, const int64_t* __restrict__ start,
     const int64_t b = start[c];
     const int cnt = (int)(start[c + 1] - b);
     for (int k = lane; k < cnt; k += 32) {
-      const int v = tmp[b + k];
-      const int ov = m_orig[v];
+      const int2 v = tmp[b + k];
+      const int i = v.x;
+      const double x = xyz[3 * (int64_t)i], y = xyz[3 * (int64_t)i + 1], z = xyz[3 * (int64_t)i + 2];
+      const double wi = w[i];
       int r = 0;
-      for (int j = 0; j < cnt; ++j) r += m_orig[tmp[b + j]] < ov;
-      perm[b + r] = v;
+      for (int j = 0; j < cnt; ++j) r += tmp[b + j].x < i;
+      const int64_t p = b + r;
+      pos4[p] = make_float4(__double2float_rn(x), __double2float_rn(y), __double2float_rn(z),
+                            pos4_flags((uint8_t)v.y));
+      posd[p] = make_double4(x, y, z, wi);
+      wl[p] = wi;
+      orig[p] = i;
+      flags[p] = (uint8_t)v.y;
+      cell_key[p] = (int)c;
     }
   }
 }
 
-__global__ void b_gather_kernel(int64_t m, const int* __restrict__ perm,
-                                const int* __restrict__ m_orig, const uint8_t* __restrict__ m_flag,
-                                const int* __restrict__ m_key, const double* __restrict__ xyz,
-                                const double* __restrict__ w, float4* __restrict__ pos4,
-                                double4* __restrict__ posd, double* __restrict__ wl,
-                                int* __restrict__ orig, uint8_t* __restrict__ flags,
-                                int* __restrict__ cell_key) {
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < m;
-       p += (int64_t)gridDim.x * blockDim.x) {
-    const int k = perm[p];
-    const int i = m_orig[k];
-    const double x = xyz[3 * (int64_t)i], y = xyz[3 * (int64_t)i + 1], z = xyz[3 * (int64_t)i + 2];
-    const uint8_t f = m_flag[k];
-    pos4[p] = make_float4(__double2float_rn(x), __double2float_rn(y), __double2float_rn(z),
-                          pos4_flags(f));
-    posd[p] = make_double4(x, y, z, w[i]);
-    wl[p] = w[i];
-    orig[p] = i;
-    flags[p] = f;
-    cell_key[p] = m_key[k];
-  }
-}
-
-__global__ void b_narrow_kernel(const int64_t* __restrict__ in, int* __restrict__ out, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = (int)in[i];
-}
 
 // blocks for n items, at most `waves` blocks per SM
 int nblocks(int64_t n, int threads, int waves = 8) {
@@ -592,8 +583,7 @@ void RegionLayout::plan(const double* d_xyz, int64_t n_pts, int64_t n_data_pts,
   m_flag.reserve(M + 1);
   m_key.reserve(M + 1);
   m_slot.reserve(M + 1);
-  tmp_perm.reserve(M + 1);
-  perm.reserve(M + 1);
+  tmp_rec.reserve(M + 1);
   cell_count.reserve(ncell + 1);
   cell_start64.reserve(ncell + 1);
   cell_start.reserve(ncell + 1);
@@ -619,17 +609,14 @@ void RegionLayout::enqueue_layout(const double* d_xyz, const double* d_w, cudaSt
     launch_members(2, d_xyz, G, s);
   }
   GR_CHECK_LAUNCH();
-  scan_i32_to_i64(cell_count.p, cell_start64.p, ncell, s, scan_tmp);
+  scan_i32_to_i64(cell_count.p, cell_start64.p, ncell, s, scan_tmp, cell_start.p);
   if (n_members > 0) {
-    b_scatter_kernel<<<nblocks(n_members, 256), 256, 0, s>>>(n_members, m_key.p, m_slot.p,
-                                                             cell_start64.p, tmp_perm.p);
-    b_order_kernel<<<nblocks(ncell * 32, 256, 16), 256, 0, s>>>(ncell, cell_start64.p,
-                                                                      tmp_perm.p, m_orig.p, perm.p);
-    b_gather_kernel<<<nblocks(n_members, 256), 256, 0, s>>>(n_members, perm.p, m_orig.p, m_flag.p,
-                                                            m_key.p, d_xyz, d_w, pos4.p, posd.p,
-                                                            w.p, orig.p, flags.p, cell_key.p);
+    b_scatter_kernel<<<nblocks(n_members, 256), 256, 0, s>>>(n_members, m_key.p, m_slot.p, m_orig.p,
+                                                             m_flag.p, cell_start64.p, tmp_rec.p);
+    b_order_gather_kernel<<<nblocks(ncell * 32, 256, 16), 256, 0, s>>>(
+        ncell, cell_start64.p, tmp_rec.p, d_xyz, d_w, pos4.p, posd.p, w.p, orig.p, flags.p,
+        cell_key.p);
   }
-  b_narrow_kernel<<<nblocks(ncell + 1, 256), 256, 0, s>>>(cell_start64.p, cell_start.p, ncell + 1);
   GR_CHECK_LAUNCH();
 }
 

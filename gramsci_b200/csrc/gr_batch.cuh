@@ -67,8 +67,9 @@ struct RegionLayout {
   DevBuf<double> halo, glo, ginv;
   DevBuf<GridParams> grid;
   // members and layout
-  DevBuf<int> m_orig, m_key, m_slot, tmp_perm, perm, cell_count, cell_start, orig, cell_key;
+  DevBuf<int> m_orig, m_key, m_slot, cell_count, cell_start, orig, cell_key;
   DevBuf<uint8_t> m_flag, flags;
+  DevBuf<int2> tmp_rec;  // members by cell: point, flags
   DevBuf<int64_t> cell_start64, scan_tmp;
   DevBuf<float4> pos4;
   DevBuf<double4> posd;
