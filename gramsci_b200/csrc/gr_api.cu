@@ -12,6 +12,7 @@
 #include <mutex>
 #include <new>
 #include <sys/stat.h>
+#include <cuda.h>
 #include <string>
 #include <vector>
 
@@ -494,6 +495,32 @@ int gr_set_stream(gr_ctx* c, void* stream) {
   GR_API_END(c)
 }
 
+// Whether kernels of this context may use `bytes` at p directly: memory of its
+// device, inside one allocation, aligned to `align`.  Anything else is left to
+// a copy, which handles other devices and pinned memory and reports the rest.
+static bool device_range(const gr_ctx* c, const void* p, size_t bytes, size_t align) {
+  typedef CUresult (*RangeFn)(CUdeviceptr*, size_t*, CUdeviceptr);
+  static const RangeFn range = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult r;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &r) !=
+            cudaSuccess ||
+        r != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<RangeFn>(f);
+  }();
+  if (bytes == 0) return true;
+  cudaPointerAttributes at{};
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const CUdeviceptr q = (CUdeviceptr)(uintptr_t)p;
+  const bool ok = p && range && q % align == 0 && cudaPointerGetAttributes(&at, p) == cudaSuccess &&
+                  at.type == cudaMemoryTypeDevice && at.device == c->device &&
+                  range(&base, &size, q) == CUDA_SUCCESS && q - base <= size && bytes <= size - (q - base);
+  cudaGetLastError();  // a pointer unknown to CUDA is no error here
+  return ok;
+}
+
 static int set_catalog_impl(gr_ctx* c, const double* xyz, const double* w, const int32_t* buffer,
                             int64_t n_data, int64_t n_rand, cudaMemcpyKind kind) {
   GR_API_BEGIN(c)
@@ -513,14 +540,17 @@ static int set_catalog_impl(gr_ctx* c, const double* xyz, const double* w, const
   c->scan.reserve(1);
   CatalogScan& h = *c->scan.p;
   std::memset(&h, 0, sizeof(h));
-  const bool host = kind == cudaMemcpyHostToDevice;
-  if (host && n > 0) {
+  // device arrays are copied by the scan itself
+  const bool direct = kind == cudaMemcpyDeviceToDevice &&
+                      device_range(c, xyz, sizeof(double) * 3 * n, sizeof(double)) &&
+                      device_range(c, w, sizeof(double) * n, sizeof(double)) &&
+                      device_range(c, buffer, buffer ? sizeof(int32_t) * n : 0, sizeof(int32_t));
+  if (!direct && n > 0) {
     GR_CUDA_TRY(cudaMemcpyAsync(c->xyz.p, xyz, sizeof(double) * 3 * n, kind, s));
     GR_CUDA_TRY(cudaMemcpyAsync(c->w.p, w, sizeof(double) * n, kind, s));
     if (buffer) GR_CUDA_TRY(cudaMemcpyAsync(c->buffer.p, buffer, sizeof(int32_t) * n, kind, s));
   }
-  // device arrays are copied by the scan itself
-  scan_catalog(host ? c->xyz.p : xyz, host ? c->w.p : w, buffer, n_data, n, c->xyz.p, c->w.p,
+  scan_catalog(direct ? xyz : c->xyz.p, direct ? w : c->w.p, buffer, n_data, n, c->xyz.p, c->w.p,
                c->buffer.p, c->scan_part, c->scan.p, c->box, s);
   if (h.word[8] & kScanWeightBad) {
     c->cat_set = false;  // nothing may be counted on a half-set catalogue
@@ -778,10 +808,7 @@ int gr_count_2pcf(gr_ctx* c, double* N2, double* N3, int64_t* counts, double* ca
 // 4PCF workload: unit weights 4.97 -> 4.34 ms, lognormal weighted sums 9.86
 // -> 8.23 ms, adjoint 12.9 -> 9.3 ms (the last roots of a block no longer
 // keep its other warps waiting at the final barrier, nor the launch waiting
-// on one heavy root).  The triangle kernel keeps label order: on the 3PCF
-// workload the order cost 0.04 ms (0.765 against 0.723 ms: the sort, and
-// neighbouring roots no longer sharing their rows in L1), and the 3M-point
-// adjoint catalogue gained nothing (398 against 396 ms, 852 against 849 ms).
+// on one heavy root); the ordering itself takes 22 us beside 1.39 ms now.
 constexpr int kRootOrderLaunches = 3;  // kernels of order_roots_by_length
 static const int* root_order(gr_ctx* c, cudaStream_t s, const int** above = nullptr,
                              int* nclass = nullptr) {
@@ -1015,9 +1042,8 @@ int gr_count_equi(gr_ctx* c, double* N2, double* N3, int64_t* counts, double* ca
 
 // Edges among R+(p) in the 4-clique kernels: the geometric pair test (rows
 // up to 255 members) or hash probes of the members' rows.  Measured on the
-// 4PCF workload (upper degree 17.5): unit weights 5.0 ms geometric against
-// 6.3 ms, lognormal weighted sums 9.8 against 10.8 ms, adjoint 13.0 against
-// 15.3 ms.
+// 4PCF workload (upper degree 17.5): unit weights 1.38 ms geometric against
+// 4.05 ms, lognormal weighted sums 3.1 against 7.4 ms.
 static int quad_geometric(const gr_ctx* c, int64_t max_deg, int nbins) {
   return (max_deg > 255 || nbins > 255 || c->clique_mode == 1) ? 0 : 1;
 }
@@ -1491,10 +1517,7 @@ static double max_abs(const double* a, int64_t n) {
 static void finish_grad(gr_ctx* c, double gscale, double* grad_w, cudaEvent_t q0) {
   cudaStream_t s = c->stream();
   const int64_t n = c->n;
-  cudaPointerAttributes at{};
-  const bool dev = grad_w && cudaPointerGetAttributes(&at, grad_w) == cudaSuccess &&
-                   at.type == cudaMemoryTypeDevice && at.device == c->device;
-  cudaGetLastError();  // a host pointer unknown to CUDA is no error
+  const bool dev = n > 0 && device_range(c, grad_w, sizeof(double) * n, sizeof(double));
   if (!dev) c->grad.reserve(n + 1);
   launch_grad_finish((int)n, c->index.orig.p, c->gfix.p, c->gfix.p + n, gscale,
                      dev ? grad_w : c->grad.p, s);

@@ -104,3 +104,33 @@ def test_non_finite_is_refused_where_it_was(dev):
         ctx.count_2pcf()
     ctx.set_catalog(put(xyz), put(w), n_data)
     assert np.asarray(ctx.count_2pcf()["counts"]).sum() > 0
+
+
+@pytest.mark.parametrize("n,pinned", [(700, True), (700, False), (5000, True)])
+def test_device_entry_takes_what_a_copy_takes(n, pinned):
+    """gr_set_catalog_dev: device arrays are read in place, also from the
+    middle of an allocation; pinned host memory, which a device-to-device copy
+    accepts, is still copied."""
+    import ctypes
+
+    from gramsci_b200.api import Context
+
+    xyz, w, n_data, _ = _catalogue(n, 11)
+    ctx = Context()
+    ctx.set_bins(RMIN, RMAX, 4)
+    ctx.set_catalog(xyz, w, n_data)
+    want = ctx.count_2pcf()
+    if pinned:
+        x, v = torch.from_numpy(xyz).pin_memory(), torch.from_numpy(w).pin_memory()
+    else:
+        room = torch.zeros(4 * n + 7, dtype=torch.float64, device="cuda")
+        x, v = room[3:3 + 3 * n], room[5 + 3 * n:5 + 4 * n]
+        x.copy_(torch.from_numpy(xyz.ravel()))
+        v.copy_(torch.from_numpy(w))
+        torch.cuda.synchronize()
+    ctx._check(ctx._lib.gr_set_catalog_dev(ctx._h, ctypes.c_void_p(x.data_ptr()),
+                                           ctypes.c_void_p(v.data_ptr()), None, n_data, n - n_data))
+    ctx.n = n
+    got = ctx.count_2pcf()
+    for k in want:
+        np.testing.assert_array_equal(want[k], got[k])
