@@ -40,12 +40,13 @@ enum {
 constexpr double kDenseCellPoints = 64.0;
 size_t pair2_smem_bytes(const PairParams& P, bool weighted);
 
-// Tile sweep for dense cells (gr_tile.cu): warp per cell, lanes over 32
-// roots, candidates staged 32 at a time per warp and tested two per packed
-// FP32x2 instruction (FP64 path: one per FP64 test), hits binned from a
-// per-warp queue; reads grids with cells at least rmax wide (sub 1) or rmax/2
-// wide (sub 2).  Same inputs, outputs and results as launch_pair2.
-// Histograms private to each warp in shared memory when they need at most
+// Tile sweep (gr_tile.cu): a warp takes a cell's points 32 at a time as roots
+// (chunks run across the cells of an x-row), candidates staged 32 at a time
+// per warp and tested two per packed FP32x2 instruction (FP64 path: one per
+// FP64 test), hits binned from a per-warp queue, one update per pair; reads
+// grids with cells at least rmax wide (sub 1) or rmax/2 wide (sub 2).  Same
+// inputs, outputs and results as launch_pair2.
+// Tables private to each warp in shared memory when they need at most
 // kMaxTileHistSmem bytes.  per_region (region layouts only): one histogram
 // per region, g_cnt nregions*nh and g_fix nregions*2*nh (region r's lo
 // words at 2*r*nh, hi words at 2*r*nh + nh), all zeroed.

@@ -5,9 +5,10 @@
 // graph does: root p with mu(p->q) if p is not a buffer point, root q with
 // mu(q->p) if q is not.
 //
-// Histograms are privatised per block in shared memory: 64-bit counts per
-// (bin, mu, category) and, for weighted catalogues, 128-bit fixed-point sums
-// of w_i w_j per category (see fix_add).
+// Histograms are privatised per block in shared memory: counts per (bin, mu,
+// category) in two 32-bit words and, for weighted catalogues, 128-bit
+// fixed-point sums of w_i w_j per category in four (hist_count_add,
+// hist_fix_add).
 #include "gr_kernels.cuh"
 
 namespace gr {

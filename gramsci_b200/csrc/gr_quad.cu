@@ -22,7 +22,7 @@
 // A second kernel (quad4g_kernel, the geometric mode) finds the edges among
 // the members of R+(p) with the graph's own membership test on their
 // positions instead of probing the members' rows; it is used whenever the
-// rows fit (up to 256 members).
+// rows fit (up to 255 members).
 #include <algorithm>
 #include <type_traits>
 

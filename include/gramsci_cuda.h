@@ -54,18 +54,18 @@ typedef struct gr_ctx gr_ctx;
                                cell with queued binning, 4/5 block per cell of 128/256 with
                                queued binning, 6 the tile sweep, 7 the tile sweep on cells
                                of rmax/2) */
-#define GR_OPT_KEEP_GRAPH 4 /* 0 (default): every count call builds the index and graph;
-                               1: keep the graph of the last call and reuse it until the
-                               catalogue, the bins or the precision change */
+#define GR_OPT_KEEP_GRAPH 4 /* 0 (default): every count call builds the index, and the
+                               graph if it reads one; 1: keep those of the last call and
+                               reuse them until the catalogue, the bins or the precision
+                               change */
 #define GR_OPT_CLIQUE_MODE 5 /* how the 3PCF / 4PCF kernels find the edges among a root's
                                larger-label neighbours: 0 automatic (default: mode 2 wherever
-                               the rows allow it), 1 hash probes of the neighbours' rows, 2
-                               the graph's membership test on the pairs of neighbours.
-                               4PCF: mode 2 takes rows up to 256
-                               neighbours (longer rows use 1).  3PCF: rows longer than 256
-                               neighbours take a second launch in mode 2 (up to 1024, then a
-                               global-memory path) unless mode 1 is forced.  Results are
-                               identical; only speed differs */
+                               the rows allow it), 1 hash probes of the neighbours' rows in
+                               the graph, 2 the graph's membership test on the pairs of
+                               neighbours.  3PCF: mode 2 needs the cell index alone and
+                               builds no graph; rows beyond a warp's capacity take a second
+                               launch.  4PCF: mode 2 takes rows up to 255 neighbours (longer
+                               rows use 1).  Results are identical; only speed differs */
 
 /* Run statistics of the last count call (gr_get_stats). */
 typedef struct gr_stats {
@@ -83,7 +83,7 @@ typedef struct gr_stats {
   int64_t probes;         /* intersection probes (3PCF/4PCF): neighbour-row entries
                              looked up in the root's row, or in the geometric
                              clique mode the pairs of the root's neighbours tested */
-  int64_t upper_edges;    /* undirected edges stored in the upper CSR            */
+  int64_t upper_edges;    /* undirected edges met (3PCF, 4PCF)                   */
 } gr_stats;
 
 /* Library version string. */
@@ -178,7 +178,8 @@ int gr_graph_export(gr_ctx* ctx, int64_t* row_ptr, int32_t* col, uint8_t* bin, u
  * one back for the same catalogue positions and bins -- it checks the point
  * count, the binning and a 64-bit fingerprint of the coordinates, and returns
  * GR_E_ARG on a mismatch -- after which the 2/3/4PCF, -equi and -tetra calls
- * reuse it (no graph build) until the catalogue, bins or precision change.
+ * reuse it, or the index beside it (neither is built again), until the
+ * catalogue, bins or precision change.
  * File: a 128-byte header ("GRAMSCSR", version 1, n, upper edges, max upper
  * degree, rmin, rmax, nbins, nmu, logbins, coordinate fingerprint, payload
  * checksum, labelling fingerprint), then row_ptr int64[n+1], records uint64[edges], full degree
@@ -196,8 +197,9 @@ int gr_graph_load(gr_ctx* ctx, const char* path);
  * all regions in one launch (cells of every region from one work queue,
  * largest region first), with the global galaxy/random flags and weight
  * normalisation, so the result equals gr_count_2pcf on the whole catalogue.
- * The first call for a catalogue/binning/split plans the layout and captures
- * the device work in a CUDA graph; later calls replay it.  Outputs as
+ * The first call for a catalogue/binning/split plans the layout and runs it;
+ * the second captures the device work in a CUDA graph, which later calls
+ * replay.  Outputs as
  * gr_count_2pcf.  gr_regions_info / gr_regions_export describe the layout
  * (member_off: nregions+1 offsets; per member its catalogue index and 1 if it
  * is a buffer point), e.g. to run the regions one launch at a time. */
@@ -250,8 +252,9 @@ int gr_regions_export(gr_ctx* ctx, int64_t* member_off, int32_t* member_orig,
  * query_graph_3pcf_all (:475-510): N2 and N3 are multilinear in the weights
  * (each point appears at most once per pair or triangle), so
  * dN2_b/dw_k = sum over the rooted pairs/triangles in bin b that contain k of
- * the product of the other weights.  gr_adjoint_3pcf reuses the graph of the
- * last count or graph build when the catalogue and bins are unchanged.
+ * the product of the other weights.  The adjoints reuse the index (4PCF: the
+ * graph) of the last count or graph build when the catalogue and bins are
+ * unchanged.
  * Gradients are accumulated in 128-bit fixed point: deterministic. */
 int gr_adjoint_2pcf(gr_ctx* ctx, const double* cot2, const double* cot3, double* grad_w);
 int gr_adjoint_3pcf(gr_ctx* ctx, const double* cot2, const double* cot3, double* grad_w);
