@@ -530,6 +530,7 @@ static int set_catalog_impl(gr_ctx* c, const double* xyz, const double* w, const
   if (n > 0 && (!xyz || !w)) return set_err(c, GR_E_ARG, "null xyz or w");
   cudaStream_t s = c->stream();
   c->cat_gen++;
+  c->cat_set = false;  // nothing may be counted on a half-set catalogue
   c->xyz.reserve(3 * n + 1);
   c->w.reserve(n + 1);
   c->has_buffer = buffer != nullptr;
@@ -552,10 +553,7 @@ static int set_catalog_impl(gr_ctx* c, const double* xyz, const double* w, const
   }
   scan_catalog(direct ? xyz : c->xyz.p, direct ? w : c->w.p, buffer, n_data, n, c->xyz.p, c->w.p,
                c->buffer.p, c->scan_part, c->scan.p, c->box, s);
-  if (h.word[8] & kScanWeightBad) {
-    c->cat_set = false;  // nothing may be counted on a half-set catalogue
-    return set_err(c, GR_E_ARG, "non-finite weights");
-  }
+  if (h.word[8] & kScanWeightBad) return set_err(c, GR_E_ARG, "non-finite weights");
   std::memcpy(&c->wgmax, &h.word[6], 8);
   std::memcpy(&c->wrmax, &h.word[7], 8);
   c->wmax = std::max(c->wgmax, c->wrmax);
