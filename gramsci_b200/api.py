@@ -97,6 +97,11 @@ class Context:
             w = w.detach().to(torch.float64).contiguous()
             buf = None if buffer is None else buffer.detach().to(torch.int32).contiguous()
             n = xyz.shape[0]
+            # the library reads n entries of each by their addresses
+            if xyz.numel() != 3 * n:
+                raise ValueError("xyz must have three coordinates per point")
+            if w.numel() < n or (buf is not None and buf.numel() < n):
+                raise ValueError("w and buffer must have one entry per point")
             self._keep = (xyz, w, buf)
             self.n = int(n)
             self._check(self._lib.gr_set_catalog_dev(
@@ -276,6 +281,12 @@ class Context:
         if out is None:
             g = np.zeros(self.n)
             return g, _ptr(g)
+        import torch
+
+        if (out.dtype != torch.float64 or not out.is_cuda or out.device.index != self.device
+                or out.numel() != self.n or not out.is_contiguous()):
+            raise ValueError("the gradient needs a contiguous float64 CUDA tensor with one entry "
+                             "per point on the context's device")
         return out, ctypes.c_void_p(out.data_ptr())
 
     def _adjoint(self, fn, cot2, cot3, shape, out=None):

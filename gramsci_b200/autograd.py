@@ -82,8 +82,10 @@ class _PCF(torch.autograd.Function):
         out = None
         if w.is_cuda:
             # the kernels write the gradient where it is needed; the library's
-            # stream is not torch's, so whatever last used this memory ends first
-            out = torch.empty(w.numel(), dtype=torch.float64, device=w.device)
+            # stream is not torch's, so whatever last used this memory ends first.
+            # One entry per point of the catalogue, whatever w's length: torch
+            # refuses a gradient that does not fit w
+            out = torch.empty(c.n, dtype=torch.float64, device=w.device)
             torch.cuda.current_stream(w.device).synchronize()
         g = fn(*cots, _out=out)
         return torch.as_tensor(g, dtype=w.dtype, device=w.device), None, None, None, None
