@@ -1508,8 +1508,9 @@ static double max_abs(const double* a, int64_t n) {
   return m;
 }
 
-// Gradient in catalogue order to grad_w: host memory through c->grad, or
-// memory of this device directly.  The read-back of 3M gradients into pageable
+// Gradient in catalogue order to grad_w: memory of this device directly, or
+// through c->grad (host memory, and device memory that device_range declines:
+// the copy's direction is left to the address).  The read-back of 3M gradients into pageable
 // memory, with the copy to the device that a caller there made of it, took 5
 // of the 25.5 ms of a weighted 2PCF with its gradient.
 static void finish_grad(gr_ctx* c, double gscale, double* grad_w, cudaEvent_t q0) {
@@ -1521,7 +1522,7 @@ static void finish_grad(gr_ctx* c, double gscale, double* grad_w, cudaEvent_t q0
                      dev ? grad_w : c->grad.p, s);
   GR_CUDA_TRY(cudaEventRecord(c->ev[3], s));
   if (n > 0 && !dev)
-    GR_CUDA_TRY(cudaMemcpyAsync(grad_w, c->grad.p, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
+    GR_CUDA_TRY(cudaMemcpyAsync(grad_w, c->grad.p, sizeof(double) * n, cudaMemcpyDefault, s));
   GR_CUDA_TRY(cudaStreamSynchronize(s));
   c->st.ms_query = ev_ms(q0, c->ev[3]);
 }
