@@ -530,7 +530,19 @@ static int set_catalog_impl(gr_ctx* c, const double* xyz, const double* w, const
   if (n > 0 && (!xyz || !w)) return set_err(c, GR_E_ARG, "null xyz or w");
   cudaStream_t s = c->stream();
   c->cat_gen++;
-  c->cat_set = false;  // nothing may be counted on a half-set catalogue
+  // nothing may be counted or exported on a half-set catalogue: what was
+  // derived from the previous one goes before its size does
+  c->cat_set = false;
+  c->csr_valid = false;
+  c->index_valid = false;
+  c->graph_loaded = false;
+  c->regions.valid = false;
+  // region ids and mocks describe the points of the previous catalogue
+  if (c->region_mode >= 2) {
+    c->regions.set_split();
+    c->regions.release_graph();
+    c->region_mode = c->nsplit > 0 ? 1 : 0;
+  }
   c->xyz.reserve(3 * n + 1);
   c->w.reserve(n + 1);
   c->has_buffer = buffer != nullptr;
@@ -563,16 +575,6 @@ static int set_catalog_impl(gr_ctx* c, const double* xyz, const double* w, const
   c->w_gal = h.w0[0];
   c->w_ran = h.w0[1];
   c->cat_set = true;
-  c->csr_valid = false;
-  c->index_valid = false;
-  c->graph_loaded = false;
-  c->regions.valid = false;
-  // region ids and mocks describe the points of the previous catalogue
-  if (c->region_mode >= 2) {
-    c->regions.set_split();
-    c->regions.release_graph();
-    c->region_mode = c->nsplit > 0 ? 1 : 0;
-  }
   GR_API_END(c)
 }
 
@@ -1443,8 +1445,8 @@ int gr_graph_load(gr_ctx* c, const char* path) {
 int gr_graph_nedges(gr_ctx* c, int64_t* n_edges) {
   GR_API_BEGIN(c)
   if (!n_edges) return set_err(c, GR_E_ARG, "null output");
+  require_ready(c);
   if (!c->csr_valid) {
-    require_ready(c);
     build_index(c);
     build_csr(c);
   }
@@ -1454,8 +1456,8 @@ int gr_graph_nedges(gr_ctx* c, int64_t* n_edges) {
 
 int gr_graph_export(gr_ctx* c, int64_t* row_ptr, int32_t* col, uint8_t* bin, uint8_t* mu) {
   GR_API_BEGIN(c)
+  require_ready(c);
   if (!c->csr_valid) {
-    require_ready(c);
     build_index(c);
     build_csr(c);
   }
