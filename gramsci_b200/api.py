@@ -42,6 +42,19 @@ def _is_torch_cuda(x):
     return hasattr(x, "is_cuda") and hasattr(x, "data_ptr") and x.is_cuda
 
 
+def _wait_for(*tensors):
+    """Until torch's current stream has computed the CUDA tensors: the library
+    reads them on a stream of its own, which is not ordered after torch's."""
+    import torch
+
+    if torch.cuda.is_current_stream_capturing():
+        return  # nothing runs that could be waited for
+    for device in {t.device for t in tensors if t is not None and t.is_cuda}:
+        stream = torch.cuda.current_stream(device)
+        if not stream.query():
+            stream.synchronize()
+
+
 class Context:
     """One library context (device state, catalogue, binning)."""
 
@@ -103,6 +116,7 @@ class Context:
             if w.numel() < n or (buf is not None and buf.numel() < n):
                 raise ValueError("w and buffer must have one entry per point")
             self._keep = (xyz, w, buf)
+            _wait_for(*self._keep)
             self.n = int(n)
             self._check(self._lib.gr_set_catalog_dev(
                 self._h, ctypes.c_void_p(xyz.data_ptr()), ctypes.c_void_p(w.data_ptr()),

@@ -54,7 +54,8 @@ def test_short_inputs_are_refused(args):
 
 
 @pytest.mark.parametrize("args", [(4,), (4, 6), (4, 4, 4), (0,)], ids=["plain", "long-w", "buffer", "empty"])
-def test_inputs_that_fit_are_taken(args):
+def test_inputs_that_fit_are_taken(monkeypatch, args):
+    monkeypatch.setattr(api, "_wait_for", lambda *tensors: None)  # no stream here
     ctx = context()
     ctx.set_catalog(*catalogue(*args))
     assert ctx.n == args[0] and ctx._lib.log == ["gr_set_catalog_dev"]
