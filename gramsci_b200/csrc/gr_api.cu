@@ -1597,7 +1597,7 @@ static int pick_adj2_layout(gr_ctx* c, const DevCatalog& C, const double* c2, co
 int gr_adjoint_2pcf(gr_ctx* c, const double* cot2, const double* cot3, double* grad_w) {
   GR_API_BEGIN(c)
   require_ready(c);
-  if (!cot2 || !grad_w) return set_err(c, GR_E_ARG, "null cot2 or grad_w");
+  if (!cot2 || (!grad_w && c->n > 0)) return set_err(c, GR_E_ARG, "null cot2 or grad_w");
   ensure_events(c);
   cudaStream_t s = c->stream();
   const int nbm = c->nbins * c->nmu;
@@ -1654,7 +1654,7 @@ int gr_adjoint_2pcf(gr_ctx* c, const double* cot2, const double* cot3, double* g
 int gr_adjoint_3pcf(gr_ctx* c, const double* cot2, const double* cot3, double* grad_w) {
   GR_API_BEGIN(c)
   require_ready(c);
-  if (!cot2 || !grad_w) return set_err(c, GR_E_ARG, "null cot2 or grad_w");
+  if (!cot2 || (!grad_w && c->n > 0)) return set_err(c, GR_E_ARG, "null cot2 or grad_w");
   ensure_events(c);
   cudaStream_t s = c->stream();
   const int nmu = c->nmu;
@@ -1731,7 +1731,7 @@ int gr_adjoint_4pcf(gr_ctx* c, const double* cot2, const double* cot3, const dou
                     const double* cotR, double* grad_w) {
   GR_API_BEGIN(c)
   require_ready(c);
-  if (!cot2 || !grad_w) return set_err(c, GR_E_ARG, "null cot2 or grad_w");
+  if (!cot2 || (!grad_w && c->n > 0)) return set_err(c, GR_E_ARG, "null cot2 or grad_w");
   ensure_events(c);
   cudaStream_t s = c->stream();
   const int nb = c->nbins;
