@@ -1703,7 +1703,12 @@ int gr_adjoint_3pcf(gr_ctx* c, const double* cot2, const double* cot3, double* g
   } else {
     c->long_list.reserve(n + 1);
     c->stage.reserve(kRootStats);
-    const RootParams T = root_params(c, false, ncfg, n, box_volume(c->index.box));
+    RootParams T = root_params(c, false, ncfg, n, box_volume(c->index.box));
+    double most = 0.0;
+    for (int k = 0; k < nc; ++k)
+      most = std::max(most, std::max(std::fabs(cot2[k]), cot3 ? std::fabs(cot2[k] - cot3[k]) : 0.0));
+    T.rscale = fix_scale(3.0 * most * c->wmax);
+    T.winv = 0x1p20 / c->wmax;
     auto run = [&](const RootLong* R) {
       launch_root3_adj(c->index.view(), T, c->cot.p, dc3, gscale, c->gfix.p, c->gfix.p + n,
                        c->stats.p, c->work.p, c->long_list.p, R, s);

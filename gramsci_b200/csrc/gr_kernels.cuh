@@ -90,6 +90,9 @@ struct RootParams {
   const uint8_t* normal;  // device find_normal table [mu1-1 + nmu*(mu2-1)]
   RankTables rank;        // 3-tuple ranks
   double fscale[4];       // fixed-point scale of the products with 0..3 randoms
+  // adjoint: fix_scale of the largest coefficient of a triangle (its three
+  // roots' cotangents) times the largest weight, and 2^20 over that weight
+  double rscale, winv;
   PairParams P;
 };
 // Second launch for the listed rows: n of them, at most cap members each, in

@@ -28,13 +28,23 @@
 // shared words, and no pair index is inverted.  The last x's of a row, fewer than 32, share the warp:
 // groups of lanes hold the same x's and take every G-th step.
 //
-// ADJ: the weight gradient.  Without mu bins the pair's coefficient times the
-// weight of y is summed in the lane that holds x, times the weight of x in y's
-// shared accumulator (each y belongs to one lane per step, so plain reads and
-// writes do, a warp barrier between steps), both in FP64; a row's sums, times
-// the root's weight, go to the 128-bit fixed-point totals once.  With mu bins
-// the queued hits add to signed 64-bit fixed-point sums per neighbour (the
-// scale leaves room for 1024 terms).
+// ADJ: the weight gradient, every sum of it an integer.  Without mu bins the
+// pair's coefficient times the weight of y is summed in the lane that holds x,
+// times the weight of x in y's shared accumulator (each y belongs to one lane
+// per step, so plain reads and writes do, a warp barrier between steps), both
+// in signed 64-bit fixed point with room for the row's weights and no more
+// (T.rscale in the cotangents' table, for a full row of the largest weight, and
+// a power of two in the row's weights); a row's sums, times the root's weight,
+// go to the 128-bit fixed-point totals once.  With mu bins the queued hits add
+// to signed 64-bit fixed-point sums per neighbour (the scale leaves room for
+// 1024 terms).  The root's own sum has 128 bits.  Rounding of an entry without
+// mu bins, rms in units of 2^-53 of the sum of its terms' sizes, lognormal and
+// equal weights: rows of 14 members 0.21 and 0.22, of 170 0.03 and 0.03, of 600
+// 0.13 and 0.35 (positive cotangents 0.6).  FP64 sums in their place: 0.22 and
+// 0.21, 0.05 and 0.10, 0.12 and 0.96 (12: equal terms round alike); terms
+// rounded at the totals' scale, as the hash-probe kernel does: 67 and 13, 3.4
+// and 5.0, 0.6 and 3.6 (2.6).  The integers cost 76.8 -> 78.5 ms on 600,000
+// points with rows of 170.
 //
 // Rows longer than a warp's capacity are listed and taken by a second launch
 // (LONG) with one block per root and the row in global memory; its adjoint
@@ -44,7 +54,7 @@
 // the limit; DRAM idle): about 100 warp instructions per 32 pairs without mu
 // bins, half of which are triangles.  Against the graph build and the triangle
 // kernel over its rows: 600,000 points with rows of 170, gradient and sums
-// 153 -> 77 ms; 160,000 points with rows of 14, 346 -> 222 us; 400,000 points
+// 153 -> 79 ms; 160,000 points with rows of 14, 346 -> 222 us; 400,000 points
 // with 5 mu bins and rows of 14, 800 -> 720 us, of which collecting the rows
 // takes 250, the pair tests 180 and the binning of the triangles 290.
 #include <algorithm>
@@ -80,7 +90,7 @@ struct GroupRoot {
 struct RowPtrs {
   float4* pos;
   double* w;
-  double* g;  // ADJ: gradient over the root's weight (MU: 64-bit integers)
+  unsigned long long* g;  // ADJ: 64-bit fixed-point gradient (not MU: over the root's weight)
   int* q;     // labels
   int* id;    // catalogue ids (MU with an asymmetric normal table)
 };
@@ -147,6 +157,15 @@ __device__ __forceinline__ Fix128 fix_from_double(double x) {
   return v;
 }
 
+// 2^e, and the number of bits that n - 1 takes (n > 0: the least e with 2^e >= n).
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+__device__ __forceinline__ int bits_of(int n) { return 32 - __clz(max(n, 1) - 1); }
+
+__device__ __forceinline__ void fix_plus(Fix128& a, const Fix128& b) {
+  a.lo += b.lo;
+  a.hi += b.hi + (a.lo < b.lo ? 1ull : 0ull);
+}
+
 template <bool MU, bool WEIGHTED, bool COUNTS, bool SHIST, bool ADJ, bool BUF, bool LONG>
 __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG ? 5 : 1)
     root3_kernel(DevCatalog C, RootParams T, unsigned long long* __restrict__ g_cnt,
@@ -156,6 +175,7 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
                  unsigned long long* __restrict__ g_lo, unsigned long long* __restrict__ g_hi) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr bool W = WEIGHTED || ADJ;
+  constexpr bool ROWSUM = ADJ && (!MU || LONG);  // sums over the root's weight, at T.rscale
   const PairParams& P = T.P;
   const int nb = T.nbins, ncfg = T.ncfg;
   const int nbin = ncfg * T.nmu, nh = nbin * 4;
@@ -188,7 +208,7 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
   if (ADJ)
     for (int k = threadIdx.x; k < nbin; k += blockDim.x) {
       // without mu bins and buffer points a triangle counts three times
-      const double f = !MU && !BUF ? 3.0 : 1.0;
+      const double f = (!MU && !BUF ? 3.0 : 1.0) * (ROWSUM ? T.rscale : 1.0);
       s_cot[k] = f * cot2[k];
       s_cot[nbin + k] = f * (cot3 ? cot2[k] - cot3[k] : cot2[k]);
     }
@@ -223,7 +243,7 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
     row = RowPtrs{R.pos + at, R.w + at, nullptr, R.q + at, R.id + at};
   } else {
     row = RowPtrs{reinterpret_cast<float4*>(wb), reinterpret_cast<double*>(wb + L.o_w),
-                  reinterpret_cast<double*>(wb + L.o_g), reinterpret_cast<int*>(wb + L.o_q),
+                  reinterpret_cast<unsigned long long*>(wb + L.o_g), reinterpret_cast<int*>(wb + L.o_q),
                   reinterpret_cast<int*>(wb + L.o_id)};
   }
 
@@ -292,7 +312,7 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
     row.q[at] = q;
     if (W) row.w[at] = C.w[q];
     if (ids) row.id[at] = C.orig[q];
-    if (ADJ && !LONG) row.g[at] = 0.0;  // zero bits either way
+    if (ADJ && !LONG) row.g[at] = 0ull;
   };
 
   // rooted triangles (BUF: else three each) and triangles of this lane
@@ -358,7 +378,8 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
   };
 
   // MU: one queued hit.
-  double gp = 0.0;  // the current root's gradient over its weight
+  // this lane's part of the current root's gradient, times 2^shift (MU: 2^10)
+  Fix128 gp = {0ull, 0ull};
   auto drain = [&](int e) {
     const uint32_t h = s_hit[e];
     const int x = (int)(h & 0xfffu), y = (int)((h >> 12) & 0xfffu);
@@ -366,10 +387,9 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
     const double cf = triangle(R, x, y);
     if (ADJ && cf != 0.0) {
       const double wx = row.w[x], wy = row.w[y];
-      unsigned long long* g = reinterpret_cast<unsigned long long*>(row.g);
-      gp = fma(cf, wx * wy, gp);
-      smem_add_s64(&g[x], __double2ll_rn(cf * (R.w * wy) * gscale));
-      smem_add_s64(&g[y], __double2ll_rn(cf * (R.w * wx) * gscale));
+      fix_acc(gp, cf * (wx * wy), 1024.0 * gscale);  // a single term, without the room for 1024
+      smem_add_s64(&row.g[x], __double2ll_rn(cf * (R.w * wy) * gscale));
+      smem_add_s64(&row.g[y], __double2ll_rn(cf * (R.w * wx) * gscale));
     }
   };
   int qn = 0;  // queued hits
@@ -383,8 +403,21 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
     const GroupRoot& R = s_root[ri];
     const float4* const pos = row.pos + off;
     const double* const rw = row.w + off;
-    double* const rg = row.g + off;
+    long long* const rg = reinterpret_cast<long long*>(row.g) + off;
     const double wp = W ? R.w : 0.0;
+    int shift = ROWSUM ? 0 : 10;  // of the root's sum, and of the row's weights
+    if (ROWSUM && !LONG) {
+      // the sum of the weights' sizes, in units of 2^-20 of the largest
+      unsigned sum = 0;
+      for (int x = lane; x < k; x += 32)
+        sum += min(__double2uint_ru(fabs(rw[x]) * T.winv), (1u << 20) + 1u);
+      sum = __reduce_add_sync(0xffffffffu, sum);
+      shift = min(32, max(0, 20 + bits_of(T.cap) - bits_of((int)sum)));
+      for (int x = lane; x < k; x += 32) row.w[off + x] *= pow2(shift);
+      __syncwarp();
+    }
+    // of the row's sums in units of the totals
+    const double rinv = ROWSUM ? gscale / T.rscale * pow2(-shift) : 0.0;
     // Whether the pair x, y is an edge, and (not MU: binned later) its radial
     // bin from 0; no branch but the rare one into FP64, which lanes without a
     // pair (on = false) must not take.  The bounds send every pair there when
@@ -473,7 +506,7 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
         const double wpx1 = WEIGHTED && !MU ? wp * wx * s_fsc[nr0 + 1] : 0.0;
         const int xbase = ADJ ? (rran && xran ? nbin : 0) : nbin * nr0;
         const int xn = BUF ? (rbuf ? 0 : 1) + (code_buffer(cx) ? 0 : 1) : 2;
-        double gx = 0.0;
+        long long gx = 0;
         for (int j0 = 1; j0 <= jmax; j0 += G) {
           const int j = j0 + grp;
           const bool on = act && j <= jmax && (ORDERED || 2 * j != k || x < j);
@@ -488,7 +521,7 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
           if (hit) {
             if (MU) {
               const double cf = triangle(R, off + x, off + y);
-              if (ADJ) gx = fma(cf, rw[y], gx);
+              if (ADJ) gx += __double2ll_rn(cf * rw[y]);
             } else {
               int e = (int)(table ? s_cfg[xrow + yr + b0] : rank3(xrow, yr, b0));
               const bool yran = code_random(cy);
@@ -499,8 +532,8 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
                 // the cotangents hold the factor 3 of a catalogue without buffers
                 double cf = s_cot[e + (yran ? xbase : 0)];
                 if (BUF) cf *= (double)n;
-                gx = fma(cf, rw[y], gx);
-                if (!ORDERED) rg[y] = fma(cf, wx, rg[y]);
+                gx += __double2ll_rn(cf * rw[y]);
+                if (!ORDERED) rg[y] += __double2ll_rn(cf * wx);
               } else {
                 e += xbase + (yran ? nbin : 0);
                 if (COUNTS) hist_count_add<SHIST>(s_cnt, nh, e, (unsigned)n);
@@ -515,19 +548,20 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
         if (ORDERED) {
           // all of x's sum; every ordered pair was met, so the root's is half
           for (int g2 = 1; g2 < G; ++g2) {
-            const double o = __shfl_sync(0xffffffffu, gx, min(31, lane - grp * r + g2 * r));
+            const long long o = __shfl_sync(0xffffffffu, gx, min(31, lane - grp * r + g2 * r));
             if (grp == 0) gx += o;
           }
           if (act && grp == 0) {
-            gp = fma(0.5 * wx, gx, gp);
+            const double sx = __ll2double_rn(gx) * rinv;
+            fix_plus(gp, fix_from_double(0.5 * wx * sx));
             const int qx = row.q[off + x];
-            const Fix128 v = fix_from_double(gx * wp * gscale);
+            const Fix128 v = fix_from_double(sx * wp);
             if (v.lo | v.hi) fix_merge(&g_lo[qx], &g_hi[qx], v.lo, v.hi);
           }
         } else if (ONE) {
           if (act) {
             rg[x] += gx;
-            gp = fma(wx, gx, gp);
+            fix_plus(gp, fix_from_double(wx * (__ll2double_rn(gx) * rinv)));
           }
           __syncwarp();
         }
@@ -539,18 +573,23 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
         const int q = row.q[x];
         Fix128 v;
         if (MU) {
-          v.lo = reinterpret_cast<const unsigned long long*>(row.g)[x];
+          v.lo = row.g[x];
           v.hi = (long long)v.lo < 0 ? ~0ull : 0ull;
         } else {
-          v = fix_from_double(row.g[x] * wp * gscale);
+          v = fix_from_double(__ll2double_rn((long long)row.g[x]) * rinv * wp);
         }
         if (v.lo | v.hi) fix_merge(&g_lo[q], &g_hi[q], v.lo, v.hi);
       }
     }
     if (ADJ) {
-      const Fix128 v = fix_warp_sum(fix_from_double(gp * gscale));
+      Fix128 v = fix_warp_sum(gp);
+      if (shift > 0) {  // to the totals' scale, rounded
+        fix_plus(v, Fix128{1ull << (shift - 1), 0ull});
+        v.lo = (v.lo >> shift) | (v.hi << (64 - shift));
+        v.hi = (unsigned long long)((long long)v.hi >> shift);
+      }
       if (lane == 0 && (v.lo | v.hi)) fix_merge(&g_lo[R.p], &g_hi[R.p], v.lo, v.hi);
-      gp = 0.0;
+      gp = Fix128{0ull, 0ull};
     }
     if (BUF) rooted += nroot;
     tris += ntri;
@@ -792,6 +831,11 @@ void launch_root(const DevCatalog& C, RootParams T, bool weighted, bool counts, 
     const int64_t need = ((int64_t)C.n + per - 1) / per;
     if (blocks > need) blocks = need;
   }
+  // room for as many terms as a row has members, below 2^63
+  const int most = LONG ? R.cap : T.cap;
+  int lg = 0;
+  while (lg < 31 && ((int64_t)1 << lg) < most) ++lg;
+  T.rscale = std::ldexp(T.rscale, 3 - lg);
   GR_CUDA_TRY(cudaMemsetAsync(work, 0, sizeof(int), s));
   auto go = [&](auto kfn) {
     GR_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
