@@ -365,15 +365,40 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
     long long v = 0;
     if (WEIGHTED) v = __double2ll_rn(R.w * row.w[x] * row.w[y] * s_fsc[nr]);
     const int e = (int)cfg + nbin * nr;
-    auto add = [&](int k) {
-      if (COUNTS) hist_count_add<SHIST>(s_cnt, nh, k, 1u);
-      if (WEIGHTED) hist_fix_add<SHIST>(s_lim, nh, k, v);
-    };
-    // vertices in the same bin are not merged first: with 32 lanes some lane
-    // needs each of the three updates
-    if (c0) add(e + ncfg * m0);
-    if (c1) add(e + ncfg * m1);
-    if (c2) add(e + ncfg * m2);
+    if (SHIST) {
+      auto add = [&](int k) {
+        if (COUNTS) hist_count_add<true>(s_cnt, nh, k, 1u);
+        if (WEIGHTED) hist_fix_add<true>(s_lim, nh, k, v);
+      };
+      // vertices in the same bin are not merged first: with 32 lanes some lane
+      // needs each of the three updates
+      if (c0) add(e + ncfg * m0);
+      if (c1) add(e + ncfg * m1);
+      if (c2) add(e + ncfg * m2);
+    } else {
+      // in global memory every lane's update counts, so vertices in the same
+      // bin are merged
+      int n0 = c0 ? 1 : 0, n1 = c1 ? 1 : 0, n2 = c2 ? 1 : 0;
+      if (n1 && m1 == m0) {
+        n1 += n0;
+        n0 = 0;
+      }
+      if (n2 && m2 == m1) {
+        n2 += n1;
+        n1 = 0;
+      }
+      if (n2 && m2 == m0) {
+        n2 += n0;
+        n0 = 0;
+      }
+      auto add = [&](int m, int n) {
+        if (COUNTS) hist_count_add<false>(s_cnt, nh, e + ncfg * m, (unsigned)n);
+        if (WEIGHTED) hist_fix_add<false>(s_lim, nh, e + ncfg * m, v * n);
+      };
+      if (n0) add(m0, n0);
+      if (n1) add(m1, n1);
+      if (n2) add(m2, n2);
+    }
     return 0.0;
   };
 
@@ -825,6 +850,15 @@ void launch_root(const DevCatalog& C, RootParams T, bool weighted, bool counts, 
                .total;
     blocks = R.blocks;
   } else {
+    if (weighted && !adj && !shist) {
+      // sums in global memory: a warp waits for each update's old value, and
+      // neighbours of a dense spot grabbed together end the launch alone (SMs
+      // busy 61% of the time with four per grab).  With vertices of one bin
+      // merged: 160,000 points, 1,540 configurations by 8 mu bins 0.61 -> 0.51
+      // ms, 816 by 2 with counts 1.74 -> 0.85 ms.
+      T.chunk = std::max(1, std::min(T.chunk, (int)(C.n / ((int64_t)sm_count() * kRootWarps * 32))));
+      T.group = std::min(T.group, T.chunk);
+    }
     root_shape(T, weighted && !adj, counts && !adj, shist, adj, nw, T.cap, smem);
     blocks = sm_count();
     const int64_t per = (int64_t)nw * T.chunk;
