@@ -917,7 +917,7 @@ static int count_tri(gr_ctx* c, bool equi, double* N2, double* N3, int64_t* coun
   unsigned long long* st = hc + 2 * (size_t)nh;
   unsigned long long* gctl = st + kRootStats;
   unsigned long long* gsts = gctl + 4;
-  std::vector<double> hs(nh, 0.0);
+  double* const hs = hv;  // the sums are formed where they arrive
   cudaEvent_t q0 = c->ev[4];  // owned by the context
   c->work.reserve(4);
   if (!hash) c->long_list.reserve(c->n + 1);
@@ -993,8 +993,6 @@ static int count_tri(gr_ctx* c, bool equi, double* N2, double* N3, int64_t* coun
     break;
   }
   if (!reuse) c->spec_gen = c->cat_gen;
-  if (weighted)
-    for (int k = 0; k < nh; ++k) hs[k] = hv[k];
   if (!weighted) {
     for (int nr = 0; nr < 4; ++nr) {
       double prod = uniform_product(c->w_gal, c->w_ran, 3 - nr, nr);
