@@ -71,7 +71,8 @@ constexpr int kShortRow = 64;
 struct QuadWindow {
   int start, stop, end[kSplitClasses];
 };
-__device__ __forceinline__ QuadWindow quad_window(const QuadParams& Q, int n, int phase) {
+__device__ __forceinline__ QuadWindow quad_window(const QuadParams& Q, int n, int phase,
+                                                  bool split = true) {
   QuadWindow W;
   W.start = 0;
   W.stop = n;
@@ -86,6 +87,7 @@ __device__ __forceinline__ QuadWindow quad_window(const QuadParams& Q, int n, in
     else
       W.start = nlong;
   }
+  if (!split) return W;
   const int limit = (int)gridDim.x * (int)(blockDim.x >> 5);
 #pragma unroll
   for (int j = 0; j < kSplitClasses; ++j)
@@ -993,20 +995,22 @@ __host__ __device__ inline int quad_bins(int cap) {
   return c * (c - 1) / 2;
 }
 
-__host__ __device__ inline QuadGLayout quadg_layout(int nbins, int ncounts) {
+// tetra: its six bins are equal, so there are no tables of perimeters (up to
+// 129 KB, which would leave room for few warps) and no kept bins
+__host__ __device__ inline QuadGLayout quadg_layout(int nbins, int ncounts, bool tetra) {
   QuadGLayout L;
   size_t o = 0;
   L.off_rank = o;
   o = qalign8(o + sizeof(int) * 4 * (size_t)(nbins + 2));
   L.off_tab = o;
-  o = qalign8(o + sizeof(int) * 2 * (size_t)nbins * nbins);
+  if (!tetra) o = qalign8(o + sizeof(int) * 2 * (size_t)nbins * nbins);
   L.off_cnt = o;
   o = o + sizeof(unsigned int) * (size_t)ncounts;
   L.off_warp = (o + 15) & ~(size_t)15;
   return L;
 }
 
-__host__ __device__ inline QuadGWarp quadg_warp(int cap, bool adj, bool lw) {
+__host__ __device__ inline QuadGWarp quadg_warp(int cap, bool adj, bool lw, bool tetra) {
   QuadGWarp W;
   const size_t nwd = (size_t)(cap + 31) / 32;
   size_t w = 0;
@@ -1019,7 +1023,7 @@ __host__ __device__ inline QuadGWarp quadg_warp(int cap, bool adj, bool lw) {
   W.adj = w;  w += (size_t)cap * nwd * 4;         // adjacency rows
   W.q = w;    w += (size_t)kQQueue * 4;           // cliques: a | b << 8 | d << 16 | bin(a,b) << 24
   W.eq = w;   w += (size_t)kQEdgeQueue * 4;       // edges: a | b << 8
-  W.bin = w;  w += (size_t)quad_bins(cap);        // bins of the pairs
+  W.bin = w;  w += tetra ? 0 : (size_t)quad_bins(cap);  // bins of the pairs
   W.bytes = (w + 15) & ~(size_t)15;
   return W;
 }
@@ -1035,7 +1039,7 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
     unsigned long long* __restrict__ g_hi) {
   constexpr bool LW = WEIGHTED || ADJ;
   extern __shared__ __align__(16) unsigned char smem[];
-  const QuadGLayout L = quadg_layout(Q.nbins, SHC ? nh + nd : 0);
+  const QuadGLayout L = quadg_layout(Q.nbins, SHC ? nh + nd : 0, TETRA);
   QuadCtx X;
   quad_setup<SHC, ADJ>(X, Q, smem + L.off_rank, smem + L.off_cnt, g_cnt, g_fix, d_cnt, d_fix, nh,
                        nd, fscale, dscale, cot);
@@ -1045,7 +1049,7 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
   // s_t34[b3, b4] (bins from 0)
   int* const s_t12 = reinterpret_cast<int*>(smem + L.off_tab);
   int* const s_t34 = s_t12 + nb * nb;
-  for (int k = threadIdx.x; k < nb * nb; k += blockDim.x) {
+  for (int k = TETRA ? nb * nb : threadIdx.x; k < nb * nb; k += blockDim.x) {
     const int i = k / nb + 1, j = k % nb + 1, n2 = nb + 2;
     const int* F = X.F;
     s_t12[k] = i <= j ? (F[i] - F[1]) + (F[n2 + j] - F[n2 + i]) - F[2 * n2 + j] : kNoPerimeter;
@@ -1060,12 +1064,12 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
   const int wid = threadIdx.x >> 5;
   const bool big = wid < Q.long_warps;
   const int cap = big || Q.long_warps == 0 ? Q.cap : Q.short_cap;
-  const QuadGWarp A = quadg_warp(cap, ADJ, LW);
+  const QuadGWarp A = quadg_warp(cap, ADJ, LW, TETRA);
   unsigned char* wb = smem + L.off_warp;
   if (big || Q.long_warps == 0)
     wb += A.bytes * wid;
   else
-    wb += quadg_warp(Q.cap, ADJ, LW).bytes * Q.long_warps + A.bytes * (wid - Q.long_warps);
+    wb += quadg_warp(Q.cap, ADJ, LW, TETRA).bytes * Q.long_warps + A.bytes * (wid - Q.long_warps);
   float4* const s_pos = reinterpret_cast<float4*>(wb + A.pos);
   double* const s_w = reinterpret_cast<double*>(wb + A.w);
   unsigned* const s_grad = reinterpret_cast<unsigned*>(wb + A.g);  // four words per neighbour, cap apart
@@ -1099,7 +1103,11 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
   };
 
   int phase = big ? 0 : 1;  // long rows first, then the others (work[1], work[0])
-  QuadWindow win = quad_window(Q, C.n, phase);
+  // -tetra with three bins or more: staging and testing a row is nearly all of
+  // its work, which shares would repeat (40,000 points, rows up to 256, 20 bins
+  // 5.0 ms with shares, 0.9 without; one bin, where every edge stays, 14 and 21)
+  const bool split = !TETRA || nb <= 2;
+  QuadWindow win = quad_window(Q, C.n, phase, split);
   for (;;) {
     int item = 0;
     if (lane == 0) item = atomicAdd(work + (1 - phase), 1);
@@ -1108,7 +1116,7 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
     if (!quad_item(Q, win, item, p, part, nparts)) {
       if (phase == 1) break;
       phase = 1;
-      win = quad_window(Q, C.n, 1);
+      win = quad_window(Q, C.n, 1, split);
       continue;
     }
     const int64_t b0 = G.start[p];
@@ -1160,7 +1168,7 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
     // pass 1: adjacency among the members of R+(p), and their bins
     const int npair = k * (k - 1) / 2;
     const int k2m1 = 2 * k - 1;
-    const bool mat = npair <= quad_bins(cap);  // their bins are kept
+    const bool mat = !TETRA && npair <= quad_bins(cap);  // their bins are kept
     // index of the pair (x, y) is s_tb[x] + y
     for (int x = lane; x < k; x += 32) s_tb[x] = x * (k2m1 - x) / 2 - x - 1;
     if (lane == 0 && part == 0) probes += (unsigned long long)npair;  // once per root
@@ -1173,7 +1181,11 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
     for (int t = lane; t < npair; t += 32) {
       int x, y, bin;
       pair_of(t, x, y);
-      if (pair_bin(x, y, bin)) {
+      // -tetra: an edge in another bin than both of its ends' to the root is in
+      // no clique that counts (120,000 points, rows up to 120, weighted: 4 bins
+      // 1.6 -> 0.45 ms, 127 bins 1.3 -> 0.3; rows of 200: 4.4 -> 0.4)
+      if (pair_bin(x, y, bin) &&
+          (!TETRA || (bin == (s_code[x] & 0xff) && bin == (s_code[y] & 0xff)))) {
         atomicOr(&s_adj[x * nwk + (y >> 5)], 1u << (y & 31));
         if (mat) s_bin[t] = (uint8_t)bin;
       }
@@ -1186,6 +1198,32 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
       const uint32_t qe = act ? s_q[e] : 0u;
       const int x = (int)(qe & 0xffu), y = (int)((qe >> 8) & 0xffu), z = (int)((qe >> 16) & 0xffu);
       const int cx = s_code[x], cy = s_code[y], cz = s_code[z];
+      if constexpr (TETRA) {
+        // only cliques with all edges in one bin are queued: each of the four
+        // vertices that can be a root is one
+        if (!act) return;
+        QVerts V;
+        auto flags = [](int code) {
+          return (uint8_t)(((code >> 8) & 1 ? FLAG_RANDOM : 0) | ((code >> 9) & 1 ? 0 : FLAG_BUFFER));
+        };
+        V.fl[0] = fp;
+        V.fl[1] = flags(cx);
+        V.fl[2] = flags(cy);
+        V.fl[3] = flags(cz);
+        V.og[0] = 2 * rank_p;  // places in id order
+        V.og[1] = 2 * x + 1;
+        V.og[2] = 2 * y + 1;
+        V.og[3] = 2 * z + 1;
+        V.w[0] = LW ? s_w[slot] : 0.0;
+        V.w[1] = LW ? s_w[x] : 0.0;
+        V.w[2] = LW ? s_w[y] : 0.0;
+        V.w[3] = LW ? s_w[z] : 0.0;
+        const uint32_t b = pack_meta((cx & 0xff) + 1, 1, 1), m[6] = {b, b, b, b, b, b};
+        const int nroot = tetra_contrib<WEIGHTED, SHC>(X, V, m);
+        quads += nroot > 0 ? 1 : 0;
+        rooted += (unsigned)nroot;
+        return;
+      }
       int bxz = 0, byz = 0;
       if (act) {
         if (mat) {
@@ -1223,23 +1261,18 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
       // histogram index of each root, or none when its perimeter is not
       // canonical
       int kk[4] = {0, 0, 0, 0};
-      if (TETRA) {
-        if (!(b01 == b02 && b01 == b03 && b01 == b12 && b01 == b13 && b01 == b23)) vm = 0u;
-        kk[0] = kk[1] = kk[2] = kk[3] = b01;
-      } else {
-        auto root = [&](int i, int b1, int b2, int b3, int b4, int d1, int d2) {
-          const int cfg = s_t12[b1 * nb + b2] + s_t34[b3 * nb + b4];
-          if (!((unsigned)cfg < (1u << 28) && b2 <= b3)) vm &= ~(1u << i);
-          kk[i] = cfg + X.ncfg * (d1 + nb * d2);
-        };
-        root(0, b01, b12, b23, b03, b02, b13);
-        root(1, b01, b02, b23, b13, b12, b03);
-        root(2, b02, b01, b13, b23, b12, b03);
-        root(3, b03, b01, b12, b23, b13, b02);
-      }
+      auto root = [&](int i, int b1, int b2, int b3, int b4, int d1, int d2) {
+        const int cfg = s_t12[b1 * nb + b2] + s_t34[b3 * nb + b4];
+        if (!((unsigned)cfg < (1u << 28) && b2 <= b3)) vm &= ~(1u << i);
+        kk[i] = cfg + X.ncfg * (d1 + nb * d2);
+      };
+      root(0, b01, b12, b23, b03, b02, b13);
+      root(1, b01, b02, b23, b13, b12, b03);
+      root(2, b02, b01, b13, b23, b12, b03);
+      root(3, b03, b01, b12, b23, b13, b02);
       quads += vm ? 1 : 0;
       rooted += (unsigned)__popc(vm);
-      if constexpr (!LW && !TETRA) {
+      if constexpr (!LW) {
         // the pattern of root i: its randomness, then that of the others
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -1293,22 +1326,6 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
               else
                 smem_fix_add(s_grad + pos[j], cap, __double2ll_rn(g[j] * gscale));
             }
-          } else if constexpr (TETRA) {
-            qcount<SHC>(X, kr + nb * onr);
-            if (WEIGHTED)
-              qfix(X, qfx(X.fix, kr + nb * onr), qfx(X.fix, kr + nb * (onr + 5)),
-                   ((w[0] * w[1]) * w[2]) * w[3], X.fscale);
-#pragma unroll
-            for (int tt = 0; tt < 6; ++tt) {
-              const int ua = term_gate(tt), ub = term_pu(tt), uc = term_pv(tt);
-              if (!rb[ua]) continue;
-              const int nr3 = (int)(rb[ua] + rb[ub] + rb[uc]);
-              const int kt = kr + nb * tt + nb * 6 * nr3;
-              // discR (all three random) equals category 3 and is copied on the host
-              qdcount<SHC>(X, kt);
-              if (WEIGHTED)
-                qfix(X, qfx(X.dfix, kt), qfx(X.dfix, kt + X.dhi), (w[ua] * w[ub]) * w[uc], X.dscale);
-            }
           } else {
             qcount<SHC>(X, kr + X.nbin * onr);
             qfix(X, qfx(X.fix, kr + X.nbin * onr), qfx(X.fix, kr + X.nbin * (onr + 5)),
@@ -1340,7 +1357,7 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
         cm = s_adj[x * nwk + cw] & s_adj[y * nwk + cw];
         if (mat)
           bxy = s_bin[s_tb[x] + y];
-        else
+        else if (!TETRA)
           pair_bin(x, y, bxy);
       }
       for (;;) {
@@ -1443,12 +1460,12 @@ constexpr int kLongWarps = 4;
 static QuadParams quadg_shape(const QuadParams& Q0, int ncounts, bool adj, bool lw, int maxw, int& nw,
                               size_t& smem) {
   QuadParams Q = Q0;
-  const size_t fixed = quadg_layout(Q.nbins, ncounts).off_warp;
-  const size_t big = quadg_warp(Q.cap, adj, lw).bytes;
+  const size_t fixed = quadg_layout(Q.nbins, ncounts, Q.tetra != 0).off_warp;
+  const size_t big = quadg_warp(Q.cap, adj, lw, Q.tetra != 0).bytes;
   Q.long_warps = 0;
   Q.short_cap = kShortRow;
   if (Q.cap > kShortRow && Q.order && Q.above && Q.nclass > kShortRow && 2 * Q.mean_row < kShortRow) {
-    const size_t small = quadg_warp(kShortRow, adj, lw).bytes;
+    const size_t small = quadg_warp(kShortRow, adj, lw, Q.tetra != 0).bytes;
     nw = maxw;
     while (nw > kLongWarps && fixed + kLongWarps * big + (nw - kLongWarps) * small > kQuadSmemLimit) --nw;
     smem = fixed + kLongWarps * big + (nw - kLongWarps) * small;
