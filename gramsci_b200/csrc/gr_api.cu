@@ -1039,11 +1039,11 @@ int gr_count_equi(gr_ctx* c, double* N2, double* N3, int64_t* counts, double* ca
 }
 
 // Edges among R+(p) in the 4-clique kernels: the geometric pair test (rows
-// up to 255 members) or hash probes of the members' rows.  Measured on the
+// up to 256 members) or hash probes of the members' rows.  Measured on the
 // 4PCF workload (upper degree 17.5): unit weights 1.38 ms geometric against
 // 4.05 ms, lognormal weighted sums 3.1 against 7.4 ms.
 static int quad_geometric(const gr_ctx* c, int64_t max_deg, int nbins) {
-  return (max_deg > 255 || nbins > 255 || c->clique_mode == 1) ? 0 : 1;
+  return (max_deg > 256 || nbins > 255 || c->clique_mode == 1) ? 0 : 1;
 }
 
 static int count_quad(gr_ctx* c, bool tetra, double* N2, double* N3, double* discN, double* discR,

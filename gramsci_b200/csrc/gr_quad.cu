@@ -22,7 +22,7 @@
 // A second kernel (quad4g_kernel, the geometric mode) finds the edges among
 // the members of R+(p) with the graph's own membership test on their
 // positions instead of probing the members' rows; it is used whenever the
-// rows fit (up to 255 members).
+// rows fit (up to 256 members).
 #include <algorithm>
 #include <type_traits>
 
@@ -952,8 +952,8 @@ __global__ void __launch_bounds__((WEIGHTED || ADJ ? kQuadMaxWarps : kQuadMaxWar
 // queued 32 at a time, each lane ANDs its two rows word by word and emits one
 // clique per set bit into the clique queue, which is drained 32 at a time.  No
 // row other than R+(p) is read; the tests are k(k-1)/2 per root instead of the
-// sum over R+(p) of the members' row lengths.  Rows up to 255 members (8-bit
-// positions, one for the root).
+// sum over R+(p) of the members' row lengths.  Rows up to 256 members (8-bit
+// positions).
 //
 // What a clique adds depends on its six radial bins, on the catalogue-id order
 // of its vertices and on their flags.  Three things are therefore done once
@@ -987,8 +987,6 @@ struct QuadGWarp {
   size_t pos, w, g, col, code, tb, adj, bin, q, eq, bytes;
 };
 
-// position of the root beside the members' (its weight is staged there)
-__host__ __device__ inline int quad_root_slot(int cap) { return cap < 255 ? cap : 255; }
 // pairs whose bins a warp can keep
 __host__ __device__ inline int quad_bins(int cap) {
   const int c = cap < kMatCap ? cap : kMatCap;
@@ -1080,7 +1078,7 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
   uint32_t* const s_q = reinterpret_cast<uint32_t*>(wb + A.q);
   uint32_t* const s_eq = reinterpret_cast<uint32_t*>(wb + A.eq);
   uint8_t* const s_bin = wb + A.bin;
-  const int slot = quad_root_slot(cap);
+  const int slot = cap;  // position of the root beside the members' (its weight is staged there)
   unsigned long long quads = 0, rooted = 0, probes = 0;
   const float guard = P.f32 ? P.tguard : INFINITY;
   // edge test and radial bin (from 0) of members x, y (see bin_pair_f32)
@@ -1284,8 +1282,10 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
         // the warp's valid roots, ordered by vertex, then lane
         const unsigned three = (unsigned)(x | (y << 8) | (z << 16));
         const unsigned lowb = r == 0 ? 0u : (0xffffffu >> (24 - 8 * r));
-        const unsigned vpos = (three & lowb) | ((unsigned)slot << (8 * r)) |
-                              (r == 3 ? 0u : (three & ~lowb) << 8);
+        // the root's byte is empty: its place is kept beside the random bits,
+        // which leaves all 256 positions to members
+        const unsigned vpos = (three & lowb) | (r == 3 ? 0u : (three & ~lowb) << 8);
+        const unsigned vrnd = rnd | ((unsigned)r << 4);
         unsigned mr[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) mr[i] = __ballot_sync(0xffffffffu, (vm >> i) & 1u);
@@ -1298,7 +1298,7 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
           const unsigned mR = R == 0 ? mr[0] : (R == 1 ? mr[1] : (R == 2 ? mr[2] : mr[3]));
           const int o = i < total ? (int)__fns(mR, 0, i - base + 1) : 0;
           // every lane takes part in each shuffle; the select comes after
-          const unsigned ornd = __shfl_sync(0xffffffffu, rnd, o);
+          const unsigned ornd = __shfl_sync(0xffffffffu, vrnd, o);
           const unsigned opos = __shfl_sync(0xffffffffu, vpos, o);
           const int q0 = __shfl_sync(0xffffffffu, kk[0], o), q1 = __shfl_sync(0xffffffffu, kk[1], o),
                     q2 = __shfl_sync(0xffffffffu, kk[2], o), q3 = __shfl_sync(0xffffffffu, kk[3], o);
@@ -1311,7 +1311,7 @@ __global__ void __launch_bounds__((ADJ ? kQuadGWarpsA : (WEIGHTED ? kQuadGWarpsW
           double w[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            pos[j] = (int)((opos >> (8 * v[j])) & 0xffu);
+            pos[j] = v[j] == (int)(ornd >> 4) ? slot : (int)((opos >> (8 * v[j])) & 0xffu);
             rb[j] = (ornd >> v[j]) & 1u;
             w[j] = LW ? s_w[pos[j]] : 0.0;
           }

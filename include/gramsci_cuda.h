@@ -64,7 +64,7 @@ typedef struct gr_ctx gr_ctx;
                                the graph, 2 the graph's membership test on the pairs of
                                neighbours.  3PCF: mode 2 needs the cell index alone and
                                builds no graph; rows beyond a warp's capacity take a second
-                               launch.  4PCF: mode 2 takes rows up to 255 neighbours (longer
+                               launch.  4PCF: mode 2 takes rows up to 256 neighbours (longer
                                rows use 1).  Results are identical; only speed differs */
 
 /* Run statistics of the last count call (gr_get_stats). */
