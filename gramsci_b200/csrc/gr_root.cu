@@ -544,6 +544,8 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
           const int yr = code_byte(cy, 0);
           if (!MU && T.equi) hit = hit && xr == yr && b0 * (table ? nb : 1) == xr;
           if (hit) {
+            // an ordered pair's triangle counts from its smaller member
+            const unsigned root0 = nroot, tri0 = ntri;
             if (MU) {
               const double cf = triangle(R, off + x, off + y);
               if (ADJ) gx += __double2ll_rn(cf * rw[y]);
@@ -566,6 +568,10 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
                   hist_fix_add<SHIST>(s_lim, nh, e,
                                       __double2ll_rn((yran ? wpx1 : wpx0) * rw[y]) * n);
               }
+            }
+            if (ORDERED && y < x) {
+              nroot = root0;
+              ntri = tri0;
             }
           }
           if (ONE) __syncwarp();
@@ -775,11 +781,6 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
         p += ng;
       }
     }
-  }
-  if (MU && !ADJ && !LONG) {
-    // the last drain's triangles
-    if (BUF) rooted += nroot;
-    tris += ntri;
   }
   if (!BUF) rooted = 3 * tris;
   unsigned long long sums[6] = {tris, rooted, probes, edges, cands, rechecks};
