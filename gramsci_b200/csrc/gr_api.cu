@@ -992,7 +992,7 @@ static int count_tri(gr_ctx* c, bool equi, double* N2, double* N3, int64_t* coun
     }
     break;
   }
-  if (!reuse) c->spec_gen = c->cat_gen;
+  if (hash && !reuse) c->spec_gen = c->cat_gen;
   if (!weighted) {
     for (int nr = 0; nr < 4; ++nr) {
       double prod = uniform_product(c->w_gal, c->w_ran, 3 - nr, nr);
