@@ -746,7 +746,7 @@ int gr_count_2pcf(gr_ctx* c, double* N2, double* N3, int64_t* counts, double* ca
   int sub = 1;
   if (c->autotune == 1) sub = 0;
   if (c->autotune == 2 + kPairTile2) sub = 2;
-  const bool reuse = reuse_graph(c);
+  const bool reuse = reuse_index(c);
   ZeroList z;
   z.add(c->hcnt.p, sizeof(unsigned long long) * nh);
   z.add(c->hfix.p, sizeof(unsigned long long) * 2 * nh);
@@ -799,7 +799,7 @@ int gr_count_2pcf(gr_ctx* c, double* N2, double* N3, int64_t* counts, double* ca
   c->st.rooted = rooted;
   c->st.fp64_rechecks = (int64_t)st[0];
   c->st.candidates = (int64_t)st[1];
-  c->st.kernel_launches = c->index.launches + 2;
+  c->st.kernel_launches = (reuse ? 1 : c->index.launches) + 2;
   GR_API_END(c)
 }
 
@@ -1613,7 +1613,8 @@ int gr_adjoint_2pcf(gr_ctx* c, const double* cot2, const double* cot3, double* g
   GR_CUDA_TRY(cudaMemcpyAsync(c->cot.p, cots.data(), sizeof(double) * cots.size(),
                               cudaMemcpyHostToDevice, s));
   GR_CUDA_TRY(cudaEventRecord(c->ev[0], s));
-  if (!reuse_graph(c)) {
+  const bool reuse = reuse_index(c);
+  if (!reuse) {
     // dense catalogues: cells of rmax/2 and the tile sweep
     int sub = 1;
     if (c->autotune == 1) sub = 0;
@@ -1645,7 +1646,7 @@ int gr_adjoint_2pcf(gr_ctx* c, const double* cot2, const double* cot3, double* g
   c->st.ms_index = ev_ms(c->ev[0], c->ev[1]);
   c->st.ms_total = c->st.ms_index + c->st.ms_query;
   c->st.n_points = n;
-  c->st.kernel_launches = c->index.launches + 2;
+  c->st.kernel_launches = (reuse ? 0 : c->index.launches) + 2;
   GR_API_END(c)
 }
 
