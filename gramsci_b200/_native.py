@@ -63,6 +63,7 @@ SIGNATURES = {
     "gr_destroy": (ctypes.c_int, [_ctx]),
     "gr_last_error": (ctypes.c_char_p, [_ctx]),
     "gr_set_stream": (ctypes.c_int, [_ctx, _vp]),
+    "gr_wait_stream": (ctypes.c_int, [_ctx, _vp]),
     "gr_set_catalog": (ctypes.c_int, [_ctx, _vp, _vp, _vp, ctypes.c_int64, ctypes.c_int64]),
     "gr_set_catalog_dev": (ctypes.c_int, [_ctx, _vp, _vp, _vp, ctypes.c_int64, ctypes.c_int64]),
     "gr_set_bins": (ctypes.c_int, [_ctx, ctypes.c_double, ctypes.c_double, ctypes.c_int32,

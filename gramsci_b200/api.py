@@ -42,17 +42,11 @@ def _is_torch_cuda(x):
     return hasattr(x, "is_cuda") and hasattr(x, "data_ptr") and x.is_cuda
 
 
-def _wait_for(*tensors):
-    """Until torch's current stream has computed the CUDA tensors: the library
-    reads them on a stream of its own, which is not ordered after torch's."""
+def _torch_stream(index):
+    """Handle of torch's current stream on a device."""
     import torch
 
-    if torch.cuda.is_current_stream_capturing():
-        return  # nothing runs that could be waited for
-    for device in {t.device for t in tensors if t is not None and t.is_cuda}:
-        stream = torch.cuda.current_stream(device)
-        if not stream.query():
-            stream.synchronize()
+    return torch._C._cuda_getCurrentRawStream(index)
 
 
 class Context:
@@ -116,7 +110,10 @@ class Context:
             if w.numel() < n or (buf is not None and buf.numel() < n):
                 raise ValueError("w and buffer must have one entry per point")
             self._keep = (xyz, w, buf)
-            _wait_for(*self._keep)
+            # the library's stream is not ordered after torch's, which may still
+            # be computing these
+            for index in {t.get_device() for t in self._keep if t is not None and t.is_cuda}:
+                self._check(self._lib.gr_wait_stream(self._h, ctypes.c_void_p(_torch_stream(index))))
             self.n = int(n)
             self._check(self._lib.gr_set_catalog_dev(
                 self._h, ctypes.c_void_p(xyz.data_ptr()), ctypes.c_void_p(w.data_ptr()),

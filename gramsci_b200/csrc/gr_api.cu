@@ -495,6 +495,29 @@ int gr_set_stream(gr_ctx* c, void* stream) {
   GR_API_END(c)
 }
 
+int gr_wait_stream(gr_ctx* c, void* stream) {
+  GR_API_BEGIN(c)
+  const cudaStream_t o = reinterpret_cast<cudaStream_t>(stream);
+  if (o == c->stream()) return GR_OK;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(o, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return GR_OK;  // nothing runs that could be waited for
+  }
+  const cudaError_t e = cudaStreamQuery(o);
+  if (e == cudaSuccess) return GR_OK;
+  if (e != cudaErrorNotReady) GR_CUDA_TRY(e);
+  cudaGetLastError();
+  if (!c->bev[0]) GR_CUDA_TRY(cudaEventCreateWithFlags(&c->bev[0], cudaEventDisableTiming));
+  if (cudaEventRecord(c->bev[0], o) == cudaSuccess) {
+    GR_CUDA_TRY(cudaStreamWaitEvent(c->stream(), c->bev[0], 0));
+  } else {
+    cudaGetLastError();  // a stream of another device
+    GR_CUDA_TRY(cudaStreamSynchronize(o));
+  }
+  GR_API_END(c)
+}
+
 // Whether kernels of this context may use `bytes` at p directly: memory of its
 // device, inside one allocation, aligned to `align`.  Anything else is left to
 // a copy, which handles other devices and pinned memory and reports the rest.

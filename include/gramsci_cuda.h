@@ -99,6 +99,10 @@ const char* gr_last_error(const gr_ctx* ctx);
  * restores the context's own stream.  Count calls wait on the stream for
  * their results, so they cannot be captured into a caller's CUDA graph. */
 int gr_set_stream(gr_ctx* ctx, void* stream);
+/* Order the context's work after what `stream` (a cudaStream_t; NULL: the
+ * default stream) holds now, without waiting on the host: for device arrays
+ * that are still being computed there when gr_set_catalog_dev takes them. */
+int gr_wait_stream(gr_ctx* ctx, void* stream);
 
 /* Catalogue.  Replaces read_files_2's result (src/gramsci.F90:1364-1396):
  *   xyz    points(3,N) in Fortran order, i.e. x,y,z interleaved, N = n_data+n_rand

@@ -1,6 +1,6 @@
 """Catalogues that torch's stream is still computing when they are handed to
-the library, which reads them on its own stream: the call waits for them, the
-conversions that it queues itself included."""
+the library, which reads them on its own stream: its work is ordered after
+them, the conversions that the call queues itself included."""
 import numpy as np
 import pytest
 import torch
@@ -10,27 +10,12 @@ from gramsci_b200 import api
 from test_device_arrays import catalogue, context
 
 
-class Stream:
-    def __init__(self, log, busy):
-        self.log, self.busy = log, busy
-
-    def query(self):
-        self.log.append("query")
-        return not self.busy
-
-    def synchronize(self):
-        self.log.append("synchronize")
-        self.busy = False
-
-
-@pytest.mark.parametrize("busy", [False, True])
-def test_waits_before_the_library_reads(monkeypatch, busy):
-    log = []
-    stream = Stream(log, busy)
-    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: stream)
-    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
-    context(log).set_catalog(*catalogue(4, 4, 4))
-    assert log == ["query"] + ["synchronize"] * busy + ["gr_set_catalog_dev"]
+def test_the_library_waits_first(monkeypatch):
+    asked = []
+    monkeypatch.setattr(api, "_torch_stream", lambda index: asked.append(index) or 7)
+    ctx = context()
+    ctx.set_catalog(*catalogue(4, 4, 4))
+    assert asked == [0] and ctx._lib.log == ["gr_wait_stream", "gr_set_catalog_dev"]
 
 
 @pytest.mark.gpu
