@@ -775,14 +775,15 @@ def sub_batched(args, stream, flush):
                                 "per_region_sum_f64": res["f64"][1]},
            "clocks": ck.clocks}
     # issue and shared-atomic ceilings of the tile sweep, from its ncu summary
-    # (10%-scale catalogue: the same density, so the same instructions per
-    # pair test), over the whole batched call's device time (layout kernels
+    # (10%-scale catalogue: the same density, so about the same instructions
+    # per binned pair, though not per pair tested: smaller regions have more
+    # halo), over the whole batched call's device time (layout kernels
     # included: a lower bound for the sweep kernel alone)
     prof = roofline.profile("pair2_tile_kernel", "c4")
     n_sm = torch.cuda.get_device_properties(0).multi_processor_count
     rf = {"kernel": "pair2_tile_kernel", "ms": tb, "ms_is": "whole batched call"}
-    rf["issue"] = roofline.issue_roofline(prof, st["candidates"], tb, ck.clocks.get("sm_mhz"), n_sm)
-    rf["atomics"] = roofline.atomic_roofline(prof, st["candidates"], tb, ck.clocks.get("sm_mhz"), n_sm)
+    rf["issue"] = roofline.issue_roofline(prof, st["tuples"], tb, ck.clocks.get("sm_mhz"), n_sm)
+    rf["atomics"] = roofline.atomic_roofline(prof, st["tuples"], tb, ck.clocks.get("sm_mhz"), n_sm)
     rf["fp32"] = roofline.fp32_binning_roofline(rec["rooted"], sp["nmu"], tb, ck.clocks.get("sm_mhz"),
                                                 n_sm)
     rec["roofline"] = roofline.mark_binding(rf)
