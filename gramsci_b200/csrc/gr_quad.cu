@@ -1611,8 +1611,4 @@ void quad_cot_lines(const double* cot2, const double* cot3, const double* cotN,
   }
 }
 
-size_t quad4_smem_bytes(int nbins, int cap) {
-  return quad_layout(nbins, cap, quad4_warps(nbins, cap, 0), 0).total;
-}
-
 }  // namespace gr
