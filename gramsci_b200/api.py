@@ -340,7 +340,8 @@ class Context:
         """How the 3PCF / 4PCF kernels find the edges among a root's
         larger-label neighbours: "auto", "hash" (probes of the neighbours'
         rows) or "geometric" (the graph's membership test on the pairs).
-        Results are identical."""
+        Counts and the 4PCF's sums are identical, the 3PCF's sums and gradients
+        equal to rounding."""
         v = {"auto": 0, "hash": 1, "geometric": 2}[mode]
         self._check(self._lib.gr_set_option(self._h, _native.GR_OPT_CLIQUE_MODE, v))
 

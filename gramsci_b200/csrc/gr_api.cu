@@ -840,7 +840,7 @@ static const int* root_order(gr_ctx* c, cudaStream_t s, const int** above = null
   int* scratch = c->qorder.p + c->n;
   order_roots_by_length(c->csr.view(), (int)c->n, cap, c->qorder.p, scratch, s);
   // after the ordering, scratch[b] holds the number of roots in the classes
-  // above b (classes 0..cap)
+  // from b on (classes 0..cap)
   if (above) *above = scratch;
   if (nclass) *nclass = cap + 1;
   return c->qorder.p;

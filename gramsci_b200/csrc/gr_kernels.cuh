@@ -173,7 +173,7 @@ struct QuadParams {
   const int* order; // roots in the order the work counter hands them out
                     // (order_roots_by_length), or null: label order
   const int* above;  // with order: above[b] = the number of roots whose row
-                     // length class (min(length, nclass - 1)) exceeds b, or null
+                     // length class (min(length, nclass - 1)) is b or more, or null
   int nclass;
   int mean_row;     // average row length
   int long_warps, short_cap;  // set by the launch (quadg_shape)

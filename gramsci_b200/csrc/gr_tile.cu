@@ -62,11 +62,11 @@ namespace {
 
 constexpr int kTileWarps = 8;
 constexpr int kTileThreads = kTileWarps * 32;
-// resident blocks per SM the register allocation is sized for: 3 (at most
-// 85 registers); the adjoint on cells of rmax/2 runs best at 4 (64
-// registers, no spills; measured on the 3M-point adjoint catalogue: 23.5
-// against 27.8 ms, while the forward sweep is faster at 3: 19.4 against
-// 20.4 ms)
+// Resident blocks per SM the register allocation is sized for: 3 (at most 85
+// registers, up to 48 bytes spilled); 4 for the adjoint on cells of rmax/2 (64
+// registers, 20 bytes spilled), where the two are level: 3M weighted points
+// with their gradient, 20.4 ms at 4 and 20.3 ms at 3.  The forward sweep at 4:
+// 59.8 -> 66.1 ms on 12M points in 125 regions, 20.4 -> 21.4 on the 3M.
 #ifndef GR_TILE_MIN_BLOCKS
 #define GR_TILE_MIN_BLOCKS 3
 #endif

@@ -65,7 +65,9 @@ typedef struct gr_ctx gr_ctx;
                                neighbours.  3PCF: mode 2 needs the cell index alone and
                                builds no graph; rows beyond a warp's capacity take a second
                                launch.  4PCF: mode 2 takes rows up to 256 neighbours (longer
-                               rows use 1).  Results are identical; only speed differs */
+                               rows use 1).  Counts and the 4PCF's sums are identical; the 3PCF's
+                               weighted sums agree to two roundings of each product, its
+                               gradients to the rounding of their terms */
 
 /* Run statistics of the last count call (gr_get_stats). */
 typedef struct gr_stats {
@@ -259,7 +261,8 @@ int gr_regions_export(gr_ctx* ctx, int64_t* member_off, int32_t* member_orig,
  * the product of the other weights.  The adjoints reuse the index (4PCF: the
  * graph) of the last count or graph build when the catalogue and bins are
  * unchanged.
- * Gradients are accumulated in 128-bit fixed point: deterministic. */
+ * Gradients are accumulated in fixed point, 64-bit within a row of neighbours
+ * and 128-bit in the totals: deterministic. */
 int gr_adjoint_2pcf(gr_ctx* ctx, const double* cot2, const double* cot3, double* grad_w);
 int gr_adjoint_3pcf(gr_ctx* ctx, const double* cot2, const double* cot3, double* grad_w);
 
