@@ -166,7 +166,14 @@ __device__ __forceinline__ void fix_plus(Fix128& a, const Fix128& b) {
   a.hi += b.hi + (a.lo < b.lo ? 1ull : 0ull);
 }
 
-template <bool MU, bool WEIGHTED, bool COUNTS, bool SHIST, bool ADJ, bool BUF, bool LONG>
+// Where integer counts go.
+enum : int {
+  kNoCounts = 0,
+  kWithSums = 1,    // shared or global memory like the sums (SHIST)
+  kCountsApart = 2  // global memory, the sums in shared memory
+};
+
+template <bool MU, bool WEIGHTED, int CMODE, bool SHIST, bool ADJ, bool BUF, bool LONG>
 __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG ? 5 : 1)
     root3_kernel(DevCatalog C, RootParams T, unsigned long long* __restrict__ g_cnt,
                  unsigned long long* __restrict__ g_lim, unsigned long long* __restrict__ stats,
@@ -175,15 +182,16 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
                  unsigned long long* __restrict__ g_lo, unsigned long long* __restrict__ g_hi) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr bool W = WEIGHTED || ADJ;
+  constexpr bool COUNTS = CMODE != kNoCounts, SCOUNTS = SHIST && CMODE == kWithSums;
   constexpr bool ROWSUM = ADJ && (!MU || LONG);  // sums over the root's weight, at T.rscale
   const PairParams& P = T.P;
   const int nb = T.nbins, ncfg = T.ncfg;
   const int nbin = ncfg * T.nmu, nh = nbin * 4;
   const bool ids = MU && T.asym;
-  const RootLayout L = root_layout(nh, T.nmu, nb, LONG ? 0 : T.cap, SHIST, WEIGHTED, COUNTS,
+  const RootLayout L = root_layout(nh, T.nmu, nb, LONG ? 0 : T.cap, SHIST, WEIGHTED, SCOUNTS,
                                    blockDim.x >> 5, ADJ, MU, ids, LONG ? 1 : T.group);
   unsigned long long* const s_cnt =
-      SHIST ? reinterpret_cast<unsigned long long*>(smem + L.off_cnt) : g_cnt;
+      SCOUNTS ? reinterpret_cast<unsigned long long*>(smem + L.off_cnt) : g_cnt;
   unsigned long long* const s_lim =
       SHIST ? reinterpret_cast<unsigned long long*>(smem + L.off_lim) : g_lim;
   double* const s_cot = reinterpret_cast<double*>(smem + L.off_cot);
@@ -214,7 +222,7 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
     }
   if (SHIST)
     for (int k = threadIdx.x; k < nh; k += blockDim.x) {
-      if (COUNTS) s_cnt[k] = 0ull;
+      if (SCOUNTS) s_cnt[k] = 0ull;
       if (WEIGHTED) {
         s_lim[k] = 0ull;
         s_lim[nh + k] = 0ull;
@@ -365,17 +373,19 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
     long long v = 0;
     if (WEIGHTED) v = __double2ll_rn(R.w * row.w[x] * row.w[y] * s_fsc[nr]);
     const int e = (int)cfg + nbin * nr;
+    auto add = [&](int m, int n, bool count, bool sum) {
+      if (COUNTS && count) hist_count_add<SCOUNTS>(s_cnt, nh, e + ncfg * m, (unsigned)n);
+      if (WEIGHTED && sum) hist_fix_add<SHIST>(s_lim, nh, e + ncfg * m, v * n);
+    };
+    constexpr bool GCOUNTS = COUNTS && !SCOUNTS, GSUMS = WEIGHTED && !SHIST;
     if (SHIST) {
-      auto add = [&](int k) {
-        if (COUNTS) hist_count_add<true>(s_cnt, nh, k, 1u);
-        if (WEIGHTED) hist_fix_add<true>(s_lim, nh, k, v);
-      };
       // vertices in the same bin are not merged first: with 32 lanes some lane
       // needs each of the three updates
-      if (c0) add(e + ncfg * m0);
-      if (c1) add(e + ncfg * m1);
-      if (c2) add(e + ncfg * m2);
-    } else {
+      if (c0) add(m0, 1, !GCOUNTS, true);
+      if (c1) add(m1, 1, !GCOUNTS, true);
+      if (c2) add(m2, 1, !GCOUNTS, true);
+    }
+    if (GCOUNTS || GSUMS) {
       // in global memory every lane's update counts, so vertices in the same
       // bin are merged
       int n0 = c0 ? 1 : 0, n1 = c1 ? 1 : 0, n2 = c2 ? 1 : 0;
@@ -391,13 +401,9 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
         n2 += n0;
         n0 = 0;
       }
-      auto add = [&](int m, int n) {
-        if (COUNTS) hist_count_add<false>(s_cnt, nh, e + ncfg * m, (unsigned)n);
-        if (WEIGHTED) hist_fix_add<false>(s_lim, nh, e + ncfg * m, v * n);
-      };
-      if (n0) add(m0, n0);
-      if (n1) add(m1, n1);
-      if (n2) add(m2, n2);
+      if (n0) add(m0, n0, GCOUNTS, GSUMS);
+      if (n1) add(m1, n1, GCOUNTS, GSUMS);
+      if (n2) add(m2, n2, GCOUNTS, GSUMS);
     }
     return 0.0;
   };
@@ -563,7 +569,7 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
                 if (!ORDERED) rg[y] += __double2ll_rn(cf * wx);
               } else {
                 e += xbase + (yran ? nbin : 0);
-                if (COUNTS) hist_count_add<SHIST>(s_cnt, nh, e, (unsigned)n);
+                if (COUNTS) hist_count_add<SCOUNTS>(s_cnt, nh, e, (unsigned)n);
                 if (WEIGHTED)
                   hist_fix_add<SHIST>(s_lim, nh, e,
                                       __double2ll_rn((yran ? wpx1 : wpx0) * rw[y]) * n);
@@ -793,7 +799,7 @@ __global__ void __launch_bounds__(LONG ? kLongWarps * 32 : kRootWarps * 32, LONG
   if (SHIST) {
     __syncthreads();
     for (int k = threadIdx.x; k < nh; k += blockDim.x) {
-      if (COUNTS) {
+      if (SCOUNTS) {
         const unsigned long long v = hist_count_value(s_cnt, nh, k);
         if (v) atomicAdd(&g_cnt[k], v);
       }
@@ -841,13 +847,17 @@ void launch_root(const DevCatalog& C, RootParams T, bool weighted, bool counts, 
                  const RootArgs& A, unsigned long long* stats, int* work, int* long_list,
                  const RootLong& R, cudaStream_t s) {
   const int nh = T.ncfg * T.nmu * 4;
-  const bool shist = !adj && root_shist(nh, weighted, counts);
+  // all histograms in shared memory, else the sums alone: adding to counts in
+  // global memory returns nothing to wait for
+  const bool all = !adj && root_shist(nh, weighted, counts);
+  const bool shist = all || (!adj && weighted && root_shist(nh, true, false));
+  const bool scounts = counts && all;
   const bool ids = T.rsd && T.asym;
   int nw = kLongWarps;
   size_t smem = 0;
   int64_t blocks = 0;
   if (LONG) {
-    smem = root_layout(nh, T.nmu, T.nbins, 0, shist, weighted && !adj, counts && !adj, nw, adj, T.rsd != 0, ids, 1)
+    smem = root_layout(nh, T.nmu, T.nbins, 0, shist, weighted && !adj, scounts, nw, adj, T.rsd != 0, ids, 1)
                .total;
     blocks = R.blocks;
   } else {
@@ -856,11 +866,11 @@ void launch_root(const DevCatalog& C, RootParams T, bool weighted, bool counts, 
       // neighbours of a dense spot grabbed together end the launch alone (SMs
       // busy 61% of the time with four per grab).  With vertices of one bin
       // merged: 160,000 points, 1,540 configurations by 8 mu bins 0.61 -> 0.51
-      // ms, 816 by 2 with counts 1.74 -> 0.85 ms.
+      // ms.
       T.chunk = std::max(1, std::min(T.chunk, (int)(C.n / ((int64_t)sm_count() * kRootWarps * 32))));
       T.group = std::min(T.group, T.chunk);
     }
-    root_shape(T, weighted && !adj, counts && !adj, shist, adj, nw, T.cap, smem);
+    root_shape(T, weighted && !adj, scounts, shist, adj, nw, T.cap, smem);
     blocks = sm_count();
     const int64_t per = (int64_t)nw * T.chunk;
     const int64_t need = ((int64_t)C.n + per - 1) / per;
@@ -878,16 +888,17 @@ void launch_root(const DevCatalog& C, RootParams T, bool weighted, bool counts, 
                                                 A.cot2, A.cot3, A.gscale, A.g_lo, A.g_hi);
   };
   if (adj) {
-    go(root3_kernel<MU, false, false, false, true, BUF, LONG>);
+    go(root3_kernel<MU, false, kNoCounts, false, true, BUF, LONG>);
   } else if (weighted && counts) {
-    if (shist) go(root3_kernel<MU, true, true, true, false, BUF, LONG>);
-    else go(root3_kernel<MU, true, true, false, false, BUF, LONG>);
+    if (all) go(root3_kernel<MU, true, kWithSums, true, false, BUF, LONG>);
+    else if (shist) go(root3_kernel<MU, true, kCountsApart, true, false, BUF, LONG>);
+    else go(root3_kernel<MU, true, kWithSums, false, false, BUF, LONG>);
   } else if (weighted) {
-    if (shist) go(root3_kernel<MU, true, false, true, false, BUF, LONG>);
-    else go(root3_kernel<MU, true, false, false, false, BUF, LONG>);
+    if (shist) go(root3_kernel<MU, true, kNoCounts, true, false, BUF, LONG>);
+    else go(root3_kernel<MU, true, kNoCounts, false, false, BUF, LONG>);
   } else {
-    if (shist) go(root3_kernel<MU, false, true, true, false, BUF, LONG>);
-    else go(root3_kernel<MU, false, true, false, false, BUF, LONG>);
+    if (shist) go(root3_kernel<MU, false, kWithSums, true, false, BUF, LONG>);
+    else go(root3_kernel<MU, false, kWithSums, false, false, BUF, LONG>);
   }
   GR_CHECK_LAUNCH();
 }
