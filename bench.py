@@ -775,9 +775,8 @@ def sub_batched(args, stream, flush):
                                 "per_region_sum_f64": res["f64"][1]},
            "clocks": ck.clocks}
     # issue and shared-atomic ceilings of the tile sweep, from its ncu summary
-    # (10%-scale catalogue: the same density, so about the same instructions
-    # per binned pair, though not per pair tested: smaller regions have more
-    # halo), over the whole batched call's device time (layout kernels
+    # (10%-scale catalogue: the same density, so the same instructions per
+    # binned pair), over the whole batched call's device time (layout kernels
     # included: a lower bound for the sweep kernel alone)
     prof = roofline.profile("pair2_tile_kernel", "c4")
     n_sm = torch.cuda.get_device_properties(0).multi_processor_count
