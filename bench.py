@@ -20,9 +20,11 @@ parity     the GPU result on the full catalogue against that CPU result
 fp64_path  the same steps with every pair in FP64 (GR_OPT_PRECISION=1), and
            whether its counts and sums are identical to the FP32 path's
 
-With one GPU the line also carries the other workloads as sub-records, each
-with its device-time value, end-to-end value (host inputs), parity against
-the oracle and CPU baseline:
+The line on standard output is short: the result, its end-to-end form, clocks,
+and of roofline and parity the summary.  The whole record goes to standard
+error as one line.  With one GPU it also carries the other workloads as
+sub-records, each with its device-time value, end-to-end value (host inputs),
+parity against the oracle and CPU baseline:
 pcf2       plain 2PCF: 20,000 + 50,000 uniform points in [0,1000]^3, rmin 10,
            rmax 50, 10 bins
 quad       4PCF: 30,000 Neyman-Scott galaxies + 90,000 randoms in [0,300]^3,
@@ -534,7 +536,8 @@ def run_ours(args):
             except Exception as e:  # recorded, not hidden: the line says what failed
                 line[key] = {"error": f"{type(e).__name__}: {e}"}
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        print(json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(short_line(line)), flush=True)
     if world > 1:
         import torch.distributed as dist
 
@@ -892,6 +895,19 @@ def sub_adjoint(args, stream, flush):
         del xyz_d, w_d, wt
         torch.cuda.empty_cache()
     return rec
+
+
+def short_line(line):
+    """What is printed of a record on standard output, in 1.5 KB."""
+    keys = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+            "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "config", "e2e",
+            "clocks", "gpu_launches")
+    out = {k: line[k] for k in keys if k in line}
+    for key, parts in (("roofline", ("kernel", "frac", "binding", "binding_frac")),
+                       ("parity", ("counts_exact", "max_rel_catsum"))):
+        if key in line:
+            out[key] = {k: line[key][k] for k in parts if k in line[key]}
+    return out
 
 
 def run_sub(args, fn):
