@@ -32,7 +32,9 @@ def _context(device):
 
 def _load(c, w, xyz, n_data, bins):
     """Hand the catalogue to the library: CUDA tensors by device pointer
-    (gr_set_catalog_dev, no host round trip), host tensors through NumPy."""
+    (gr_set_catalog_dev, no host round trip), host tensors through NumPy.
+    No forward call's catalogue is held from here on, also when this fails."""
+    _holder.pop(id(c), None)
     if xyz.is_cuda and w.is_cuda:
         c.set_catalog(xyz.detach(), w.detach(), n_data)
     else:
